@@ -4,24 +4,25 @@
 // einsums.  Here every term is contracted as it is generated, in float64:
 //
 //   k_grad_dm   dm0 = 2 C_occ C_occ^T, dme0 = 2 C_occ eps_occ C_occ^T (nanoDFT.py:405-406);
-//   k_grad_2e   d/dR of 1/2 <D, J> - hyb/4 <D, K> (the vj / vk terms, nanoDFT.py:416-418): one
-//               warp per task of the ERI work list (bra shell pair x up to 32 kets of one
-//               class), one canonical shell quartet per lane, class-specialised;
-//   k_grad_1e   d/dR of <D, T + V_nuc> - <dme0, S> (h1aos and s1, nanoDFT.py:420-424): one CTA
-//               per molecule, one ordered shell pair per thread;
+//   k_grad_sp   d/dR of 1/2 <D, J> - hyb/4 <D, K> (the vj / vk terms, nanoDFT.py:416-418): one
+//               warp per super-shell slice x 32 ket pairs of one class, one ket primitive per
+//               lane (grad_sp.cuh);
+//   k_grad_1e   d/dR of <D, T + V_nuc> - <dme0, S> (h1aos and s1, nanoDFT.py:420-424): one warp
+//               per super-shell slice, lanes over nuclei;
 //   k_grad_xc   d/dR of E_xc at fixed density and grid (V_xc, nanoDFT.py:408-415): one CTA per
 //               32 grid points of one molecule, AO values, D-products and B3LYP staged in
 //               shared memory;
 //   k_grad_nuc  nuclear repulsion (grad_nuc, nanoDFT.py:428-438).
 //
-// The per-term math is grad_math.cuh, the same code the host-check build tests against the
-// finite-difference oracle.
+// The per-term math is grad_sp.cuh and grad_math.cuh, the same code the host-check build tests
+// against the finite-difference oracle.
 #include <algorithm>
-#include <utility>
+#include <cstring>
 #include <vector>
 #include "device_plan.cuh"
 #include "devmem.cuh"
 #include "grad_math.cuh"
+#include "grad_sp.cuh"
 
 #define B2G_TP 32                  // grid points per XC tile (one warp's lanes)
 #define B2G_XC_THREADS 256
@@ -47,331 +48,306 @@ k_grad_dm(const B2MolDev *__restrict__ mols, const double *__restrict__ C, const
   }
 }
 
-// Two-electron part over canonical shell quartets: one warp per task of the float32 ERI work
-// list (bra shell pair IJ x up to 32 kets of one class, the group G fixing all four angular
-// momenta); the warp takes the task's canonical kets (KL <= IJ; the list also holds kets KL > IJ
-// of the bra's last shell, which the s8 writer needs) one after the other and shares the work
-// of each shell quartet over its lanes:
-//   * primitive pairs: the bra's (once per task) and the ket's (once per quartet) Gaussian
-//     products, one pair per lane, into shared memory; pairs with |K| < 1e-20 (coefficients
-//     included) are dropped;
-//   * primitive quartets in batches of 32, one per lane: the quartet's scalars (W - P, W - Q,
-//     the recursion factors, pref x Boys F_0..F_L) into shared memory;
-//   * per primitive quartet of the batch, the lanes split the Obara-Saika vertical recursion
-//     for [e0|f0]^(m) level by level (one buffer per warp; the recursion steps of the class --
-//     target, sources, direction, factors -- are tabulated once per CTA), once with the bra
-//     raised by one (the bra-centre derivatives) and once with the ket raised by one (the
-//     derivative on the centre of K); the weighted sums over primitives (1, 2 alpha, 2 beta;
-//     1, 2 gamma) stay in the registers of the lane that owns the (e, f) entry;
-//   * the horizontal recursion and the contraction with the symmetrised Gamma run with the
-//     quartet's components spread over the lanes; the derivatives on the centres of K and L
-//     (the latter by translation invariance) are reduced over the warp per quartet, the bra
-//     centres' once per task.
-// Same formulas as the serial b2g_canonical_quartet (grad_math.cuh), which the host build runs.
-// v[e][f][m] of NCB primitive quartets at once (buffer c at v + c NV; v[0][0][m] already set),
-// lanes over (step, quartet) pairs level by level.  Quartet c's scalars: cs + c B2G_CS (W - P,
-// W - Q, rho/zeta, rho/eta, 1/(2 zeta), 1/(2 eta), 1/(2 (zeta + eta))) and its pair records
-// (P - A from the bra's, Q - C from the ket's), selected by idx[c].
-template <typename S, int LE, int LF, int NCB>
-__device__ __forceinline__ void b2g_vrr_warp(double *v, const B2gOp *ops, int lane, int nv, const double *cs,
-                                             const double *bpr, const double *kpr, const unsigned char (*idx)[2]);
-#define B2G_PP 12                  // doubles per primitive-pair record
-#define B2G_CS 18                  // doubles per primitive-quartet record
-#define B2G_KTHR 1e-20             // primitive pairs with |K| below this are dropped
+// ---- two-electron and one-electron parts: super-shell slices (grad_sp.cuh)
+//
+// Tables of a call, in one scratch block: per molecule the super-shell and pair ranges, the super
+// shells (host), the screened primitive pairs of every super-shell pair (k_gs_prims), and the
+// task prefix of each kernel.
+struct B2gsMol {
+  int ns, np, su_off, pad;         // s-only and sp super shells, first super shell
+  long long pr_off;                // first super-shell pair
+};
+#define B2GS_TABLE (B2_BOYS_NT * B2_BOYS_NM)
 
-template <typename S, int LE, int LF, int NCB>
-__device__ __forceinline__ void b2g_vrr_warp(double *v, const B2gOp *ops, int lane, int nv, const double *cs,
-                                             const double *bpr, const double *kpr, const unsigned char (*idx)[2]) {
-#pragma unroll
-  for (int l1 = 1; l1 <= LE; ++l1) {
-    const int lo = b2g_cstart(l1) - 1, n = (b2g_cstart(l1 + 1) - 1 - lo) * NCB;
-    for (int t = lane; t < n; t += 32) {
-      const int o = lo + t / NCB, c = t - (t / NCB) * NCB;
-      if (c >= nv) continue;
-      const B2gOp op = ops[o];
-      const double *q = cs + c * B2G_CS, *B = bpr + idx[c][0] * B2G_PP;
-      const double x = B[6 + op.dd], y = q[op.dd];
-      const double cc = (double)op.c1 * q[8], rb = q[6];
-      double *vc = v + c * S::NV;
-#pragma unroll
-      for (int m = 0; m < S::SM; ++m)              // independent in m: unrolled, predicated
-        if (m <= op.mmax) {
-          double u = x * vc[op.s1 + m] + y * vc[op.s1 + m + 1];
-          if (op.s2 >= 0) u += cc * (vc[op.s2 + m] - rb * vc[op.s2 + m + 1]);
-          vc[op.dst + m] = u;
-        }
-    }
-    __syncwarp();
+__device__ __forceinline__ int b2gs_find(const long long *__restrict__ off, int n, long long x) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= x) lo = mid; else hi = mid - 1;
   }
-#pragma unroll
-  for (int l2 = 1; l2 <= LF; ++l2) {
-    const int lo = S::NOB + (b2g_cstart(l2) - 1) * S::NE;
-    const int n = (b2g_cstart(l2 + 1) - b2g_cstart(l2)) * S::NE * NCB;
-    for (int t = lane; t < n; t += 32) {
-      const int o = lo + t / NCB, c = t - (t / NCB) * NCB;
-      if (c >= nv) continue;
-      const B2gOp op = ops[o];
-      if (op.mmax < 0) continue;
-      const double *q = cs + c * B2G_CS, *K = kpr + idx[c][1] * B2G_PP;
-      const double x = K[6 + op.dd], y = q[3 + op.dd];
-      const double cc = (double)op.c1 * q[9], rk = q[7], c3 = (double)op.c3 * q[10];
-      double *vc = v + c * S::NV;
-#pragma unroll
-      for (int m = 0; m < S::SM; ++m)
-        if (m <= op.mmax) {
-          double u = x * vc[op.s1 + m] + y * vc[op.s1 + m + 1];
-          if (op.s2 >= 0) u += cc * (vc[op.s2 + m] - rk * vc[op.s2 + m + 1]);
-          if (op.s3 >= 0) u += c3 * vc[op.s3 + m + 1];
-          vc[op.dst + m] = u;
-        }
-    }
-    __syncwarp();
-  }
+  return lo;
 }
 
-// per-class sizes of the two-electron kernel's shared memory (doubles per warp)
-template <int G> struct B2g2e {
-  static constexpr int LA = b2g_group_l(G, 0), LB = b2g_group_l(G, 1), LC = b2g_group_l(G, 2),
-                       LD = b2g_group_l(G, 3);
-  static constexpr int L = LA + LB + LC + LD + 1;
-  using SB = B2gVrr<LA + LB + 1, LC + LD, L>;              // bra raised by one
-  using SK = B2gVrr<LA + LB, LC + LD + 1, L>;              // ket raised by one
-  static constexpr int NVB = SB::NV > SK::NV ? SB::NV : SK::NV;
-  static constexpr int NACC = 3 * SB::NACC + 2 * SK::NACC;
-  // primitive quartets whose recursions run side by side (buffers of at most 1200 doubles)
-  static constexpr int NCB = 1200 / NVB >= 4 ? 4 : (1200 / NVB >= 2 ? 2 : 1);
-  static constexpr int NBUF = NCB * NVB > NACC ? NCB * NVB : NACC;
-  static constexpr int PER_WARP = NBUF + 2 * B2_MAXPRIM * B2_MAXPRIM * B2G_PP + 32 * B2G_CS;
-  static constexpr size_t SMEM = sizeof(double) * 4 * PER_WARP;
+// primitive pairs of every super-shell pair, one thread per pair: the surviving ones packed
+// (nine slots per pair), their number in pn
+__global__ void __launch_bounds__(128)
+k_gs_prims(const B2gsMol *__restrict__ gm, const long long *__restrict__ poff, int nmol,
+           const B2gSuper *__restrict__ su, B2gPrim *__restrict__ pr, unsigned char *__restrict__ pn) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= poff[nmol]) return;
+  const int m = b2gs_find(poff, nmol, t);
+  const B2gsMol g = gm[m];
+  int A, B;
+  b2gs_pair(g.ns, g.np, (int)(t - g.pr_off), A, B);
+  const B2gSuper a = su[g.su_off + A], b = su[g.su_off + B];
+  int n = 0;
+  for (int p = 0; p < a.nprim; ++p)
+    for (int q = 0; q < b.nprim; ++q) {
+      B2gPrim r;
+      if (b2gs_prim(a, b, p, q, r)) pr[t * B2_MAXPP + n++] = r;
+    }
+  pn[t] = (unsigned char)n;
+}
+
+// per-warp shared memory of the two-electron kernel
+struct __align__(16) B2gsWarp {
+  B2gBraRec bra[B2_MAXPP];
+  double CD[32][3], wt[32], acc[32][6];
+  int ao[32][4], off[32], pair[32];
+  unsigned char map[32 * B2_MAXPP];
 };
 
-// primitive pair (p, q) of shells (s, t): exponents, zeta, P, P - R_s, K (coefficients
-// included), 1 / zeta
-__device__ __forceinline__ void b2g_pair_rec(const B2Shell &s, const B2Shell &t, int p, int q, double R2,
-                                             double *o) {
-  const double al = s.exp[p], be = t.exp[q], z = al + be, iz = 1.0 / z;
-  o[0] = al;
-  o[1] = be;
-  o[2] = z;
+// density factors, bra loop and centre sums of one ket primitive (axis KF of the ket's p
+// function relative to the bra's)
+template <int TB, int TK, int KF>
+__device__ __forceinline__ void b2gs_lane(const B2gsWarp &W, int nb, int k, const B2gPrim &r, const double *AB, int f,
+                                          int F, const int *bi, const double *__restrict__ Dm, int N, double hyb,
+                                          const double *tab, double *gA, double *gB, double *gC, double *gD) {
+  using C = B2gsClass<TB, TK>;
+  const int cs = W.ao[k][0], cp = W.ao[k][1], ds = W.ao[k][2], dp = W.ao[k][3];
+  const int F2 = TK == 2 ? (cp < 0 ? -1 : cp + (f + KF) % 3) : cs;
+  int di[4] = {ds, -1, -1, -1};
+  double CD[3], QD[3], Q[3];
+#pragma unroll
   for (int x = 0; x < 3; ++x) {
-    const double P = (al * s.R[x] + be * t.R[x]) * iz;
-    o[3 + x] = P;
-    o[6 + x] = P - s.R[x];
+    const int px = f + x >= 3 ? f + x - 3 : f + x;
+    if (TK && dp >= 0) di[1 + x] = dp + px;
+    CD[x] = W.CD[k][x];
+    QD[x] = r.ra * CD[x];
+    Q[x] = px == 0 ? r.P[0] : (px == 1 ? r.P[1] : r.P[2]);
   }
-  o[9] = exp(-al * be * iz * R2) * s.coef[p] * t.coef[q];
-  o[10] = iz;
-  o[11] = 0.0;
-}
-
-// lanes 0..np-1 each form one primitive pair; the surviving ones are packed into rec; returns
-// their number (same value on every lane)
-__device__ __forceinline__ int b2g_pairs_warp(const B2Shell &s, const B2Shell &t, double R2, double *rec, int lane) {
-  const int np = s.nprim * t.nprim;
-  double o[B2G_PP];
-  bool keep = false;
-  if (lane < np) {
-    b2g_pair_rec(s, t, lane / t.nprim, lane - (lane / t.nprim) * t.nprim, R2, o);
-    keep = fabs(o[9]) >= B2G_KTHR;
-  }
-  const unsigned bal = __ballot_sync(0xffffffffu, keep);
-  if (keep) {
-    const int pos = __popc(bal & ((1u << lane) - 1u));
+  B2gKet<C::NB, C::NK> q;
+  b2gs_ket<C::NB, C::NK>(Dm, N, hyb, W.wt[k], F, bi, F2, di, TK == 2 ? r.kps : r.kss, TK == 2 ? r.kpp : r.ksp, QD, q);
+  q.v = r.u;
+  q.FC = (r.ra - 1.0) * CD[KF < 0 ? 0 : KF];
+  B2gOut s;
+  s.E = s.C = 0.0;
 #pragma unroll
-    for (int k = 0; k < B2G_PP; ++k) rec[pos * B2G_PP + k] = o[k];
-  }
-  __syncwarp();
-  return __popc(bal);
-}
-
-template <int G>
-__global__ void __launch_bounds__(128)
-k_grad_2e(const B2EriTask *__restrict__ tasks, long long ntask, const B2MolDev *__restrict__ mols,
-          const B2PairInfo *__restrict__ pinfo, const int *__restrict__ cls_list,
-          const B2Shell *__restrict__ shells, const double *__restrict__ btab, const double *__restrict__ D,
-          double hyb, double *__restrict__ grad) {
-  using C2 = B2g2e<G>;
-  constexpr int LA = C2::LA, LB = C2::LB, LC = C2::LC, LD = C2::LD, L = C2::L;
-  constexpr int na = 2 * LA + 1, nb = 2 * LB + 1, nc = 2 * LC + 1, nd = 2 * LD + 1, NCMP = na * nb * nc * nd;
-  using SB = typename C2::SB;
-  using SK = typename C2::SK;
-  constexpr int KB = (SB::NACC + 31) / 32, KK = (SK::NACC + 31) / 32;
-  extern __shared__ __align__(16) double g2_smem[];
-  __shared__ B2gOp sopB[SB::NOP], sopK[SK::NOP];
-  __shared__ unsigned char sIdx[4][32][2];
-  for (int o = threadIdx.x; o < SB::NOP; o += blockDim.x) sopB[o] = SB::op(o);
-  for (int o = threadIdx.x; o < SK::NOP; o += blockDim.x) sopK[o] = SK::op(o);
-  __syncthreads();
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long ti = (long long)blockIdx.x * 4 + w;
-  if (ti >= ntask) return;                        // whole warp (no CTA barrier follows)
-  double *v = g2_smem + (size_t)w * C2::PER_WARP;
-  double *bpr = v + C2::NBUF, *kpr = bpr + B2_MAXPRIM * B2_MAXPRIM * B2G_PP;
-  double *cs = kpr + B2_MAXPRIM * B2_MAXPRIM * B2G_PP;
-  const B2EriTask tk = tasks[ti];
-  const B2MolDev md = mols[tk.mol];
-  const B2PairInfo bp = pinfo[md.sp_off + tk.IJ];
-  const B2Shell &a = shells[md.sh_off + bp.I], &b = shells[md.sh_off + bp.J];
-  const double *Dm = D + md.mat_off;
-  const int N = md.nao;
-  double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};   // this lane's part of the bra-centre sums
-  double AB[3], AB2 = 0;
-  for (int x = 0; x < 3; ++x) { AB[x] = a.R[x] - b.R[x]; AB2 += AB[x] * AB[x]; }
-  const int nbp = b2g_pairs_warp(a, b, AB2, bpr, lane);
-  double *gm = grad + 3ll * md.atm_off;
-  for (int kq = 0; kq < tk.count; ++kq) {
-    const int KL = cls_list[md.sp_off + md.cls_start[tk.cls] + tk.start + kq];
-    if (KL > tk.IJ) continue;                     // uniform over the warp
-    const B2PairInfo kp = pinfo[md.sp_off + KL];
-    const B2Shell &c = shells[md.sh_off + kp.I], &d = shells[md.sh_off + kp.J];
-    double CD[3], CD2 = 0;
-    for (int x = 0; x < 3; ++x) { CD[x] = c.R[x] - d.R[x]; CD2 += CD[x] * CD[x]; }
-    const int nkp = b2g_pairs_warp(c, d, CD2, kpr, lane);
-    double accB[3][KB], accK[2][KK];
+  for (int x = 0; x < 3; ++x) s.dP[x] = s.D[x] = 0.0;
+#pragma unroll 1
+  for (int p = 0; p < nb; ++p) {
+    B2gOut o;
+    b2gs_eval<TB, TK, KF>(W.bra[p], q, Q, r.z, tab, o);
+    b2gs_add_bra<TB>(W.bra[p], AB, o, gA, gB);
+    s.E += o.E;
 #pragma unroll
-    for (int k = 0; k < KB; ++k) accB[0][k] = accB[1][k] = accB[2][k] = 0.0;
-#pragma unroll
-    for (int k = 0; k < KK; ++k) accK[0][k] = accK[1][k] = 0.0;
-    const int ncombo = nbp * nkp;
-    for (int c0 = 0; c0 < ncombo; c0 += 32) {
-      // ---- scalars of up to 32 primitive quartets, one per lane
-      const int cb = c0 + lane;
-      if (cb < ncombo) {
-        const int ib = cb / nkp, ik = cb - (cb / nkp) * nkp;
-        const double *B = bpr + ib * B2G_PP, *K = kpr + ik * B2G_PP;
-        const double z = B[2], e = K[2], iz = B[10], ie = K[10];
-        const double rs = rsqrt(z + e), inv = rs * rs;          // 1/sqrt(zeta+eta), 1/(zeta+eta)
-        double *o = cs + lane * B2G_CS;
-        double PQ2 = 0;
-        for (int x = 0; x < 3; ++x) {
-          const double P = B[3 + x], Q = K[3 + x];
-          const double W = (z * P + e * Q) * inv;
-          o[x] = W - P;                             // WP
-          o[3 + x] = W - Q;                         // WQ
-          PQ2 += (P - Q) * (P - Q);
-        }
-        const double rho = z * e * inv;
-        const double pref = 34.98683665524972 * iz * ie * rs * B[9] * K[9];   // 2 pi^(5/2) / (z e sqrt(z+e)) K K
-        double F[L + 1];
-        b2_boys<double, L, double>(rho * PQ2, btab, F);
-        o[6] = e * inv;                           // rho / zeta
-        o[7] = z * inv;                           // rho / eta
-        o[8] = 0.5 * iz;
-        o[9] = 0.5 * ie;
-        o[10] = 0.5 * inv;
-#pragma unroll
-        for (int m = 0; m <= L; ++m) o[11 + m] = pref * F[m];
-        sIdx[w][lane][0] = (unsigned char)ib;
-        sIdx[w][lane][1] = (unsigned char)ik;
-      }
-      __syncwarp();
-      const int nq = min(32, ncombo - c0);
-      constexpr int NCB = C2::NCB;
-      for (int q0 = 0; q0 < nq; q0 += NCB) {
-        const int nv = min(NCB, nq - q0);
-        const double *csq = cs + q0 * B2G_CS;
-        // bra raised: [e0|f0], e <= LA + LB + 1, f <= LC + LD
-        for (int t = lane; t < nv * (L + 1); t += 32) {
-          const int c = t / (L + 1), m = t - (t / (L + 1)) * (L + 1);
-          v[c * SB::NV + m] = csq[c * B2G_CS + 11 + m];
-        }
-        __syncwarp();
-        b2g_vrr_warp<SB, LA + LB + 1, LC + LD, NCB>(v, sopB, lane, nv, csq, bpr, kpr, sIdx[w] + q0);
-#pragma unroll
-        for (int k = 0; k < KB; ++k) {
-          const int t = lane + 32 * k;
-          if (t < SB::NACC) {
-            const int ie = t / SB::NF, jf = t - (t / SB::NF) * SB::NF;
-            for (int c = 0; c < nv; ++c) {
-              const double x = v[c * SB::NV + ie * SB::SE + jf * SB::SM];
-              const double *B = bpr + sIdx[w][q0 + c][0] * B2G_PP;
-              accB[0][k] += x;
-              accB[1][k] += 2.0 * B[0] * x;
-              accB[2][k] += 2.0 * B[1] * x;
-            }
-          }
-        }
-        __syncwarp();
-        // ket raised: e <= LA + LB, f <= LC + LD + 1
-        for (int t = lane; t < nv * (L + 1); t += 32) {
-          const int c = t / (L + 1), m = t - (t / (L + 1)) * (L + 1);
-          v[c * SK::NV + m] = csq[c * B2G_CS + 11 + m];
-        }
-        __syncwarp();
-        b2g_vrr_warp<SK, LA + LB, LC + LD + 1, NCB>(v, sopK, lane, nv, csq, bpr, kpr, sIdx[w] + q0);
-#pragma unroll
-        for (int k = 0; k < KK; ++k) {
-          const int t = lane + 32 * k;
-          if (t < SK::NACC) {
-            const int ie = t / SK::NF, jf = t - (t / SK::NF) * SK::NF;
-            for (int c = 0; c < nv; ++c) {
-              const double x = v[c * SK::NV + ie * SK::SE + jf * SK::SM];
-              const double *K = kpr + sIdx[w][q0 + c][1] * B2G_PP;
-              accK[0][k] += x;
-              accK[1][k] += 2.0 * K[0] * x;
-            }
-          }
-        }
-        __syncwarp();
-      }
-    }
-    // weighted sums to shared memory: accB[w][e][f], then accK[w][e][f]
-#pragma unroll
-    for (int k = 0; k < KB; ++k) {
-      const int t = lane + 32 * k;
-      if (t < SB::NACC)
-        for (int q = 0; q < 3; ++q) v[q * SB::NACC + t] = accB[q][k];
-    }
-#pragma unroll
-    for (int k = 0; k < KK; ++k) {
-      const int t = lane + 32 * k;
-      if (t < SK::NACC)
-        for (int q = 0; q < 2; ++q) v[3 * SB::NACC + q * SK::NACC + t] = accK[q][k];
-    }
-    __syncwarp();
-    const auto *aB = reinterpret_cast<const double (*)[SB::NE][SB::NF]>(v);
-    const auto *aK = reinterpret_cast<const double (*)[SK::NE][SK::NF]>(v + 3 * SB::NACC);
-    const double deg = (bp.I == bp.J ? 1.0 : 2.0) * (kp.I == kp.J ? 1.0 : 2.0) * (KL == tk.IJ ? 1.0 : 2.0);
-    double gC[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
-    for (int cmp = lane; cmp < NCMP; cmp += 32) {
-      const int id = cmp % nd, ic = (cmp / nd) % nc, ib = (cmp / (nd * nc)) % nb, ia = cmp / (nd * nc * nb);
-      const int i = a.ao0 + ia, j = b.ao0 + ib, k = c.ao0 + ic, l = d.ao0 + id;
-      const double gmv = deg * (0.5 * Dm[i * N + j] * Dm[k * N + l] -
-                                0.125 * hyb * (Dm[i * N + l] * Dm[j * N + k] + Dm[i * N + k] * Dm[j * N + l]));
-      if (gmv == 0.0) continue;
-      int ea[3], eb[3], ec[3], ed[3];
-      b2g_comp(LA, ia, ea); b2g_comp(LB, ib, eb); b2g_comp(LC, ic, ec); b2g_comp(LD, id, ed);
-      for (int x = 0; x < 3; ++x) {
-        int up[3], dn[3];
-        for (int q = 0; q < 3; ++q) { up[q] = ea[q] + (q == x); dn[q] = ea[q] - (q == x); }
-        double dA = b2g_hrr(aB, 1, up, eb, ec, ed, AB, CD);
-        if (ea[x]) dA -= (double)ea[x] * b2g_hrr(aB, 0, dn, eb, ec, ed, AB, CD);
-        for (int q = 0; q < 3; ++q) { up[q] = eb[q] + (q == x); dn[q] = eb[q] - (q == x); }
-        double dB = b2g_hrr(aB, 2, ea, up, ec, ed, AB, CD);
-        if (eb[x]) dB -= (double)eb[x] * b2g_hrr(aB, 0, ea, dn, ec, ed, AB, CD);
-        for (int q = 0; q < 3; ++q) { up[q] = ec[q] + (q == x); dn[q] = ec[q] - (q == x); }
-        double dC = b2g_hrr(aK, 1, ea, eb, up, ed, AB, CD);
-        if (ec[x]) dC -= (double)ec[x] * b2g_hrr(aK, 0, ea, eb, dn, ed, AB, CD);
-        gA[x] += gmv * dA;
-        gB[x] += gmv * dB;
-        gC[x] += gmv * dC;
-        g3[x] -= gmv * (dA + dB + dC);
-      }
-    }
     for (int x = 0; x < 3; ++x) {
-      double u = gC[x], t = g3[x];
+      s.dP[x] += o.dP[x];
+      if (TK) s.D[x] += o.D[x];
+    }
+    if (TK == 2) s.C += o.C;
+  }
+  b2gs_add_ket<TK, KF>(r.ra, r.mu2, CD, s, gC, gD);
+}
+
+// Two-electron part of one class (bra slices of type TB, ket slices of type TK <= TB; each
+// unordered slice quartet once).  One warp per task (molecule, bra slice, 32 kets): the kets'
+// surviving primitive pairs are packed over the lanes; a lane contracts its ket primitive with the
+// density factors once and runs over the bra's primitive pairs in shared memory, so a lane holds
+// one primitive quartet's derivative tensor (up to 56 values) in registers and no integral is ever
+// stored.  The bra centres' sums stay in registers for the whole task; the ket centres' are summed
+// over the lanes of a ket by a segmented scan.  CTAs stay resident and stride over the tasks; the
+// Boys table sits in shared memory (its rows are gathered at random: from global memory those
+// gathers took longer than the arithmetic of the small classes).
+// Bound by FP64 issue and latency (118-255 registers: 8-16 warps per SM); the whole gradient of
+// 160 uneven molecules takes 31 ms, of one molecule with 5 heavy atoms 0.26 ms.  Before (one warp
+// per shell quartet and l class in 16 kernels, contracted Obara-Saika [e0|f0] arrays through
+// shared memory and a horizontal recursion per quartet): 732 ms and 65 ms.
+template <int TB, int TK>
+__global__ void __launch_bounds__(128)
+k_grad_sp(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
+          const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su, const B2gPrim *__restrict__ pr,
+          const unsigned char *__restrict__ pn, const double *__restrict__ btab, const double *__restrict__ D,
+          double hyb, double *__restrict__ grad) {
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  double *tab = reinterpret_cast<double *>(gs_smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  B2gsWarp &W = reinterpret_cast<B2gsWarp *>(gs_smem + sizeof(double) * B2GS_TABLE)[w];
+  for (int e = threadIdx.x; e < B2GS_TABLE; e += blockDim.x) tab[e] = btab[e];
+  __syncthreads();
+  const long long ntask = toff[nmol];
+  for (long long task = (long long)blockIdx.x * 4 + w; task < ntask; task += (long long)gridDim.x * 4) {
+    const int m = b2gs_find(toff, nmol, task);
+    const B2gsMol g = gms[m];
+    const int nket = b2gs_nket(g.ns, g.np, TK), nch = (nket + 31) >> 5;
+    const int r0 = (int)(task - toff[m]), i = r0 / nch, k0 = (r0 - i * nch) * 32;
+    const int bpr = TB == 2 ? i / 3 : i, f = TB == 2 ? i - 3 * (i / 3) : 0;
+    const int cnt = min(32, (TB == TK ? bpr + 1 : nket) - k0);
+    if (cnt <= 0) continue;                        // whole warp: beyond the diagonal
+    const B2MolDev md = mols[m];
+    const B2gSuper *sm = su + g.su_off;
+    const double *Dm = D + md.mat_off;
+    const int N = md.nao;
+    int A, B;
+    const int pb = b2gs_ket_pair(g.ns, g.np, TB, bpr);
+    b2gs_pair(g.ns, g.np, pb, A, B);
+    double AB[3];
+    int bi[4] = {sm[B].ao_s, -1, -1, -1};
+    const int F = TB == 2 ? (sm[A].ao_p < 0 ? -1 : sm[A].ao_p + f) : sm[A].ao_s;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      const int px = f + x >= 3 ? f + x - 3 : f + x;
+      AB[x] = sm[A].R[px] - sm[B].R[px];
+      if (TB && sm[B].ao_p >= 0) bi[1 + x] = sm[B].ao_p + px;
+    }
+    const int nb = pn[g.pr_off + pb];
+    __syncwarp();                                  // the previous task's shared memory is consumed
+    if (lane < nb) b2gs_bra(pr[(g.pr_off + pb) * B2_MAXPP + lane], TB, f, AB, W.bra[lane]);
+    int nq = 0, ca = 0, da = 0;
+    if (lane < cnt) {
+      int c, d;
+      const int pk = b2gs_ket_pair(g.ns, g.np, TK, k0 + lane);
+      b2gs_pair(g.ns, g.np, pk, c, d);
+      const B2gSuper &sc = sm[c], &sd = sm[d];
+      nq = pn[g.pr_off + pk];
+      ca = sc.atom;
+      da = sd.atom;
+      W.pair[lane] = pk;
+      W.ao[lane][0] = sc.ao_s;
+      W.ao[lane][1] = sc.ao_p;
+      W.ao[lane][2] = sd.ao_s;
+      W.ao[lane][3] = sd.ao_p;
+      W.wt[lane] = (A == B ? 1.0 : 2.0) * (c == d ? 1.0 : 2.0) * (TB == TK && k0 + lane == bpr ? 1.0 : 2.0);
+#pragma unroll
+      for (int x = 0; x < 3; ++x) {
+        const int px = f + x >= 3 ? f + x - 3 : f + x;
+        W.CD[lane][x] = sc.R[px] - sd.R[px];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 6; ++x) W.acc[lane][x] = 0.0;
+    int inc = nq;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    const int E = __shfl_sync(0xffffffffu, inc, 31);
+    W.off[lane] = inc - nq;
+    for (int j = 0; j < nq; ++j) W.map[inc - nq + j] = (unsigned char)lane;
+    __syncwarp();
+    double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const bool valid = e < E;
+      const int k = valid ? (int)W.map[e] : -1 - lane;      // entries past the end: unique keys
+      double gk[6] = {0, 0, 0, 0, 0, 0};
+      if (valid) {
+        const B2gPrim r = pr[(g.pr_off + W.pair[k]) * B2_MAXPP + (e - W.off[k])];
+        if constexpr (TK == 2) {
+          b2gs_lane<TB, TK, 0>(W, nb, k, r, AB, f, F, bi, Dm, N, hyb, tab, gA, gB, gk, gk + 3);
+          b2gs_lane<TB, TK, 1>(W, nb, k, r, AB, f, F, bi, Dm, N, hyb, tab, gA, gB, gk, gk + 3);
+          b2gs_lane<TB, TK, 2>(W, nb, k, r, AB, f, F, bi, Dm, N, hyb, tab, gA, gB, gk, gk + 3);
+        } else {
+          b2gs_lane<TB, TK, -1>(W, nb, k, r, AB, f, F, bi, Dm, N, hyb, tab, gA, gB, gk, gk + 3);
+        }
+      }
+#pragma unroll
+      for (int o = 1; o < 16; o <<= 1) {                     // same-ket inclusive scan (<= 9 lanes)
+        const int ko = __shfl_up_sync(0xffffffffu, k, o);
+        const bool take = lane >= o && ko == k;
+#pragma unroll
+        for (int x = 0; x < 6; ++x) {
+          const double y = __shfl_up_sync(0xffffffffu, gk[x], o);
+          if (take) gk[x] += y;
+        }
+      }
+      const int kn = __shfl_down_sync(0xffffffffu, k, 1);
+      if (valid && (lane == 31 || kn != k))
+#pragma unroll
+        for (int x = 0; x < 6; ++x) W.acc[k][x] += gk[x];
+      __syncwarp();
+    }
+    double *gm = grad + 3ll * md.atm_off;
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      const int px = f + x >= 3 ? f + x - 3 : f + x;
+      if (lane < cnt) {
+        atomicAdd(gm + 3 * ca + px, W.acc[lane][x]);
+        atomicAdd(gm + 3 * da + px, W.acc[lane][3 + x]);
+      }
+      double u = gA[x], t = gB[x];
 #pragma unroll
       for (int o = 16; o; o >>= 1) {
         u += __shfl_xor_sync(0xffffffffu, u, o);
         t += __shfl_xor_sync(0xffffffffu, t, o);
       }
       if (lane == 0) {
-        atomicAdd(gm + 3 * c.atom + x, u);
-        atomicAdd(gm + 3 * d.atom + x, t);
+        atomicAdd(gm + 3 * sm[A].atom + px, u);
+        atomicAdd(gm + 3 * sm[B].atom + px, t);
       }
     }
-    __syncwarp();                                 // v and the pair records are rewritten next
   }
-  // the bra centres are the warp's: one sum over the lanes, one atomic per component
+}
+
+// One-electron part: one warp per bra slice of a molecule.  Overlap and kinetic energy: one
+// primitive pair per lane; nuclear attraction: lanes over (primitive pair, nucleus), the nuclei
+// of a molecule padded to 8, 16 or 32 lanes, so every lane keeps its nucleus' gradient in
+// registers over the primitive pairs.  Before: one thread per ordered shell pair with all
+// primitive pairs and nuclei in its local-memory recursion tables, one CTA per molecule.
+template <int TB>
+__device__ __forceinline__ void b2gs_one(const B2gsMol &g, int i, const B2MolDev &md, const B2gSuper *__restrict__ sm,
+                                         const B2gPrim *__restrict__ prm, const unsigned char *__restrict__ pnm,
+                                         const double *__restrict__ xyz, const int *__restrict__ Z,
+                                         const double *tab, const double *__restrict__ Dm,
+                                         const double *__restrict__ Wm, double *__restrict__ gm, int lane) {
+  constexpr int NB = TB ? 1 : 0;
+  const int bpr = TB == 2 ? i / 3 : i, f = TB == 2 ? i - 3 * (i / 3) : 0, N = md.nao;
+  const int pb = b2gs_ket_pair(g.ns, g.np, TB, bpr);
+  int A, B;
+  b2gs_pair(g.ns, g.np, pb, A, B);
+  const B2gSuper &sa = sm[A], &sb = sm[B];
+  const int F = TB == 2 ? (sa.ao_p < 0 ? -1 : sa.ao_p + f) : sa.ao_s;
+  const double wt = A == B ? 1.0 : 2.0;
+  double AB[3], dg[NB ? 4 : 1], wg[NB ? 4 : 1];            // density factors of T / V and of S
+#pragma unroll
+  for (int b = 0; b < (NB ? 4 : 1); ++b) {
+    const int bb = b == 0 ? sb.ao_s : (sb.ao_p < 0 ? -1 : sb.ao_p + (f + b - 1) % 3);
+    const bool ok = F >= 0 && bb >= 0;
+    dg[b] = ok ? wt * Dm[F * N + bb] : 0.0;
+    wg[b] = ok ? -wt * Wm[F * N + bb] : 0.0;
+  }
+#pragma unroll
+  for (int x = 0; x < 3; ++x) AB[x] = sa.R[(f + x) % 3] - sb.R[(f + x) % 3];
+  const int nb = pnm[pb];
+  double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};
+  if (lane < nb) {
+    B2gBraRec r;
+    b2gs_bra(prm[(long long)pb * B2_MAXPP + lane], TB, f, AB, r);
+    double gk[3];
+    b2gs_st<TB>(r, dg, wg, AB, gk);
+#pragma unroll
+    for (int x = 0; x < 3; ++x) { gA[x] += gk[x]; gB[x] -= gk[x]; }
+  }
+  const int lg = md.natm <= 8 ? 3 : (md.natm <= 16 ? 4 : 5), G = 1 << lg, step = 32 >> lg;
+  for (int c0 = 0; c0 < md.natm; c0 += G) {
+    const int c = c0 + (lane & (G - 1));
+    double gN[3] = {0, 0, 0};
+    if (c < md.natm) {
+      const double q0 = -(double)Z[c] * (6.283185307179586 / 5.914967172795613);   // 2 pi over the pair constant
+      const double C[3] = {xyz[3 * c + f], xyz[3 * c + (f + 1) % 3], xyz[3 * c + (f + 2) % 3]};
+      B2gKet<NB, 0> q;
+#pragma unroll
+      for (int b = 0; b < (NB ? 4 : 1); ++b) q.gs[b] = q0 * dg[b];
+      q.v = q.FC = 0.0;
+      for (int p = lane >> lg; p < nb; p += step) {
+        B2gBraRec r;
+        b2gs_bra(prm[(long long)pb * B2_MAXPP + p], TB, f, AB, r);
+        B2gOut o;
+        b2gs_eval_point<TB>(r, q, C, tab, o);
+        b2gs_add_bra<TB>(r, AB, o, gA, gB);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) gN[x] -= o.dP[x];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+      double v = gN[x];
+      for (int o = G; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane < G && c < md.natm) atomicAdd(gm + 3 * c + (f + x) % 3, v);
+    }
+  }
+#pragma unroll
   for (int x = 0; x < 3; ++x) {
     double u = gA[x], t = gB[x];
 #pragma unroll
@@ -380,42 +356,40 @@ k_grad_2e(const B2EriTask *__restrict__ tasks, long long ntask, const B2MolDev *
       t += __shfl_xor_sync(0xffffffffu, t, o);
     }
     if (lane == 0) {
-      atomicAdd(gm + 3 * a.atom + x, u);
-      atomicAdd(gm + 3 * b.atom + x, t);
+      atomicAdd(gm + 3 * sa.atom + (f + x) % 3, u);
+      atomicAdd(gm + 3 * sb.atom + (f + x) % 3, t);
     }
   }
 }
 
-// One-electron part: each thread one ordered shell pair (I, J) of the CTA's molecule; the terms
-// on the nuclei (nuclear attraction moving with the nucleus) and on the pair's centres collect
-// in shared memory, then one atomic per component per molecule.
 __global__ void __launch_bounds__(128)
-k_grad_1e(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
-          const double *__restrict__ atom_xyz, const int *__restrict__ atom_z, const double *__restrict__ btab,
-          const double *__restrict__ D, const double *__restrict__ W, double *__restrict__ grad) {
-  __shared__ double sZ[B2_MAXNAO], sR[3 * B2_MAXNAO], sG[3 * B2_MAXNAO];
-  const B2MolDev md = mols[blockIdx.x];
-  const int natm = md.natm, nbas = md.nbas, N = md.nao;
-  for (int e = threadIdx.x; e < natm; e += blockDim.x) sZ[e] = (double)atom_z[md.atm_off + e];
-  for (int e = threadIdx.x; e < 3 * natm; e += blockDim.x) {
-    sR[e] = atom_xyz[3ll * md.atm_off + e];
-    sG[e] = 0.0;
-  }
+k_grad_1e(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
+          const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su, const B2gPrim *__restrict__ pr,
+          const unsigned char *__restrict__ pn, const double *__restrict__ atom_xyz, const int *__restrict__ atom_z,
+          const double *__restrict__ btab, const double *__restrict__ D, const double *__restrict__ Wd,
+          double *__restrict__ grad) {
+  extern __shared__ __align__(16) unsigned char gs_smem[];
+  double *tab = reinterpret_cast<double *>(gs_smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int e = threadIdx.x; e < B2GS_TABLE; e += blockDim.x) tab[e] = btab[e];
   __syncthreads();
-  const double *Dm = D + md.mat_off, *Wm = W + md.mat_off;
-  for (int it = threadIdx.x; it < nbas * nbas; it += blockDim.x) {
-    const int I = it / nbas, J = it - (it / nbas) * nbas;
-    const B2Shell &a = shells[md.sh_off + I], &b = shells[md.sh_off + J];
-    double g2[2][3];
-    b2g_pair_grad_1e<double>(a, b, Dm, Wm, N, natm, sZ, sR, btab, g2,
-                             [&](int c, int x, double v) { atomicAdd(&sG[3 * c + x], v); });
-    for (int x = 0; x < 3; ++x) {
-      atomicAdd(&sG[3 * a.atom + x], g2[0][x]);
-      atomicAdd(&sG[3 * b.atom + x], g2[1][x]);
-    }
+  const long long ntask = toff[nmol];
+  for (long long task = (long long)blockIdx.x * 4 + w; task < ntask; task += (long long)gridDim.x * 4) {
+    const int m = b2gs_find(toff, nmol, task);
+    const B2gsMol g = gms[m];
+    const B2MolDev md = mols[m];
+    int i = (int)(task - toff[m]);
+    const int n0 = b2gs_nslice(g.ns, g.np, 0), n1 = b2gs_nslice(g.ns, g.np, 1);
+    const B2gSuper *sm = su + g.su_off;
+    const B2gPrim *prm = pr + g.pr_off * B2_MAXPP;
+    const unsigned char *pnm = pn + g.pr_off;
+    const double *xyz = atom_xyz + 3ll * md.atm_off, *Dm = D + md.mat_off, *Wm = Wd + md.mat_off;
+    const int *Z = atom_z + md.atm_off;
+    double *gm = grad + 3ll * md.atm_off;
+    if (i < n0) b2gs_one<0>(g, i, md, sm, prm, pnm, xyz, Z, tab, Dm, Wm, gm, lane);
+    else if ((i -= n0) < n1) b2gs_one<1>(g, i, md, sm, prm, pnm, xyz, Z, tab, Dm, Wm, gm, lane);
+    else b2gs_one<2>(g, i - n1, md, sm, prm, pnm, xyz, Z, tab, Dm, Wm, gm, lane);
   }
-  __syncthreads();
-  for (int e = threadIdx.x; e < 3 * natm; e += blockDim.x) atomicAdd(grad + 3ll * md.atm_off + e, sG[e]);
 }
 
 // Exchange-correlation part on 32 grid points of one molecule (tile t of molecule m, tile_off:
@@ -557,228 +531,121 @@ k_grad_nuc(const B2MolDev *__restrict__ mols, const double *__restrict__ atom_xy
   }
 }
 
-// Classes with L = l_I + l_J + l_K + l_L + 1 <= 3 (at most two p shells): the recursion arrays
-// are small, so each lane takes one primitive quartet of the batch and runs both recursions in
-// registers (every step and index fixed at compile time from the class's step table); after
-// each batch the lanes' weighted [e0|f0] values are summed over the warp (a transpose through
-// shared memory, 32 entries at a time) into the entry's owner lane.  Pair records, the horizontal recursion and the contraction are
-// those of k_grad_2e.
-template <typename S, int O>
-__device__ __forceinline__ void b2g_vrr_lane_op(double *v, const double *X, const double *Y, double hb, double rb,
-                                                const double *Xk, const double *Yk, double hk, double rk, double h3) {
-  constexpr B2gOp op = S::op(O);
-  if constexpr (op.mmax >= 0) {
-    constexpr bool bra = O < S::NOB;
-    const double x = bra ? X[op.dd] : Xk[op.dd], y = bra ? Y[op.dd] : Yk[op.dd];
-    const double c = (double)op.c1 * (bra ? hb : hk), r = bra ? rb : rk, c3 = (double)op.c3 * h3;
-#pragma unroll
-    for (int m = 0; m <= op.mmax; ++m) {
-      double t = x * v[op.s1 + m] + y * v[op.s1 + m + 1];
-      if constexpr (op.s2 >= 0) t += c * (v[op.s2 + m] - r * v[op.s2 + m + 1]);
-      if constexpr (op.s3 >= 0) t += c3 * v[op.s3 + m + 1];
-      v[op.dst + m] = t;
-    }
-  }
-}
-template <typename S, int... O>
-__device__ __forceinline__ void b2g_vrr_lane(double *v, const double *X, const double *Y, double hb, double rb,
-                                             const double *Xk, const double *Yk, double hk, double rk, double h3,
-                                             std::integer_sequence<int, O...>) {
-  (b2g_vrr_lane_op<S, O>(v, X, Y, hb, rb, Xk, Yk, hk, rk, h3), ...);
-}
-__device__ __forceinline__ double b2g_warp_sum(double x) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-  return x;
-}
+// host tables of the slice kernels and their device copies (one scratch block, freed in stream
+// order): super shells, molecules, prefixes of the pairs, of the six two-electron classes' tasks
+// (order as launched) and of the one-electron slices
+struct B2gsTables {
+  void *block = nullptr;
+  const B2gSuper *su = nullptr;
+  const B2gsMol *gm = nullptr;
+  const long long *off = nullptr;                 // [8][nmol + 1]
+  B2gPrim *pr = nullptr;
+  unsigned char *pn = nullptr;
+  long long n[8];                                 // totals: pairs, classes 0..5, one-electron
+};
+static const int b2gs_tb[6] = {2, 2, 2, 1, 1, 0}, b2gs_tk[6] = {2, 1, 0, 1, 0, 0};
 
-template <int G>
-__global__ void __launch_bounds__(128)
-k_grad_2e_l(const B2EriTask *__restrict__ tasks, long long ntask, const B2MolDev *__restrict__ mols,
-            const B2PairInfo *__restrict__ pinfo, const int *__restrict__ cls_list,
-            const B2Shell *__restrict__ shells, const double *__restrict__ btab, const double *__restrict__ D,
-            double hyb, double *__restrict__ grad) {
-  using C2 = B2g2e<G>;
-  constexpr int LA = C2::LA, LB = C2::LB, LC = C2::LC, LD = C2::LD, L = C2::L;
-  static_assert(L <= 3, "per-lane form: small classes only");
-  constexpr int na = 2 * LA + 1, nb = 2 * LB + 1, nc = 2 * LC + 1, nd = 2 * LD + 1, NCMP = na * nb * nc * nd;
-  using SB = typename C2::SB;
-  using SK = typename C2::SK;
-  constexpr int NTOT = 3 * SB::NACC + 2 * SK::NACC, NCH = (NTOT + 31) / 32;
-  constexpr int PER_WARP = NTOT + 2 * B2_MAXPRIM * B2_MAXPRIM * B2G_PP + 32 * 33;
-  __shared__ double sbuf[4][PER_WARP];
-  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long ti = (long long)blockIdx.x * 4 + w;
-  if (ti >= ntask) return;                        // whole warp
-  double *acc = sbuf[w], *bpr = acc + NTOT, *kpr = bpr + B2_MAXPRIM * B2_MAXPRIM * B2G_PP;
-  double *red = kpr + B2_MAXPRIM * B2_MAXPRIM * B2G_PP;
-  const B2EriTask tk = tasks[ti];
-  const B2MolDev md = mols[tk.mol];
-  const B2PairInfo bp = pinfo[md.sp_off + tk.IJ];
-  const B2Shell &a = shells[md.sh_off + bp.I], &b = shells[md.sh_off + bp.J];
-  const double *Dm = D + md.mat_off;
-  const int N = md.nao;
-  double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};
-  double AB[3], AB2 = 0;
-  for (int x = 0; x < 3; ++x) { AB[x] = a.R[x] - b.R[x]; AB2 += AB[x] * AB[x]; }
-  const int nbp = b2g_pairs_warp(a, b, AB2, bpr, lane);
-  double *gm = grad + 3ll * md.atm_off;
-  for (int kq = 0; kq < tk.count; ++kq) {
-    const int KL = cls_list[md.sp_off + md.cls_start[tk.cls] + tk.start + kq];
-    if (KL > tk.IJ) continue;                     // uniform over the warp
-    const B2PairInfo kp = pinfo[md.sp_off + KL];
-    const B2Shell &c = shells[md.sh_off + kp.I], &d = shells[md.sh_off + kp.J];
-    double CD[3], CD2 = 0;
-    for (int x = 0; x < 3; ++x) { CD[x] = c.R[x] - d.R[x]; CD2 += CD[x] * CD[x]; }
-    const int nkp = b2g_pairs_warp(c, d, CD2, kpr, lane);
-    double accu[NCH];                             // owner-lane sums: entry u = 32 k + lane
-#pragma unroll
-    for (int k = 0; k < NCH; ++k) accu[k] = 0.0;
-    const int ncombo = nbp * nkp;
-    for (int c0 = 0; c0 < ncombo; c0 += 32) {
-      const int cb = c0 + lane;
-      double vb[SB::NV], vk[SK::NV];
-      double al2 = 0, be2 = 0, ga2 = 0;
-      if (cb < ncombo) {
-        const int ib = cb / nkp, ik = cb - (cb / nkp) * nkp;
-        const double *B = bpr + ib * B2G_PP, *K = kpr + ik * B2G_PP;
-        const double z = B[2], e = K[2], iz = B[10], ie = K[10];
-        const double rs = rsqrt(z + e), inv = rs * rs;          // 1/sqrt(zeta+eta), 1/(zeta+eta)
-        double PA[3], QC[3], WP[3], WQ[3], PQ2 = 0;
-        for (int x = 0; x < 3; ++x) {
-          const double P = B[3 + x], Q = K[3 + x];
-          const double W = (z * P + e * Q) * inv;
-          PA[x] = B[6 + x];
-          QC[x] = K[6 + x];
-          WP[x] = W - P;
-          WQ[x] = W - Q;
-          PQ2 += (P - Q) * (P - Q);
-        }
-        const double rho = z * e * inv;
-        const double pref = 34.98683665524972 * iz * ie * rs * B[9] * K[9];   // 2 pi^(5/2) / (z e sqrt(z+e)) K K
-        double F[L + 1];
-        b2_boys<double, L, double>(rho * PQ2, btab, F);
-        const double hb = 0.5 * iz, rb = e * inv, hk = 0.5 * ie, rk = z * inv, h3 = 0.5 * inv;
-#pragma unroll
-        for (int m = 0; m <= L; ++m) vb[m] = vk[m] = pref * F[m];
-        b2g_vrr_lane<SB>(vb, PA, WP, hb, rb, QC, WQ, hk, rk, h3, std::make_integer_sequence<int, SB::NOP>{});
-        b2g_vrr_lane<SK>(vk, PA, WP, hb, rb, QC, WQ, hk, rk, h3, std::make_integer_sequence<int, SK::NOP>{});
-        al2 = 2.0 * B[0];
-        be2 = 2.0 * B[1];
-        ga2 = 2.0 * K[0];
-      } else {
-#pragma unroll
-        for (int t = 0; t < SB::NV; ++t) vb[t] = 0.0;
-#pragma unroll
-        for (int t = 0; t < SK::NV; ++t) vk[t] = 0.0;
-      }
-      // weighted values of every entry u summed over the batch's quartets -> owner lane u % 32:
-      // 32 entries at a time through a 32 x 33 shared-memory transpose (lane = row)
-#pragma unroll
-      for (int ch = 0; ch < NCH; ++ch) {
-#pragma unroll
-        for (int jj = 0; jj < 32; ++jj) {
-          const int u = 32 * ch + jj;
-          if (u < NTOT) {
-            double x;
-            if (u < 3 * SB::NACC) {
-              const int q = u / SB::NACC, t = u - q * SB::NACC;
-              x = vb[(t / SB::NF) * SB::SE + (t % SB::NF) * SB::SM] * (q == 0 ? 1.0 : (q == 1 ? al2 : be2));
-            } else {
-              const int q = (u - 3 * SB::NACC) / SK::NACC, t = u - 3 * SB::NACC - q * SK::NACC;
-              x = vk[(t / SK::NF) * SK::SE + (t % SK::NF) * SK::SM] * (q == 0 ? 1.0 : ga2);
-            }
-            red[lane * 33 + jj] = x;
-          }
-        }
-        __syncwarp();
-        if (32 * ch + lane < NTOT) {
-          double sum = 0.0;
-#pragma unroll 8
-          for (int r = 0; r < 32; ++r) sum += red[r * 33 + lane];
-          accu[ch] += sum;
-        }
-        __syncwarp();
-      }
+static int b2gs_tables(const B2PlanDev &P, B2gsTables &T, cudaStream_t st) {
+  const int nmol = P.h.nmol;
+  std::vector<B2gSuper> su;
+  std::vector<B2gsMol> gm(nmol);
+  std::vector<long long> off(8ll * (nmol + 1), 0);
+  su.reserve(P.h.n_sh);
+  std::vector<B2gSuper> tmp(std::max(1, P.h.max_nbas));
+  for (int m = 0; m < nmol; ++m) {
+    const B2MolDev &md = P.h.mols[m];
+    int nt = 0;
+    const int ns = b2gs_supers(P.h.shells.data() + md.sh_off, md.nbas, tmp.data(), &nt), np = nt - ns;
+    gm[m] = B2gsMol{ns, np, (int)su.size(), 0, off[m]};
+    su.insert(su.end(), tmp.begin(), tmp.begin() + nt);
+    long long *o = off.data() + m;
+    o[1] = o[0] + b2gs_npair(ns, np);
+    int all = 0;
+    for (int t = 0; t < 3; ++t) all += b2gs_nslice(ns, np, t);
+    for (int c = 0; c < 6; ++c) {
+      long long *q = o + (c + 1) * (nmol + 1ll);
+      q[1] = q[0] + (long long)b2gs_nslice(ns, np, b2gs_tb[c]) * ((b2gs_nket(ns, np, b2gs_tk[c]) + 31) / 32);
     }
-#pragma unroll
-    for (int k = 0; k < NCH; ++k) {
-      const int u = 32 * k + lane;
-      if (u < NTOT) acc[u] = accu[k];
-    }
-    __syncwarp();
-    const auto *aB = reinterpret_cast<const double (*)[SB::NE][SB::NF]>(acc);
-    const auto *aK = reinterpret_cast<const double (*)[SK::NE][SK::NF]>(acc + 3 * SB::NACC);
-    const double deg = (bp.I == bp.J ? 1.0 : 2.0) * (kp.I == kp.J ? 1.0 : 2.0) * (KL == tk.IJ ? 1.0 : 2.0);
-    double gC[3] = {0, 0, 0}, g3[3] = {0, 0, 0};
-    for (int cmp = lane; cmp < NCMP; cmp += 32) {
-      const int id = cmp % nd, ic = (cmp / nd) % nc, ib = (cmp / (nd * nc)) % nb, ia = cmp / (nd * nc * nb);
-      const int i = a.ao0 + ia, j = b.ao0 + ib, k = c.ao0 + ic, l = d.ao0 + id;
-      const double gmv = deg * (0.5 * Dm[i * N + j] * Dm[k * N + l] -
-                                0.125 * hyb * (Dm[i * N + l] * Dm[j * N + k] + Dm[i * N + k] * Dm[j * N + l]));
-      if (gmv == 0.0) continue;
-      int ea[3], eb[3], ec[3], ed[3];
-      b2g_comp(LA, ia, ea); b2g_comp(LB, ib, eb); b2g_comp(LC, ic, ec); b2g_comp(LD, id, ed);
-      for (int x = 0; x < 3; ++x) {
-        int up[3], dn[3];
-        for (int q = 0; q < 3; ++q) { up[q] = ea[q] + (q == x); dn[q] = ea[q] - (q == x); }
-        double dA = b2g_hrr(aB, 1, up, eb, ec, ed, AB, CD);
-        if (ea[x]) dA -= (double)ea[x] * b2g_hrr(aB, 0, dn, eb, ec, ed, AB, CD);
-        for (int q = 0; q < 3; ++q) { up[q] = eb[q] + (q == x); dn[q] = eb[q] - (q == x); }
-        double dB = b2g_hrr(aB, 2, ea, up, ec, ed, AB, CD);
-        if (eb[x]) dB -= (double)eb[x] * b2g_hrr(aB, 0, ea, dn, ec, ed, AB, CD);
-        for (int q = 0; q < 3; ++q) { up[q] = ec[q] + (q == x); dn[q] = ec[q] - (q == x); }
-        double dC = b2g_hrr(aK, 1, ea, eb, up, ed, AB, CD);
-        if (ec[x]) dC -= (double)ec[x] * b2g_hrr(aK, 0, ea, eb, dn, ed, AB, CD);
-        gA[x] += gmv * dA;
-        gB[x] += gmv * dB;
-        gC[x] += gmv * dC;
-        g3[x] -= gmv * (dA + dB + dC);
-      }
-    }
-    for (int x = 0; x < 3; ++x) {
-      const double u = b2g_warp_sum(gC[x]), t = b2g_warp_sum(g3[x]);
-      if (lane == 0) {
-        atomicAdd(gm + 3 * c.atom + x, u);
-        atomicAdd(gm + 3 * d.atom + x, t);
-      }
-    }
-    __syncwarp();                                 // acc and the pair records are rewritten next
+    long long *q = o + 7 * (nmol + 1ll);
+    q[1] = q[0] + all;
   }
-  for (int x = 0; x < 3; ++x) {
-    const double u = b2g_warp_sum(gA[x]), t = b2g_warp_sum(gB[x]);
-    if (lane == 0) {
-      atomicAdd(gm + 3 * a.atom + x, u);
-      atomicAdd(gm + 3 * b.atom + x, t);
-    }
-  }
-}
-
-template <int G>
-static int b2g_launch_2e(const B2PlanDev &P, const double *D, double hyb, double *grad, cudaStream_t st) {
-  const long long t0 = P.eri_goff32[G], n = P.eri_goff32[G + 1] - t0;
-  if constexpr (B2g2e<G>::L <= 3) {
-    if (n > 0) {
-      k_grad_2e_l<G><<<(unsigned)((n + 3) / 4), 128, 0, st>>>(P.eri_tasks32 + t0, n, P.mols, P.pinfo, P.cls_list,
-                                                             P.shells, P.boys, D, hyb, grad);
-      b2_count_launches(1);
-    }
-  } else if (n > 0) {
-    static bool attr[8] = {false};                 // per device: shared memory above 48 KB
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 8) return B2_ERR_CUDA;
-    if (!attr[dev]) {
-      if (cudaFuncSetAttribute(k_grad_2e<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B2g2e<G>::SMEM) !=
-          cudaSuccess)
-        return B2_ERR_CUDA;
-      attr[dev] = true;
-    }
-    k_grad_2e<G><<<(unsigned)((n + 3) / 4), 128, B2g2e<G>::SMEM, st>>>(P.eri_tasks32 + t0, n, P.mols, P.pinfo,
-                                                                       P.cls_list, P.shells, P.boys, D, hyb, grad);
+  for (int k = 0; k < 8; ++k) T.n[k] = off[k * (nmol + 1ll) + nmol];
+  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+  const size_t b0 = up(sizeof(B2gSuper) * su.size()), b1 = up(sizeof(B2gsMol) * gm.size()),
+               b2 = up(sizeof(long long) * off.size()), b3 = up(sizeof(B2gPrim) * B2_MAXPP * (size_t)T.n[0]);
+  unsigned char *d = nullptr;
+  B2_CUDA_TRY(b2_dmalloc_t(&d, b0 + b1 + b2 + b3 + (size_t)T.n[0], st));
+  T.block = d;
+  T.su = reinterpret_cast<B2gSuper *>(d);
+  T.gm = reinterpret_cast<B2gsMol *>(d + b0);
+  T.off = reinterpret_cast<long long *>(d + b0 + b1);
+  T.pr = reinterpret_cast<B2gPrim *>(d + b0 + b1 + b2);
+  T.pn = d + b0 + b1 + b2 + b3;
+  std::vector<unsigned char> h(b0 + b1 + b2);
+  std::memcpy(h.data(), su.data(), sizeof(B2gSuper) * su.size());
+  std::memcpy(h.data() + b0, gm.data(), sizeof(B2gsMol) * gm.size());
+  std::memcpy(h.data() + b0 + b1, off.data(), sizeof(long long) * off.size());
+  // pageable source: the call returns once the data is staged, so h may go out of scope
+  B2_CUDA_TRY(cudaMemcpyAsync(d, h.data(), h.size(), cudaMemcpyHostToDevice, st));
+  if (T.n[0] > 0) {
+    k_gs_prims<<<(unsigned)((T.n[0] + 127) / 128), 128, 0, st>>>(T.gm, T.off, nmol, T.su, T.pr, T.pn);
     b2_count_launches(1);
   }
-  if constexpr (G < 15) return b2g_launch_2e<G + 1>(P, D, hyb, grad, st);
+  B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
+}
+
+// resident CTAs of 4 warps, tasks strided over them
+static unsigned b2gs_grid(long long ntask) { return (unsigned)std::min<long long>((ntask + 3) / 4, 148ll * 8); }
+
+template <int C>
+static int b2gs_launch_2e(const B2PlanDev &P, const B2gsTables &T, const double *D, double hyb, double *grad,
+                          cudaStream_t st) {
+  constexpr int TB = C < 3 ? 2 : (C < 5 ? 1 : 0), TK = C == 0 ? 2 : (C == 1 || C == 3 ? 1 : 0);
+  const long long n = T.n[C + 1];
+  if (n > 0) {
+    const size_t smem = sizeof(double) * B2GS_TABLE + 4 * sizeof(B2gsWarp);
+    B2_CUDA_TRY(cudaFuncSetAttribute(k_grad_sp<TB, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_grad_sp<TB, TK><<<b2gs_grid(n), 128, smem, st>>>(T.off + (C + 1) * (P.h.nmol + 1ll), P.h.nmol, T.gm, P.mols,
+                                                        T.su, T.pr, T.pn, P.boys, D, hyb, grad);
+    b2_count_launches(1);
+  }
+  return B2_OK;
+}
+
+// the six two-electron classes and the one-electron part side by side on the plan's streams
+// (forked from and joined back to `st`): every kernel adds to grad with atomics
+static int b2gs_launch(const B2PlanDev &P, const B2gsTables &T, int parts, double hyb, const double *D,
+                       const double *W, double *grad, cudaStream_t st) {
+  const bool fork = P.bkt_stream[0] != nullptr;
+  cudaStream_t s[B2_NBKT];
+  if (fork) B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
+  for (int b = 0; b < B2_NBKT; ++b) {
+    s[b] = fork ? P.bkt_stream[b] : st;
+    if (fork) B2_CUDA_TRY(cudaStreamWaitEvent(s[b], P.bkt_ev[B2_NBKT], 0));
+  }
+  int rc = B2_OK;
+  if (parts & 2) {
+    rc = b2gs_launch_2e<0>(P, T, D, hyb, grad, s[0]);
+    if (!rc) rc = b2gs_launch_2e<1>(P, T, D, hyb, grad, s[1]);
+    if (!rc) rc = b2gs_launch_2e<3>(P, T, D, hyb, grad, s[2]);
+    if (!rc) rc = b2gs_launch_2e<4>(P, T, D, hyb, grad, s[3]);
+    if (!rc) rc = b2gs_launch_2e<2>(P, T, D, hyb, grad, s[4]);
+    if (!rc) rc = b2gs_launch_2e<5>(P, T, D, hyb, grad, s[2]);
+  }
+  if (!rc && (parts & 1) && T.n[7] > 0) {
+    k_grad_1e<<<b2gs_grid(T.n[7]), 128, sizeof(double) * B2GS_TABLE, s[0]>>>(
+        T.off + 7 * (P.h.nmol + 1ll), P.h.nmol, T.gm, P.mols, T.su, T.pr, T.pn, P.atom_xyz, P.atom_z, P.boys, D, W,
+        grad);
+    b2_count_launches(1);
+  }
+  if (fork)
+    for (int b = 0; b < B2_NBKT; ++b) {
+      cudaEventRecord(P.bkt_ev[b], s[b]);
+      cudaStreamWaitEvent(st, P.bkt_ev[b], 0);
+    }
+  if (!rc) B2_CUDA_TRY(cudaGetLastError());
+  return rc;
 }
 
 int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const double *mo_energy,
@@ -794,14 +661,11 @@ int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const d
     k_grad_dm<<<nmol, 256, 0, st>>>(P.mols, C, mo_energy, D, W);
     b2_count_launches(1);
   }
-  if (parts & 1) {
-    k_grad_1e<<<nmol, 128, 0, st>>>(P.mols, P.shells, P.atom_xyz, P.atom_z, P.boys, D, W, grad);
-    b2_count_launches(1);
-  }
-  if (parts & 2) {
-    int rc = b2_eri_tasks_ready(P, 32, st);        // canonical quartets grouped by class
-    if (rc) return rc;
-    rc = b2g_launch_2e<0>(P, D, hyb, grad, st);     // the 16 class combinations
+  if (parts & 3) {
+    B2gsTables T;
+    int rc = b2gs_tables(P, T, st);
+    if (!rc) rc = b2gs_launch(P, T, parts, hyb, D, W, grad, st);
+    b2_dfree(T.block, st);
     if (rc) return rc;
   }
   if (parts & 4) {

@@ -4,6 +4,7 @@
 // It is never loaded by the product path (libb200dft.so has no CPU fallback).
 #include "eri_sq.cuh"
 #include "grad_math.cuh"
+#include "grad_sp.cuh"
 #include "xc_math.cuh"
 #include <algorithm>
 #include <vector>
@@ -136,6 +137,133 @@ static void b2hc_vrr_all(const double *tab, double *rel) {
   rel[2 * G] = b2hc_vrr_table<LA + LB + 1, LC + LD, false>(sh[0], sh[1], sh[2], sh[3], tab);
   rel[2 * G + 1] = b2hc_vrr_table<LA + LB, LC + LD + 1, true>(sh[0], sh[1], sh[2], sh[3], tab);
   if constexpr (G < 15) b2hc_vrr_all<G + 1>(tab, rel);
+}
+
+// The super-shell form of the two-electron gradient (grad_sp.cuh) on the host: slice quartets in
+// the GPU kernels' order, every primitive quartet through the code the kernels run.
+template <int TB, int TK, int KF>
+static void b2hc_gs_ket(const B2gBraRec *bra, int nb, const double *AB, int f, int F, const int *bi,
+                        const std::vector<B2gPrim> &kp, const B2gSuper &c, const B2gSuper &d, double wt,
+                        const double *D, int N, double hyb, const double *tab, double g[4][3]) {
+  using C = B2gsClass<TB, TK>;
+  const int F2 = TK == 2 ? (c.ao_p < 0 ? -1 : c.ao_p + (f + KF) % 3) : c.ao_s;
+  int di[4] = {d.ao_s, -1, -1, -1};
+  double CD[3], pA[3] = {0, 0, 0}, pB[3] = {0, 0, 0}, pC[3] = {0, 0, 0}, pD[3] = {0, 0, 0};
+  for (int k = 0; k < 3; ++k) {
+    if (TK && d.ao_p >= 0) di[1 + k] = d.ao_p + (f + k) % 3;
+    CD[k] = c.R[(f + k) % 3] - d.R[(f + k) % 3];
+  }
+  for (const B2gPrim &r : kp) {
+    B2gKet<C::NB, C::NK> q;
+    double QD[3], Q[3];
+    for (int k = 0; k < 3; ++k) { QD[k] = r.ra * CD[k]; Q[k] = r.P[(f + k) % 3]; }
+    b2gs_ket<C::NB, C::NK>(D, N, hyb, wt, F, bi, F2, di, TK == 2 ? r.kps : r.kss, TK == 2 ? r.kpp : r.ksp, QD, q);
+    q.v = r.u;
+    q.FC = (r.ra - 1.0) * CD[KF < 0 ? 0 : KF];
+    for (int p = 0; p < nb; ++p) {
+      B2gOut o;
+      b2gs_eval<TB, TK, KF>(bra[p], q, Q, r.z, tab, o);
+      b2gs_add_bra<TB>(bra[p], AB, o, pA, pB);
+      b2gs_add_ket<TK, KF>(r.ra, r.mu2, CD, o, pC, pD);
+    }
+  }
+  for (int k = 0; k < 3; ++k) {
+    const int x = (f + k) % 3;
+    g[0][x] += pA[k]; g[1][x] += pB[k]; g[2][x] += pC[k]; g[3][x] += pD[k];
+  }
+}
+
+template <int TB, int TK>
+static void b2hc_gs_class(const std::vector<B2gSuper> &S, int ns, int np, const double *D, int N, double hyb,
+                          const double *tab, double *g) {
+  auto prims = [&](const B2gSuper &a, const B2gSuper &b) {
+    std::vector<B2gPrim> v;
+    for (int p = 0; p < a.nprim; ++p)
+      for (int q = 0; q < b.nprim; ++q) {
+        B2gPrim r;
+        if (b2gs_prim(a, b, p, q, r)) v.push_back(r);
+      }
+    return v;
+  };
+  for (int i = 0; i < b2gs_nslice(ns, np, TB); ++i) {
+    const int bpr = TB == 2 ? i / 3 : i, f = TB == 2 ? i - 3 * (i / 3) : 0;
+    int A, B;
+    b2gs_pair(ns, np, b2gs_ket_pair(ns, np, TB, bpr), A, B);
+    double AB[3];
+    for (int k = 0; k < 3; ++k) AB[k] = S[A].R[(f + k) % 3] - S[B].R[(f + k) % 3];
+    B2gBraRec bra[B2_MAXPP];
+    int nb = 0;
+    for (const B2gPrim &r : prims(S[A], S[B])) b2gs_bra(r, TB, f, AB, bra[nb++]);
+    const int F = TB == 2 ? (S[A].ao_p < 0 ? -1 : S[A].ao_p + f) : S[A].ao_s;
+    int bi[4] = {S[B].ao_s, -1, -1, -1};
+    for (int k = 0; k < 3; ++k)
+      if (TB && S[B].ao_p >= 0) bi[1 + k] = S[B].ao_p + (f + k) % 3;
+    const int nk = TB == TK ? bpr + 1 : b2gs_nket(ns, np, TK);
+    for (int kk = 0; kk < nk; ++kk) {
+      int c, d;
+      b2gs_pair(ns, np, b2gs_ket_pair(ns, np, TK, kk), c, d);
+      const double wt = (A == B ? 1.0 : 2.0) * (c == d ? 1.0 : 2.0) * (TB == TK && kk == bpr ? 1.0 : 2.0);
+      double g4[4][3] = {};
+      const std::vector<B2gPrim> kp = prims(S[c], S[d]);
+      if constexpr (TK == 2) {
+        b2hc_gs_ket<TB, TK, 0>(bra, nb, AB, f, F, bi, kp, S[c], S[d], wt, D, N, hyb, tab, g4);
+        b2hc_gs_ket<TB, TK, 1>(bra, nb, AB, f, F, bi, kp, S[c], S[d], wt, D, N, hyb, tab, g4);
+        b2hc_gs_ket<TB, TK, 2>(bra, nb, AB, f, F, bi, kp, S[c], S[d], wt, D, N, hyb, tab, g4);
+      } else {
+        b2hc_gs_ket<TB, TK, -1>(bra, nb, AB, f, F, bi, kp, S[c], S[d], wt, D, N, hyb, tab, g4);
+      }
+      const int at[4] = {S[A].atom, S[B].atom, S[c].atom, S[d].atom};
+      for (int s = 0; s < 4; ++s)
+        for (int x = 0; x < 3; ++x) g[3 * at[s] + x] += g4[s][x];
+    }
+  }
+}
+
+template <int TB>
+static void b2hc_gs_one(const B2PlanHost &P, const std::vector<B2gSuper> &S, int ns, int np, const double *D,
+                        const double *W, const double *tab, double *g) {
+  constexpr int NB = TB ? 1 : 0;
+  const int N = P.mols[0].nao, natm = P.mols[0].natm;
+  for (int i = 0; i < b2gs_nslice(ns, np, TB); ++i) {
+    const int bpr = TB == 2 ? i / 3 : i, f = TB == 2 ? i - 3 * (i / 3) : 0;
+    int A, B;
+    b2gs_pair(ns, np, b2gs_ket_pair(ns, np, TB, bpr), A, B);
+    const B2gSuper &a = S[A], &b = S[B];
+    const int F = TB == 2 ? (a.ao_p < 0 ? -1 : a.ao_p + f) : a.ao_s;
+    double AB[3], dg[4] = {}, wg[4] = {}, gA[3] = {}, gB[3] = {};
+    for (int k = 0; k < (NB ? 4 : 1); ++k) {
+      const int bb = k == 0 ? b.ao_s : (b.ao_p < 0 ? -1 : b.ao_p + (f + k - 1) % 3);
+      if (F < 0 || bb < 0) continue;
+      dg[k] = (A == B ? 1.0 : 2.0) * D[F * N + bb];
+      wg[k] = -(A == B ? 1.0 : 2.0) * W[F * N + bb];
+    }
+    for (int k = 0; k < 3; ++k) AB[k] = a.R[(f + k) % 3] - b.R[(f + k) % 3];
+    for (int p = 0; p < a.nprim; ++p)
+      for (int q = 0; q < b.nprim; ++q) {
+        B2gPrim pr;
+        if (!b2gs_prim(a, b, p, q, pr)) continue;
+        B2gBraRec r;
+        b2gs_bra(pr, TB, f, AB, r);
+        double gk[3];
+        b2gs_st<TB>(r, dg, wg, AB, gk);
+        for (int k = 0; k < 3; ++k) { gA[k] += gk[k]; gB[k] -= gk[k]; }
+        for (int c = 0; c < natm; ++c) {
+          B2gKet<NB, 0> ket;
+          for (int k = 0; k < (NB ? 4 : 1); ++k)
+            ket.gs[k] = -(double)P.atom_z[c] * (6.283185307179586 / 5.914967172795613) * dg[k];
+          ket.v = ket.FC = 0;
+          const double C[3] = {P.atom_xyz[3 * c + f], P.atom_xyz[3 * c + (f + 1) % 3], P.atom_xyz[3 * c + (f + 2) % 3]};
+          B2gOut o;
+          b2gs_eval_point<TB>(r, ket, C, tab, o);
+          b2gs_add_bra<TB>(r, AB, o, gA, gB);
+          for (int k = 0; k < 3; ++k) g[3 * c + (f + k) % 3] -= o.dP[k];
+        }
+      }
+    for (int k = 0; k < 3; ++k) {
+      g[3 * a.atom + (f + k) % 3] += gA[k];
+      g[3 * b.atom + (f + k) % 3] += gB[k];
+    }
+  }
 }
 
 extern "C" {
@@ -273,6 +401,50 @@ int b2hc_grad_2e_tasks(int nmol, const int *natm, const int *nbas, const int *at
   for (int i = 0; i < 3 * P.n_atm; ++i) g[i] = 0;
   *bad = 0;
   b2hc_2e_group<0>(P, tasks, goff, D, hyb, tab.data(), g, bad);
+  return 0;
+}
+
+// one-electron gradient of one molecule at fixed D and W by the super-shell form (grad_sp.cuh)
+int b2hc_grad_1e_super(int natm, int nbas, const int *atm, const int *bas, const double *env, const double *D,
+                       const double *W, double *g) {
+  B2PlanHost P;
+  const long long eo = 0;
+  int rc = b2_plan_build(P, 1, &natm, &nbas, atm, bas, env, &eo);
+  if (rc) return rc;
+  std::vector<double> tab(B2_BOYS_NT * B2_BOYS_NM);
+  b2_boys_fill_table(tab.data());
+  for (int i = 0; i < 3 * natm; ++i) g[i] = 0;
+  std::vector<B2gSuper> S(nbas);
+  int nt = 0;
+  const int ns = b2gs_supers(P.shells.data(), nbas, S.data(), &nt), np = nt - ns;
+  b2hc_gs_one<0>(P, S, ns, np, D, W, tab.data(), g);
+  b2hc_gs_one<1>(P, S, ns, np, D, W, tab.data(), g);
+  b2hc_gs_one<2>(P, S, ns, np, D, W, tab.data(), g);
+  return 0;
+}
+
+// two-electron gradient of one molecule at fixed D by the super-shell form (grad_sp.cuh)
+int b2hc_grad_2e_super(int natm, int nbas, const int *atm, const int *bas, const double *env, const double *D,
+                       double hyb, double *g, int *counts) {
+  B2PlanHost P;
+  const long long eo = 0;
+  int rc = b2_plan_build(P, 1, &natm, &nbas, atm, bas, env, &eo);
+  if (rc) return rc;
+  const int N = P.mols[0].nao;
+  std::vector<double> tab(B2_BOYS_NT * B2_BOYS_NM);
+  b2_boys_fill_table(tab.data());
+  for (int i = 0; i < 3 * natm; ++i) g[i] = 0;
+  std::vector<B2gSuper> S(nbas);
+  int nt = 0;
+  const int ns = b2gs_supers(P.shells.data(), nbas, S.data(), &nt), np = nt - ns;
+  counts[0] = ns;
+  counts[1] = np;
+  b2hc_gs_class<0, 0>(S, ns, np, D, N, hyb, tab.data(), g);
+  b2hc_gs_class<1, 0>(S, ns, np, D, N, hyb, tab.data(), g);
+  b2hc_gs_class<1, 1>(S, ns, np, D, N, hyb, tab.data(), g);
+  b2hc_gs_class<2, 0>(S, ns, np, D, N, hyb, tab.data(), g);
+  b2hc_gs_class<2, 1>(S, ns, np, D, N, hyb, tab.data(), g);
+  b2hc_gs_class<2, 2>(S, ns, np, D, N, hyb, tab.data(), g);
   return 0;
 }
 

@@ -88,3 +88,39 @@ def test_nanodft_grad_drop_in_matches_oracle():
     ref = ograd.gradient(mol, mo_coeff, mo_energy, coords, weights)
     assert np.abs(ref).max() > 1e-2
     np.testing.assert_allclose(g, ref, atol=1e-6, rtol=0)     # oracle truncation ~1e-8
+
+
+@pytest.mark.parametrize("heavy, odd", [(1, True), (2, False), (4, True), (9, False)])
+def test_gradient_slices_over_sizes(heavy, odd):
+    """two- and one-electron parts against the host build of the same slices: one to several
+    32-ket chunks per class, 8 / 16 / 32 lanes of nuclei, shells off the STO-3G pattern, a random
+    density.  Same formulas in another order of float64 sums: 1e-10 of the largest component."""
+    import torch
+    from test_hostcheck import _gs_args, _hc, _p, odd_shells
+    from b200dft.engine import Plan
+    from b200dft._lib import check, lib, ptr, stream_handle
+    from b200dft.molgen import random_molecule
+    mol = Mole(random_molecule(np.random.default_rng(heavy), heavy))
+    mol = odd_shells(mol) if odd else mol
+    hc, N = _hc(), mol.nao
+    rng = np.random.default_rng(5)
+    D, W = (np.ascontiguousarray(a + a.T) for a in rng.normal(size=(2, N, N)) * 0.3)
+    plan = Plan([mol])
+    try:
+        t = lambda a: torch.from_numpy(a.reshape(-1)).cuda()
+        d, w = t(D), t(W)
+        got = []
+        for parts in (1, 2):
+            g = torch.full((mol.natm, 3), float("nan"), dtype=torch.float64, device="cuda")
+            check(lib().b2_grad(plan.h, parts, HYB, None, None, None, None, ptr(d), ptr(w), ptr(g), stream_handle()),
+                  "b2_grad")
+            got.append(g.cpu().numpy())
+    finally:
+        plan.close()
+    ref1, ref2, n = np.zeros((mol.natm, 3)), np.zeros((mol.natm, 3)), np.zeros(2, np.int32)
+    keep, a = _gs_args(mol, D, W)
+    assert hc.b2hc_grad_1e_super(*a, _p(ref1, ctypes.c_double)) == 0
+    keep, a = _gs_args(mol, D)
+    assert hc.b2hc_grad_2e_super(*a, ctypes.c_double(HYB), _p(ref2, ctypes.c_double), _p(n, ctypes.c_int)) == 0
+    for g, ref in zip(got, (ref1, ref2)):
+        np.testing.assert_allclose(g, ref, atol=1e-10 * max(1.0, np.abs(ref).max()), rtol=0)

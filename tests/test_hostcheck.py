@@ -279,3 +279,56 @@ def test_gradient_math_compiles_for_sm100a(tmp_path):
                         "--expt-relaxed-constexpr", "-I", csrc, "-c", str(src), "-o", str(tmp_path / "k.o")],
                        capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+def odd_shells(mol):
+    """the molecule with shells off the STO-3G pattern: the first heavy atom's p shell on its own
+    exponents (no s partner), the last hydrogen's s shell cut to one primitive and, if there is
+    another, one cut to two"""
+    m = Mole.__new__(Mole)
+    m.__dict__.update(mol.__dict__)
+    bas, env = mol._bas.copy(), mol._env
+    p = int(np.where(bas[:, 1] == 1)[0][0])
+    env = np.concatenate([env, env[bas[p, 5]:bas[p, 5] + 3] * 1.07])
+    bas[p, 5] = len(mol._env)
+    s = [k for k in range(len(bas)) if mol.charges[bas[k, 0]] == 1]
+    for k, n in zip(s[::-1], (1, 2)):
+        bas[k, 2] = n
+    m._bas, m._env = bas, env
+    return m
+
+
+def _gs_args(mol, *mats):
+    atm = np.ascontiguousarray(mol._atm, np.int32)
+    bas = np.ascontiguousarray(mol._bas, np.int32)
+    env = np.ascontiguousarray(mol._env, np.float64)
+    return (atm, bas, env), (mol.natm, len(bas), _p(atm, ctypes.c_int), _p(bas, ctypes.c_int),
+                             _p(env, ctypes.c_double)) + tuple(_p(a, ctypes.c_double) for a in mats)
+
+
+@pytest.mark.parametrize("atom, odd, counts", [
+    ("H 0 0 0; H 0 0.1 0.74", False, (2, 0)),                                      # s shells only
+    ("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7532 -0.4792", False, (3, 1)),
+    ("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7532 -0.4792", True, (4, 1)),       # p without its s
+    ("N 0 0 0; C 0 0 1.4; H 0.9 0.2 -0.4; H -0.6 0.7 -0.3; H 0.8 0.6 1.8", True, (6, 2)),
+])
+def test_gradient_super_shell_form(atom, odd, counts):
+    """the GPU gradient's super-shell slices (grad_sp.cuh: every class, 2s/2p merged or not, one to
+    three primitives) against the Obara-Saika forms on random symmetric D and W.  Both are float64
+    sums of terms up to ~1e2 that cancel to ~1: 1e-12 of the largest component is ~1e4 roundings."""
+    hc = _hc()
+    mol = Mole(atom)
+    mol = odd_shells(mol) if odd else mol
+    N = mol.nao
+    rng = np.random.default_rng(7)
+    D, W = (np.ascontiguousarray(a + a.T) for a in rng.normal(size=(2, N, N)) * 0.3)
+    keep, a = _gs_args(mol, D)
+    g, gs, n = np.zeros((mol.natm, 3)), np.zeros((mol.natm, 3)), np.zeros(2, np.int32)
+    assert hc.b2hc_grad_2e(*a, ctypes.c_double(0.2), _p(g, ctypes.c_double)) == 0
+    assert hc.b2hc_grad_2e_super(*a, ctypes.c_double(0.2), _p(gs, ctypes.c_double), _p(n, ctypes.c_int)) == 0
+    assert tuple(n) == counts
+    np.testing.assert_allclose(gs, g, atol=1e-12 * max(1.0, np.abs(g).max()), rtol=0)
+    keep, a = _gs_args(mol, D, W)
+    assert hc.b2hc_grad_1e(*a, _p(g, ctypes.c_double)) == 0
+    assert hc.b2hc_grad_1e_super(*a, _p(gs, ctypes.c_double)) == 0
+    np.testing.assert_allclose(gs, g, atol=1e-12 * max(1.0, np.abs(g).max()), rtol=0)
