@@ -17,7 +17,7 @@ import numpy as np
 
 from .constants import HARTREE_TO_EV, HYB_B3LYP
 from .mole import Mole, methane
-from .engine import RKSEngine, HostSetup
+from .engine import RKSEngine, drop_in_setup
 
 hartree_to_eV = 27.2114        # dft.py:47
 mol = None
@@ -56,9 +56,10 @@ def density_functional_theory(atom_positions, args, mf_diis_space=9):
             raise ValueError(f"-{flag} (a timing switch that skips or randomises work) is not supported")
     if mol is None:
         raise RuntimeError("set b200dft.dft.mol (jax_dft does) before calling")
-    setup = HostSetup(mol, level=args.level)
-    eng = RKSEngine([mol], precision="mixed" if args.float32 else "fp64", setups=[setup])
+    eng = RKSEngine([mol], level=args.level, precision="mixed" if args.float32 else "fp64",
+                    setups=drop_in_setup(mol, args.level))
     try:
+        L_inv = eng.setup_arrays()[1]
         if getattr(args, "density_mixing", False):
             res = _run_mixing(eng, args.its, not args.skipdiis)
         else:
@@ -75,7 +76,7 @@ def density_functional_theory(atom_positions, args, mf_diis_space=9):
     mask = np.zeros(N)
     mask[:nocc] = 1
     eigenvalues = res["mo_energy"][-1, 0, :N]
-    return e, e[-1], eigenvalues, C * mask[None, :], dms, setup.L_inv
+    return e, e[-1], eigenvalues, C * mask[None, :], dms, L_inv
 
 
 def _run_mixing(eng, its, use_diis):

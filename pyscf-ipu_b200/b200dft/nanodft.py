@@ -12,7 +12,7 @@ import numpy as np
 from .constants import HARTREE_TO_EV, HYB_B3LYP, EPSILON_B3LYP
 from .mole import Mole, build_mol, methane
 from .grids import Grids
-from .engine import RKSEngine, HostSetup
+from .engine import RKSEngine, drop_in_setup
 
 __all__ = ["nanoDFT", "nanoDFT_options", "build_mol", "energy", "hlgap", "process_mol_str", "grad"]
 
@@ -74,11 +74,12 @@ def nanoDFT(mol, opts):
         raise NotImplementedError("structure optimisation is outside the SCF hot path")
     # ao_threshold > 0: AO values below it are zeroed and grid points left without any are
     # dropped (nanoDFT.py:221-230); the SCF then reads those stored AO values
-    setup = HostSetup(mol, level=opts.level, ao_threshold=opts.ao_threshold or 0.0)
+    setups = drop_in_setup(mol, opts.level, opts.ao_threshold or 0.0)
     # eri_threshold > 0: s8 entries with |v| <= it are zeroed before J/K (nanoDFT.py:280-288)
-    eng = RKSEngine([mol], precision="mixed" if opts.float32 else "fp64", setups=[setup],
+    eng = RKSEngine([mol], level=opts.level, precision="mixed" if opts.float32 else "fp64", setups=setups,
                     eri_threshold=opts.eri_threshold or 0.0)
     try:
+        Hcore, _, E_nuc, coords, weights = eng.setup_arrays()
         res = eng.run(its=opts.its, use_diis=opts.diis, log=True)
     finally:
         eng.close()
@@ -91,13 +92,13 @@ def nanoDFT(mol, opts):
     energies = np.zeros((its, 5))
     hlgaps = np.zeros(its)
     for i in range(its):
-        energies[i] = energy(D[i], setup.Hcore, diffJK[i], logged[i, 3], setup.E_nuc)
+        energies[i] = energy(D[i], Hcore, diffJK[i], logged[i, 3], E_nuc)
         mo_i = res["mo_energy"][i, 0, :N]
         hlgaps[i] = abs(mo_i[nocc] - mo_i[nocc - 1])
     mo_energy = res["mo_energy"][-1, 0, :N]
     mo_coeff = res["C"][:N * N].reshape(N, N)
     energies, logged, hlgaps = [a * HARTREE_TO_EV for a in (energies, logged, hlgaps)]
-    return energies, (logged, hlgaps, mo_energy, mo_coeff, setup.coords, setup.weights)
+    return energies, (logged, hlgaps, mo_energy, mo_coeff, coords, weights)
 
 
 def grad(mol, coords, weight, mo_coeff, mo_energy):

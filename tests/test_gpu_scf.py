@@ -222,3 +222,29 @@ def test_scf_iterate_entry_equals_individual_entries(cuda, precision):
     # the inactive molecule: b2_scf_iterate leaves its buffers untouched, the element-wise torch
     # op of the entry-point path rewrites its diff_JK; the active ones agree
     np.testing.assert_allclose(dj_i[keep], dj_e[keep], atol=1e-9, rtol=0)
+
+
+def test_drop_in_setup_routes(cuda):
+    """the drop-ins' one-electron setup: device arrays equal to the host's, a singular overlap
+    matrix refused with the host's exception, host setup beyond the device grid's 32 atoms"""
+    from b200dft.engine import drop_in_setup
+    m = Mole(methane())
+    for level in (0, 1):
+        hs = HostSetup(m, level)
+        eng = RKSEngine([m], level=level, setups=drop_in_setup(m, level))
+        got = eng.setup_arrays()
+        eng.close()
+        assert eng.setups is None
+        # same formulas in float64; weights down to 1e-9 in magnitude, hence rtol and atol
+        for a, b, tol in zip(got, (hs.Hcore, hs.L_inv, hs.E_nuc, hs.coords, hs.weights), (1e-10,) * 3 + (1e-12,) * 2):
+            np.testing.assert_allclose(a, b, atol=tol, rtol=1e-10)
+    chain = Mole("; ".join(f"H 0 0 {0.74 * k:.3f}" for k in range(34)))
+    opts, _ = nanodft.nanoDFT_options(its=3)
+    E = nanodft.nanoDFT(chain, opts)[0]
+    assert drop_in_setup(chain, 0)[0].mol is chain and np.isfinite(E).all()
+    eng = RKSEngine([m], level=0)
+    eng.device_setup()
+    eng.chol_status.fill_(-5)                      # as the Cholesky kernel reports a singular S
+    with pytest.raises(np.linalg.LinAlgError):
+        eng.setup_arrays()
+    eng.close()
