@@ -293,3 +293,34 @@ def test_chol_inv(cuda):
     assert (st.cpu().numpy() == 0).all()
     for mi, s in enumerate(eng_setups):
         np.testing.assert_allclose(P.unpack(L.cpu().numpy(), mi), s.L_inv, atol=1e-10)
+
+
+@pytest.mark.parametrize("heavy", [0, 1, 2, 3, 5, 7, 9])
+def test_xc_float64_sizes(cuda, heavy):
+    """float64 XC (matrix-instruction products over orbitals rounded up to 8, tiles of 32 points)
+    for molecules of every orbital bucket beside a water molecule, all molecules and a subset
+    active, against the oracle.  Sums of ~1e4 float64 terms of the size of V: 1e-11 relative."""
+    rng = np.random.default_rng(40 + heavy)
+    mols = [Mole("H 0 0 0; H 0 0 0.74") if heavy == 0 else Mole(random_molecule(rng, heavy)),
+            Mole("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7572 -0.4692")]
+    setups = [HostSetup(m, 0) for m in mols]
+    eng = RKSEngine(mols, level=0, precision="fp64", setups=setups)
+    ref, Ds = [], []
+    for m, s in zip(mols, setups):
+        C = rng.normal(size=(m.nao, m.nao)) * 0.1 + np.diag(rng.uniform(0.5, 1.0, m.nao))
+        D = 2.0 * C[:, :m.nelectron // 2] @ C[:, :m.nelectron // 2].T
+        Ds.append(D)
+        ref.append(rks.exchange_correlation(D, rks.ao_values(m, s.coords), s.weights)[:2])
+    D = torch.from_numpy(eng.plan.pack(Ds)).to(cuda)
+    for act in ((1, 1), (0, 1)):
+        eng.Vxc.fill_(-7.0)
+        eng.exc.fill_(-7.0)
+        eng.xc(D, active=torch.tensor(act, dtype=torch.int32, device=cuda))
+        V, E = eng.Vxc.cpu().numpy(), eng.exc.cpu().numpy()
+        for k, (Er, Vr) in enumerate(ref):
+            if act[k]:
+                np.testing.assert_allclose(eng.plan.unpack(V, k), Vr, atol=1e-11 * max(1.0, np.abs(Vr).max()), rtol=0)
+                assert abs(E[k] - Er) <= 1e-11 * abs(Er)
+            else:
+                assert (eng.plan.unpack(V, k) == -7.0).all() and E[k] == -7.0
+    eng.close()
