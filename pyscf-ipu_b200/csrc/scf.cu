@@ -8,9 +8,10 @@
 //     H <- sum_k c[k+1] H_k
 //   C = L^T eigvec(L H L^T) with L = inv(cholesky(S)) (nanoDFT.py:69, 239)
 //   D = 2 C_occ C_occ^T (nanoDFT.py:72)
-// The eigensolver is a parallel cyclic Jacobi method (round-robin pair ordering) on the
+// The eigensolver is a parallel one-sided Jacobi method (round-robin pair ordering) on the
 // matrix held in shared memory; the reference uses jnp.linalg.eigh or TessellateIPU's
 // Jacobi ipu_eigh (nanoDFT.py:370-393).
+#include <type_traits>
 #include "device_plan.cuh"
 #include "scf.cuh"
 
@@ -38,19 +39,6 @@ __device__ double b2_block_max(double v, double *red) {
   return s;
 }
 
-// C[N][N] = A * B (or A * B^T), all row-major in shared memory, ld = N
-__device__ void b2_mm(const double *A, const double *B, double *C, int N, bool transB) {
-  for (int e = threadIdx.x; e < N * N; e += blockDim.x) {
-    const int r = e / N, c = e - (e / N) * N;
-    double s = 0;
-    if (transB)
-      for (int k = 0; k < N; ++k) s += A[r * N + k] * B[c * N + k];
-    else
-      for (int k = 0; k < N; ++k) s += A[r * N + k] * B[k * N + c];
-    C[e] = s;
-  }
-}
-
 // rotation (c, s) zeroing A_pq (Golub & Van Loan, sym.schur2)
 __device__ __host__ inline void b2_schur2(double app, double aqq, double apq, double &c, double &s) {
   if (apq == 0.0) { c = 1.0; s = 0.0; return; }
@@ -62,145 +50,216 @@ __device__ __host__ inline void b2_schur2(double app, double aqq, double apq, do
   s = t * c;
 }
 
-// parallel cyclic Jacobi on A (n x n, n even, leading dimension ld = n + 1) in shared memory;
-// V (same layout) <- eigenvectors.  Rows/columns >= nreal are decoupled padding; the
-// convergence norms use the nreal block only.  Stops when the off-diagonal Frobenius norm is
-// below 1e-13 of the total (eigenvectors then accurate to ~1e-13), or after max_sweeps.
-__device__ int b2_jacobi(double *A, double *V, int n, int nreal, double *rot, int *prs,
-                         double *red, int max_sweeps) {
-  const int ld = n + 1;
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int r = e / n, c = e - (e / n) * n;
-    V[r * ld + c] = (r == c) ? 1.0 : 0.0;
+// ------------------------------------------------------------------ small dense products
+// Both SCF kernels run one molecule per CTA with 64 Q threads (2 Q warps) for the orbital bucket
+// N <= 16 Q.  acc += A B by float64 MMA (m16n8k8): warp w owns columns 8w..8w+7 and every 16-row
+// tile, so a B fragment serves Q products.  fa(r, k) and fb(k, c) return zero outside N.  The
+// inner products of the form before ran one output element per thread with two loads per FMA.
+__device__ __forceinline__ void b2_dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+template <int Q, typename FA, typename FB>
+__device__ __forceinline__ void b2_mm(double (&acc)[Q][4], int N, int K, FA fa, FB fb) {
+  const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+  for (int i = 0; i < Q; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.0;
+  if (8 * w >= N) return;
+#pragma unroll 2
+  for (int k0 = 0; k0 < K; k0 += 8) {
+    const double b[2] = {fb(k0 + t, 8 * w + g), fb(k0 + t + 4, 8 * w + g)};
+#pragma unroll
+    for (int i = 0; i < Q; ++i)
+      if (16 * i < N) {
+        const int r = 16 * i + g;
+        const double a[4] = {fa(r, k0 + t), fa(r + 8, k0 + t), fa(r, k0 + t + 4), fa(r + 8, k0 + t + 4)};
+        b2_dmma(acc[i], a, b);
+      }
+  }
+}
+// f(r, c, value) for every element of the product with r, c < N
+template <int Q, typename F>
+__device__ __forceinline__ void b2_mm_out(const double (&acc)[Q][4], int N, F f) {
+  const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
+#pragma unroll
+  for (int i = 0; i < Q; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int r = 16 * i + g + 8 * (c >> 1), col = 8 * w + 2 * t + (c & 1);
+      if (r < N && col < N) f(r, col, acc[i][c]);
+    }
+}
+
+// ------------------------------------------------------------------ eigensolver
+// One-sided Jacobi (Hestenes) on the symmetric A: G = A / |A| + 2 I (|A| the largest row sum, so
+// the spectrum of G lies in [1, 3]), columns rotated pairwise until they are orthogonal; then
+// column i = g_i v_i with v_i the eigenvector and A's eigenvalue |A| (|g_i| - 2).  Rotating
+// columns needs no eigenvector accumulation and no second (row) phase: a round-robin round is one
+// dot product, one rotation and one barrier, 8 lanes per pair, every pair of the molecule at once.
+// The two-sided form before (rotation phase on n/2 threads, then one pass over every 2 x 2 block
+// and the eigenvectors, two barriers) took 2.2 us per round at 62 orbitals.
+// The angle's tangent is taken in float32 (the rotation itself is exactly orthogonal: cosine and
+// sine follow from that tangent in float64), which leaves 1e-7 of a coupling behind and shortens
+// the round's serial chain.  A sweep whose largest cosine between columns was below 3e-9 leaves
+// couplings at rounding level and is the last.
+// G: column-major, leading dimension LD = 16 Q + 8 (8 modulo 16 doubles: neighbouring groups on
+// different banks), rows and columns beyond N zero.  ev[i] <- eigenvalues, nv[i] <- 1 / |g_i|.
+template <int Q>
+__device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv, double scale, int max_sweeps) {
+  constexpr int LD = 16 * Q + 8, RP = 2 * Q;
+  const int n = (N + 1) & ~1, half = n >> 1;
+  const int grp = threadIdx.x >> 3, li = threadIdx.x & 7;
+  const bool on = grp < half;
+  const int k = on ? grp : 0;
+  auto dot = [&](const double *a, const double *b) {
+    double x = 0;
+#pragma unroll
+    for (int j = 0; j < RP; ++j) x += a[li + 8 * j] * b[li + 8 * j];
+    x += __shfl_xor_sync(0xffffffffu, x, 4);
+    x += __shfl_xor_sync(0xffffffffu, x, 2);
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    return x;
+  };
+  auto norms = [&]() {
+    const double *c0 = G + k * LD, *c1 = G + (k + half) * LD;
+    const double a = dot(c0, c0), b = dot(c1, c1);
+    if (on && li == 0) { nrm[k] = a; nrm[k + half] = b; }
+    __syncthreads();
+  };
+  int sweep = 0;
+  bool more = true;
+  for (; sweep < max_sweeps && more; ++sweep) {
+    norms();
+    bool big = false;
+    for (int r = 0; r < n - 1; ++r) {
+      // round-robin pairs: index 0 fixed, the others rotate by r (k - 1 + r < 2 (n - 1))
+      int a = k - 1 + r, b = n - 2 - k + r;
+      if (a >= n - 1) a -= n - 1;
+      if (b >= n - 1) b -= n - 1;
+      a = (k == 0) ? 0 : a + 1;
+      b += 1;
+      double *cp = G + min(a, b) * LD, *cq = G + max(a, b) * LD;
+      const double app = on ? nrm[min(a, b)] : 0.0, aqq = on ? nrm[max(a, b)] : 0.0;
+      double vp[RP], vq[RP], x = 0;
+#pragma unroll
+      for (int j = 0; j < RP; ++j) {
+        vp[j] = on ? cp[li + 8 * j] : 0.0;
+        vq[j] = on ? cq[li + 8 * j] : 0.0;
+        x += vp[j] * vq[j];
+      }
+      x += __shfl_xor_sync(0xffffffffu, x, 4);
+      x += __shfl_xor_sync(0xffffffffu, x, 2);
+      x += __shfl_xor_sync(0xffffffffu, x, 1);
+      const double x2 = x * x, pq = app * aqq;
+      if (on && x2 > 1e-31 * pq) {
+        big = big || x2 > 1e-17 * pq;
+        // sym.schur2 (Golub & Van Loan): t = sign(d b) |b| / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 x
+        const float d = (float)(aqq - app), bb = (float)(2.0 * x);
+        const float tf = copysignf(1.0f, d * bb) * fabsf(bb) / (fabsf(d) + sqrtf(d * d + bb * bb));
+        const double t = d == 0.0f ? (x > 0 ? 1.0 : -1.0) : (double)tf;
+        const double c = rsqrt(1.0 + t * t), s = t * c;
+#pragma unroll
+        for (int j = 0; j < RP; ++j) {
+          cp[li + 8 * j] = c * vp[j] - s * vq[j];
+          cq[li + 8 * j] = s * vp[j] + c * vq[j];
+        }
+        if (li == 0) {
+          // |g_p'|^2 = c^2 app - 2 c s x + s^2 aqq, the trace is kept
+          const double np = c * c * app - 2.0 * c * s * x + s * s * aqq;
+          nrm[min(a, b)] = np;
+          nrm[max(a, b)] = app + aqq - np;
+        }
+      }
+      __syncthreads();
+    }
+    more = __syncthreads_or(big);
+  }
+  norms();
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double g = sqrt(nrm[i]);
+    ev[i] = i < N ? (g - 2.0) * scale : 1e300;
+    nv[i] = i < N ? 1.0 / g : 0.0;
   }
   __syncthreads();
-  const int half = n / 2;
-  int sweep = 0;
-  for (; sweep < max_sweeps; ++sweep) {
+  return sweep;
+}
+
+// Jacobi on the 10 x 10 DIIS matrix A (shared memory, row-major) run by one warp; V <- the
+// eigenvectors.  Round-robin order: the five rotations of a round act on disjoint pairs, so lanes
+// 0..4 compute them and 25 lanes apply G_k A_kl G_l^T to the 2 x 2 blocks, nine rounds per sweep
+// (the serial order's 45 dependent rotations per sweep took 95 us per call, most of a small
+// molecule's iteration).
+__device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
+  constexpr int n = 10;
+  const int l = threadIdx.x & 31;
+  for (int e = l; e < n * n; e += 32) V[e] = (e / n == e - (e / n) * n) ? 1.0 : 0.0;
+  __syncwarp();
+  for (int sweep = 0; sweep < 50; ++sweep) {
     double off = 0, tot = 0;
-    for (int e = threadIdx.x; e < nreal * nreal; e += blockDim.x) {
-      const int r = e / nreal, c = e - (e / nreal) * nreal;
-      const double a = A[r * ld + c];
-      tot += a * a;
-      if (r != c) off += a * a;
+    for (int e = l; e < n * n; e += 32) {
+      const double x = A[e] * A[e];
+      tot += x;
+      if (e / n != e - (e / n) * n) off += x;
     }
-    off = b2_block_sum(off, red);
-    tot = b2_block_sum(tot, red);
-    if (off <= 1e-26 * tot || off < 1e-300) break;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      off += __shfl_xor_sync(0xffffffffu, off, o);
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    }
+    if (off <= 1e-28 * tot || off < 1e-300) break;
     for (int r = 0; r < n - 1; ++r) {
-      if (threadIdx.x < half) {
-        // round-robin pairs: index 0 fixed, the others rotate by r (k - 1 + r < 2 (n - 1))
-        const int k = threadIdx.x;
+      auto pair = [&](int k, int &p, int &q) {
         int a = k - 1 + r, b = n - 2 - k + r;
         if (a >= n - 1) a -= n - 1;
         if (b >= n - 1) b -= n - 1;
         a = (k == 0) ? 0 : a + 1;
         b += 1;
-        const int p = min(a, b), q = max(a, b);
-        double c, s;
-        const double apq = A[p * ld + q], app = A[p * ld + p], aqq = A[q * ld + q];
-        if (fabs(apq) <= 1e-300 || apq * apq < 1e-34 * fabs(app * aqq)) {
-          c = 1.0; s = 0.0;                         // already negligible
-        } else {
-          // sym.schur2 (Golub & Van Loan) with tau = d / b, d = aqq - app, b = 2 apq:
-          // t = sign(tau) / (|tau| + sqrt(1 + tau^2)) = sign(tau) |b| / (|d| + sqrt(d^2 + b^2))
-          // (one square root, one division; padding never gets here: its couplings are zero)
-          const double d = aqq - app, bb = 2.0 * apq;
-          const double sg = (d == 0.0 || ((d > 0.0) == (bb > 0.0))) ? 1.0 : -1.0;
-          const double t = sg * fabs(bb) / (fabs(d) + sqrt(d * d + bb * bb));
-          c = rsqrt(1.0 + t * t);
-          s = t * c;
-        }
-        prs[2 * k] = p; prs[2 * k + 1] = q;
-        rot[2 * k] = c; rot[2 * k + 1] = s;
-      }
-      __syncthreads();
-      // one pass per round: block (k, l) of A (rows of pair k, columns of pair l) <- G_k A_kl G_l^T,
-      // rows first then columns, exactly the arithmetic of a row pass followed by a column pass;
-      // V's columns of pair l <- V G_l^T
-      for (int e = threadIdx.x; e < half * half + n * half; e += blockDim.x) {
-        if (e < half * half) {
-          const int k = e / half, l = e - (e / half) * half;
-          const int p = prs[2 * k], q = prs[2 * k + 1], pl = prs[2 * l], ql = prs[2 * l + 1];
-          const double ck = rot[2 * k], sk = rot[2 * k + 1], cl = rot[2 * l], sl = rot[2 * l + 1];
-          if (sk == 0.0 && sl == 0.0) continue;
-          double a00 = A[p * ld + pl], a01 = A[p * ld + ql], a10 = A[q * ld + pl], a11 = A[q * ld + ql];
-          if (sk != 0.0) {
-            const double b00 = ck * a00 - sk * a10, b10 = sk * a00 + ck * a10;
-            const double b01 = ck * a01 - sk * a11, b11 = sk * a01 + ck * a11;
-            a00 = b00; a10 = b10; a01 = b01; a11 = b11;
-          }
-          if (sl != 0.0) {
-            const double b00 = cl * a00 - sl * a01, b01 = sl * a00 + cl * a01;
-            const double b10 = cl * a10 - sl * a11, b11 = sl * a10 + cl * a11;
-            a00 = b00; a01 = b01; a10 = b10; a11 = b11;
-          }
-          A[p * ld + pl] = a00; A[p * ld + ql] = a01; A[q * ld + pl] = a10; A[q * ld + ql] = a11;
-        } else {
-          const int e2 = e - half * half, l = e2 / n, row = e2 - (e2 / n) * n;
-          const double cl = rot[2 * l], sl = rot[2 * l + 1];
-          if (sl == 0.0) continue;
-          const int pl = prs[2 * l], ql = prs[2 * l + 1];
-          const double vkp = V[row * ld + pl], vkq = V[row * ld + ql];
-          V[row * ld + pl] = cl * vkp - sl * vkq;
-          V[row * ld + ql] = sl * vkp + cl * vkq;
-        }
-      }
-      __syncthreads();
-    }
-  }
-  return sweep;
-}
-
-// cyclic Jacobi on the 10 x 10 DIIS matrix A (shared memory, row-major) run by one warp; V <- the
-// eigenvectors.  Each rotation (p, q) is a row phase (rows p, q) then a column phase (columns
-// p, q, and V); both are independent across k, so lane k < 10 does element k of each phase with
-// the arithmetic of the one-thread loop: the result is identical to the serial sweep order.
-// The convergence norm is summed serially by lane 0 (same order) and broadcast.
-__device__ void b2_jacobi_small_warp(double *A, double *V) {
-  constexpr int n = 10;
-  const int k = threadIdx.x & 31;
-  if (k < n)
-    for (int j = 0; j < n; ++j) V[k * n + j] = (k == j) ? 1.0 : 0.0;
-  __syncwarp();
-  for (int sweep = 0; sweep < 50; ++sweep) {
-    int done = 0;
-    if (k == 0) {
-      double off = 0, tot = 0;
-      for (int i = 0; i < n * n; ++i) { tot += A[i] * A[i]; if (i / n != i % n) off += A[i] * A[i]; }
-      done = (off <= 1e-28 * tot || off < 1e-300);
-    }
-    if (__shfl_sync(0xffffffffu, done, 0)) break;
-    for (int p = 0; p < n - 1; ++p)
-      for (int q = p + 1; q < n; ++q) {
+        p = min(a, b);
+        q = max(a, b);
+      };
+      if (l < 5) {
+        int p, q;
+        pair(l, p, q);
+        double c = 1.0, s = 0.0;
         const double apq = A[p * n + q], app = A[p * n + p], aqq = A[q * n + q];
-        if (fabs(apq) <= 1e-300 || fabs(apq) < 1e-18 * sqrt(fabs(app * aqq))) continue;
-        double c, s;
-        b2_schur2(app, aqq, apq, c, s);
-        if (s == 0.0) continue;
-        __syncwarp();
-        if (k < n) {
-          const double apk = A[p * n + k], aqk = A[q * n + k];
-          A[p * n + k] = c * apk - s * aqk;
-          A[q * n + k] = s * apk + c * aqk;
-        }
-        __syncwarp();
-        if (k < n) {
-          const double akp = A[k * n + p], akq = A[k * n + q];
-          A[k * n + p] = c * akp - s * akq;
-          A[k * n + q] = s * akp + c * akq;
-          const double vkp = V[k * n + p], vkq = V[k * n + q];
-          V[k * n + p] = c * vkp - s * vkq;
-          V[k * n + q] = s * vkp + c * vkq;
-        }
-        __syncwarp();
+        if (!(fabs(apq) <= 1e-300 || fabs(apq) < 1e-18 * sqrt(fabs(app * aqq)))) b2_schur2(app, aqq, apq, c, s);
+        rot[2 * l] = c;
+        rot[2 * l + 1] = s;
       }
+      __syncwarp();
+      if (l < 25) {
+        const int bk = l / 5, bl = l - (l / 5) * 5;
+        int p, q, u, v;
+        pair(bk, p, q);
+        pair(bl, u, v);
+        const double ck = rot[2 * bk], sk = rot[2 * bk + 1], cl = rot[2 * bl], sl = rot[2 * bl + 1];
+        const double a00 = A[p * n + u], a01 = A[p * n + v], a10 = A[q * n + u], a11 = A[q * n + v];
+        const double b00 = ck * a00 - sk * a10, b10 = sk * a00 + ck * a10;
+        const double b01 = ck * a01 - sk * a11, b11 = sk * a01 + ck * a11;
+        A[p * n + u] = cl * b00 - sl * b01;
+        A[p * n + v] = sl * b00 + cl * b01;
+        A[q * n + u] = cl * b10 - sl * b11;
+        A[q * n + v] = sl * b10 + cl * b11;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {                   // V's rows 2 bk, 2 bk + 1, columns of pair bl
+          double *vr = V + (2 * bk + h) * n;
+          const double x = vr[u], y = vr[v];
+          vr[u] = cl * x - sl * y;
+          vr[v] = sl * x + cl * y;
+        }
+      }
+      __syncwarp();
+    }
   }
 }
 
 // ------------------------------------------------------------------ Fock + DIIS
 // ring layout per molecule (offset mat_off * 9): errs[9][N*N], hams[9][N*N]; B: 100 doubles
-__global__ void __launch_bounds__(256)
+// Bound by latency at one molecule per CTA; 62 orbitals, one molecule: 175 us per call before (two
+// products with one output element per thread, serial 10 x 10 Jacobi).
+template <int Q>
+__global__ void __launch_bounds__(64 * Q)
 k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
             const int *__restrict__ iter, double hyb, int use_diis, const double *__restrict__ Hcore,
             const double *__restrict__ S, const double *__restrict__ D, const double *__restrict__ J,
@@ -209,59 +268,57 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
             double *__restrict__ Bmat, double *__restrict__ diis_err, const int *__restrict__ map) {
   const int m = map ? map[blockIdx.x] : blockIdx.x;
   if (active && !active[m]) return;
+  constexpr int LD = 16 * Q + 4;                   // 4 modulo 16 doubles: fragment loads without bank conflicts
   extern __shared__ double sm[];
   __shared__ double red[32];
   __shared__ double sc[10];
   __shared__ double stmp[9];
-  __shared__ double sA[100], sV[100];
+  __shared__ double sA[100], sV[100], sRot[10];
   const B2MolDev md = mols[m];
   const int N = md.nao, NN = N * N;
   const long long mo = md.mat_off;
-  double *sH = sm, *sS = sH + NN, *sD = sS + NN, *sT = sD + NN;
+  double *sH = sm, *sT = sH + 16 * Q * LD;
+  for (int e = threadIdx.x; e < 2 * 16 * Q * LD; e += blockDim.x) sm[e] = 0.0;   // padding stays zero
+  __syncthreads();
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     const double djk = J[mo + e] - 0.5 * hyb * K[mo + e];
     diffJK[mo + e] = djk;
-    sH[e] = Hcore[mo + e] + djk + Vxc[mo + e];
-    sS[e] = S[mo + e];
-    sD[e] = D[mo + e];
+    const double h = Hcore[mo + e] + djk + Vxc[mo + e];
+    if (!use_diis) H[mo + e] = h;
+    else sH[(e / N) * LD + e - (e / N) * N] = h;
   }
-  __syncthreads();
-  if (!use_diis) {
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) H[mo + e] = sH[e];
-    return;
-  }
+  if (!use_diis) return;
   const int it = iter[m];
   const int nd = 9, head = it % nd;
-  b2_mm(sS, sD, sT, N, false);          // S D
+  double acc[Q][4];
+  const double *gS = S + mo, *gD = D + mo;
+  b2_mm<Q>(acc, N, N, [&](int r, int k) { return r < N && k < N ? gS[r * N + k] : 0.0; },
+           [&](int k, int c) { return k < N && c < N ? gD[k * N + c] : 0.0; });      // S D
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { sT[r * LD + c] = v; });
   __syncthreads();
-  b2_mm(sT, sH, sS, N, false);          // S D H  (into sS)
+  b2_mm<Q>(acc, N, N, [&](int r, int k) { return sT[r * LD + k]; }, [&](int k, int c) { return sH[k * LD + c]; });
+  __syncthreads();
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { sT[r * LD + c] = v; });          // S D H
   __syncthreads();
   double *er = ring_err + mo * nd, *hr = ring_h + mo * nd;
-  double emax = 0;
+  const int nfill = min(it + 1, nd);
+  double emax = 0, s9[9];
+#pragma unroll
+  for (int k = 0; k < 9; ++k) s9[k] = 0.0;
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     const int a = e / N, b = e - (e / N) * N;
-    const double v = sS[a * N + b] - sS[b * N + a];
-    sT[e] = v;
+    const double v = sT[a * LD + b] - sT[b * LD + a];
     emax = fmax(emax, fabs(v));
     er[(long long)head * NN + e] = v;
-    hr[(long long)head * NN + e] = sH[e];
+    hr[(long long)head * NN + e] = sH[a * LD + b];
+    // the nine dot products <err_k, err_new> in the same pass
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+      if (k < nfill) s9[k] += (k == head ? v : er[(long long)k * NN + e]) * v;
   }
   emax = b2_block_max(emax, red);
-  __syncthreads();
-  const int nfill = min(it + 1, nd);
-  // the nine dot products <err_k, err_new> in one pass and one reduction (each thread's partial
-  // sums, the warp shuffles and the sum over warps add in the same order as nine block sums)
   {
-    __shared__ double red9[9][8];                   // 256 threads: 8 warps
-    double s9[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) s9[k] = 0.0;
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-      const double t = sT[e];
-#pragma unroll
-      for (int k = 0; k < 9; ++k)
-        if (k < nfill) s9[k] += er[(long long)k * NN + e] * t;
-    }
+    __shared__ double red9[9][10];                  // at most 320 threads: 10 warps
     const int w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
@@ -294,7 +351,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
       sA[i] = keep ? B[i] : 0.0;
     }
     __syncwarp();
-    b2_jacobi_small_warp(sA, sV);
+    b2_jacobi_small_warp(sA, sV, sRot);
     __syncwarp();
     double smax = 0;
     for (int i = 0; i < 10; ++i) smax = fmax(smax, fabs(sA[i * 10 + i]));
@@ -322,7 +379,11 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
 // sweeps run on W^T F' W, which is nearly diagonal once the SCF settles (2-3 sweeps instead of
 // 6-8); the eigenvectors are W V'.  The result is the same eigen-decomposition up to the sign
 // and order of eigenvectors, which the density does not depend on.
-__global__ void __launch_bounds__(512)
+// Products: M = L^T W, T = H M, A = M^T T, W' = W V', C = L^T W', D = 2 C_occ C_occ^T, all by
+// float64 MMA; two matrices in shared memory (74 KB at 64 orbitals, 3 CTAs per SM).  62 orbitals,
+// one molecule: 430 us per call before.
+template <int Q>
+__global__ void __launch_bounds__(64 * Q)
 k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
                const int *__restrict__ iter, const double *__restrict__ H,
                const double *__restrict__ Linv, double *__restrict__ D, double *__restrict__ mo_energy,
@@ -330,74 +391,68 @@ k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active
                const int *__restrict__ map) {
   const int m = map ? map[blockIdx.x] : blockIdx.x;
   if (active && !active[m]) return;
+  constexpr int LD = 16 * Q + 8, NM = 16 * Q;
   extern __shared__ double sm[];
-  __shared__ double red[32];
-  __shared__ double rot[B2_MAXNAO];
-  __shared__ int prs[B2_MAXNAO];
-  __shared__ int order[B2_MAXNAO];
-  __shared__ double evals[B2_MAXNAO];
+  __shared__ double red[32], nrm[NM], evals[NM], nv[NM];
+  __shared__ int order[NM];
   const B2MolDev md = mols[m];
   const int N = md.nao, NN = N * N;
   const int n = (N + 1) & ~1;                     // even size for the round-robin ordering
-  const int ld = n + 1;                            // odd leading dimension: no bank conflicts
   const long long mo = md.mat_off;
   const bool warm = ws && iter && iter[m] > 0;
-  // shared memory holds A and V only; L and W are read from global memory (L1)
-  double *sA = sm, *sV = sA + n * ld;
+  double *s1 = sm, *s2 = sm + NM * LD;             // column-major, padding zero
   const double *gL = Linv + mo, *gH = H + mo, *gW = ws ? ws + mo : nullptr;
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {                         // L H -> sV
-    const int r = e / N, c = e - (e / N) * N;
-    double s = 0;
-    for (int k = 0; k < N; ++k) s += gL[r * N + k] * gH[k * N + c];
-    sV[r * ld + c] = s;
+  for (int e = threadIdx.x; e < 2 * NM * LD; e += blockDim.x) sm[e] = 0.0;
+  __syncthreads();
+  double acc[Q][4];
+  auto LT = [&](int r, int k) { return r < N && k < N ? gL[k * N + r] : 0.0; };
+  if (warm) {                                                                    // M = L^T W
+    b2_mm<Q>(acc, N, N, LT, [&](int k, int c) { return k < N && c < N ? gW[k * N + c] : 0.0; });
+    b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { s1[c * LD + r] = v; });
+  } else {
+    for (int e = threadIdx.x; e < NN; e += blockDim.x) s1[(e / N) * LD + e - (e / N) * N] = gL[e];
   }
   __syncthreads();
-  // F' = (L H) L^T into sA (padded to n: decoupled padding sorts last); consecutive threads take
-  // consecutive rows, so the L row is a broadcast and sV / sA are read and written conflict-free
-  for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-    const int c = e / n, r = e - (e / n) * n;
-    double s = 0;
-    if (r < N && c < N)
-      for (int k = 0; k < N; ++k) s += sV[r * ld + k] * gL[c * N + k];
-    else if (r == c)
-      s = 1e30;
-    sA[r * ld + c] = s;
-  }
+  b2_mm<Q>(acc, N, N, [&](int r, int k) { return r < N && k < N ? gH[r * N + k] : 0.0; },
+           [&](int k, int c) { return s1[c * LD + k]; });                        // T = H M
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { s2[c * LD + r] = v; });
   __syncthreads();
-  if (warm) {
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) {                       // F' W -> sV
-      const int r = e / N, c = e - (e / N) * N;
-      double s = 0;
-      for (int k = 0; k < N; ++k) s += sA[r * ld + k] * gW[k * N + c];
-      sV[r * ld + c] = s;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) {                       // W^T (F' W) -> sA
-      const int r = e / N, c = e - (e / N) * N;
-      double s = 0;
-      for (int k = 0; k < N; ++k) s += gW[k * N + r] * sV[k * ld + c];
-      sA[r * ld + c] = s;
-    }
-    __syncthreads();
-  }
-  const int sw = b2_jacobi(sA, sV, n, N, rot, prs, red, 30);
-  for (int i = threadIdx.x; i < n; i += blockDim.x) evals[i] = sA[i * ld + i];
+  b2_mm<Q>(acc, N, N, [&](int r, int k) { return s1[r * LD + k]; }, [&](int k, int c) { return s2[c * LD + k]; });
   __syncthreads();
-  // eigenvectors E in the orthogonal basis: W V' (warm) or V', into sA
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { s1[c * LD + r] = v; });     // A = M^T T
+  __syncthreads();
+  // scale = largest column sum of |A|; G = A / scale + 2 I
+  double rs = 0;
+  for (int c = threadIdx.x; c < N; c += blockDim.x) {
+    double x = 0;
+    for (int r = 0; r < N; ++r) x += fabs(s1[c * LD + r]);
+    rs = fmax(rs, x);
+  }
+  rs = b2_block_max(rs, red);
+  const double scale = rs > 0.0 ? rs : 1.0, inv = 1.0 / scale;
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    const int r = e / N, c = e - (e / N) * N;
-    double s;
-    if (warm) {
-      s = 0;
-      for (int k = 0; k < N; ++k) s += gW[r * N + k] * sV[k * ld + c];
-    } else {
-      s = sV[r * ld + c];
-    }
-    sA[r * ld + c] = s;
+    const int c = e / N, r = e - (e / N) * N;
+    s1[c * LD + r] = s1[c * LD + r] * inv + (r == c ? 2.0 : 0.0);
   }
   __syncthreads();
-  if (ws)
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) ws[mo + e] = sA[(e / N) * ld + e % N];
+  const int sw = b2_jacobi1<Q>(s1, N, nrm, evals, nv, scale, 30);
+  // eigenvectors in the orthogonal basis, W' = W V' (warm) or V', into s2 and ws
+  if (warm) {
+    b2_mm<Q>(acc, N, N, [&](int r, int k) { return r < N && k < N ? gW[r * N + k] : 0.0; },
+             [&](int k, int c) { return s1[c * LD + k]; });
+    __syncthreads();                               // every warp has read W
+    b2_mm_out<Q>(acc, N, [&](int r, int c, double v) {
+      s2[c * LD + r] = v * nv[c];
+      ws[mo + r * N + c] = v * nv[c];
+    });
+  } else {
+    for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+      const int c = e / N, r = e - (e / N) * N;
+      const double v = s1[c * LD + r] * nv[c];
+      s2[c * LD + r] = v;
+      if (ws) ws[mo + r * N + c] = v;
+    }
+  }
   // ascending order of eigenvalues: a total order (NaN sorts as +inf, ties by index), so the
   // ranks are a permutation of 0..n-1 whatever the values (every order[] slot is written)
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
@@ -411,23 +466,16 @@ k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active
   }
   __syncthreads();
   for (int k = threadIdx.x; k < N; k += blockDim.x) mo_energy[(long long)m * B2_MAXNAO + k] = evals[order[k]];
-  // C[:, k] = L^T E[:, order[k]]  (all N columns, into sV)
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    const int r = e / N, k = e - (e / N) * N;
-    const int col = order[k];
-    double s = 0;
-    for (int a = 0; a < N; ++a) s += gL[a * N + r] * sA[a * ld + col];
-    sV[r * ld + k] = s;
-  }
+  // C = L^T W' (columns unsorted), into s1
+  b2_mm<Q>(acc, N, N, LT, [&](int k, int c) { return s2[c * LD + k]; });
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { s1[c * LD + r] = v; });
   __syncthreads();
   const int nocc = md.nocc;
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    const int a = e / N, b = e - (e / N) * N;
-    double s = 0;
-    for (int k = 0; k < nocc; ++k) s += sV[a * ld + k] * sV[b * ld + k];
-    D[mo + e] = 2.0 * s;
-    if (C) C[mo + e] = sV[a * ld + b];
-  }
+  auto occ = [&](int r, int k) { return k < nocc ? s1[order[k] * LD + r] : 0.0; };
+  b2_mm<Q>(acc, N, nocc, occ, [&](int k, int c) { return occ(c, k); });
+  b2_mm_out<Q>(acc, N, [&](int r, int c, double v) { D[mo + r * N + c] = 2.0 * v; });
+  if (C)
+    for (int e = threadIdx.x; e < NN; e += blockDim.x) C[mo + e] = s1[order[e - (e / N) * N] * LD + e / N];
   if (threadIdx.x == 0 && sweeps) sweeps[m] = sw;
 }
 
@@ -545,8 +593,8 @@ __global__ void k_chol_inv(const B2MolDev *__restrict__ mols, const double *__re
   if (threadIdx.x == 0 && status) status[m] = bad ? B2_ERR_NOT_PD : B2_OK;
 }
 
-static size_t b2_fock_smem(int N) { return sizeof(double) * 4 * N * N; }
-static size_t b2_eigh_smem(int N) { int n = (N + 1) & ~1; return sizeof(double) * 2 * n * (n + 1); }
+static size_t b2_fock_smem(int Q) { return sizeof(double) * 2 * 16 * Q * (16 * Q + 4); }
+static size_t b2_eigh_smem(int Q) { return sizeof(double) * 2 * 16 * Q * (16 * Q + 8); }
 
 // One launch per orbital bucket (nao <= 16, 32, 48, 64, more) with shared memory sized for that
 // bucket, so small molecules run several CTAs per SM.  The bucket launches go to the plan's
@@ -561,9 +609,8 @@ static int b2_per_bucket(const B2PlanDev &P, cudaStream_t st, F launch) {
   for (int b = B2_NBKT - 1; b >= 0; --b) {          // largest molecules first
     const int n = off[b + 1] - off[b];
     if (n <= 0) continue;
-    const int N = std::min(P.h.max_nao, 16 * (b + 1));
     B2_CUDA_TRY(cudaStreamWaitEvent(P.bkt_stream[b], P.bkt_ev[B2_NBKT], 0));
-    launch(N, n, map + off[b], P.bkt_stream[b]);
+    B2_CUDA_TRY(launch(b + 1, n, map + off[b], P.bkt_stream[b]));
     b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
     B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[b], P.bkt_stream[b]));
@@ -572,27 +619,46 @@ static int b2_per_bucket(const B2PlanDev &P, cudaStream_t st, F launch) {
   return B2_OK;
 }
 
+// f(integral constant Q) for the bucket q = Q
+template <typename F> static cudaError_t b2_by_bucket(int q, F f) {
+  switch (q) {
+    case 1: return f(std::integral_constant<int, 1>{});
+    case 2: return f(std::integral_constant<int, 2>{});
+    case 3: return f(std::integral_constant<int, 3>{});
+    case 4: return f(std::integral_constant<int, 4>{});
+    default: return f(std::integral_constant<int, 5>{});
+  }
+}
+
 int b2_launch_fock_diis(const B2PlanDev &P, const int *active, const int *iter, double hyb,
                         int use_diis, const double *Hcore, const double *S, const double *D,
                         const double *J, const double *K, const double *Vxc, double *H,
                         double *diffJK, double *ring_err, double *ring_h, double *Bmat,
                         double *diis_err, cudaStream_t st) {
-  B2_CUDA_TRY(cudaFuncSetAttribute(k_fock_diis, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)b2_fock_smem(P.h.max_nao)));
-  return b2_per_bucket(P, st, [&](int N, int n, const int *map, cudaStream_t s) {
-    k_fock_diis<<<n, 256, b2_fock_smem(N), s>>>(P.mols, active, iter, hyb, use_diis, Hcore, S, D, J, K,
-                                                Vxc, H, diffJK, ring_err, ring_h, Bmat, diis_err, map);
+  return b2_per_bucket(P, st, [&](int q, int n, const int *map, cudaStream_t s) {
+    return b2_by_bucket(q, [&](auto Q) {
+      cudaError_t e = cudaFuncSetAttribute(k_fock_diis<Q.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)b2_fock_smem(q));
+      if (e == cudaSuccess)
+        k_fock_diis<Q.value><<<n, 64 * q, b2_fock_smem(q), s>>>(P.mols, active, iter, hyb, use_diis, Hcore, S, D, J, K,
+                                                                Vxc, H, diffJK, ring_err, ring_h, Bmat, diis_err, map);
+      return e;
+    });
   });
 }
 
 int b2_launch_eigh_density(const B2PlanDev &P, const int *active, const int *iter, const double *H,
                            const double *Linv, double *D, double *mo_energy, double *C, double *ws,
                            int *sweeps, cudaStream_t st) {
-  B2_CUDA_TRY(cudaFuncSetAttribute(k_eigh_density, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)b2_eigh_smem(P.h.max_nao)));
-  return b2_per_bucket(P, st, [&](int N, int n, const int *map, cudaStream_t s) {
-    k_eigh_density<<<n, N > 32 ? 512 : 256, b2_eigh_smem(N), s>>>(P.mols, active, iter, H, Linv, D, mo_energy, C, ws,
-                                                   sweeps, map);
+  return b2_per_bucket(P, st, [&](int q, int n, const int *map, cudaStream_t s) {
+    return b2_by_bucket(q, [&](auto Q) {
+      cudaError_t e = cudaFuncSetAttribute(k_eigh_density<Q.value>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)b2_eigh_smem(q));
+      if (e == cudaSuccess)
+        k_eigh_density<Q.value><<<n, 64 * q, b2_eigh_smem(q), s>>>(P.mols, active, iter, H, Linv, D, mo_energy, C, ws,
+                                                                   sweeps, map);
+      return e;
+    });
   });
 }
 
