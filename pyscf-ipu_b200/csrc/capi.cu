@@ -109,10 +109,10 @@ static void b2_plan_free(B2PlanDev *P) {
   b2_subset_free(P);
   b2_grid_free(*P);
   b2_dfree(P->mols); b2_dfree(P->row_off); b2_dfree(P->shells); b2_dfree(P->pinfo);
-  b2_dfree(P->pp64); b2_dfree(P->pp32); b2_dfree(P->pp32_n); b2_dfree(P->ao2sh); b2_dfree(P->cls_list);
-  b2_dfree(P->cls_cnt); b2_dfree(P->atom_xyz); b2_dfree(P->atom_z); b2_dfree(P->boys); b2_dfree(P->boys32);
+  b2_dfree(P->su.su); b2_dfree(P->su.mol); b2_dfree(P->su.off);
+  b2_dfree(P->su.pr64); b2_dfree(P->su.pr32); b2_dfree(P->su.pn); b2_dfree(P->ao2sh);
+  b2_dfree(P->atom_xyz); b2_dfree(P->atom_z); b2_dfree(P->boys); b2_dfree(P->boys32);
   b2_dfree(P->jk_chunk_off);
-  b2_dfree(P->eri_tasks32); b2_dfree(P->eri_tasks64);
   b2_dfree(P->sv_off); b2_dfree(P->sv_work); b2_dfree(P->bkt_map);
   for (int b = 0; b < B2_NBKT; ++b) if (P->bkt_stream[b]) cudaStreamDestroy(P->bkt_stream[b]);
   for (int b = 0; b <= B2_NBKT; ++b) if (P->bkt_ev[b]) cudaEventDestroy(P->bkt_ev[b]);
@@ -199,7 +199,14 @@ int b2_plan_create(int nmol, const int *natm, const int *nbas, const int *atm, c
   b2_boys_fill_table(tab.data());
   std::vector<float> tab32(tab.begin(), tab.end());
   const B2PlanHost &H = P->h;
-  size_t need = 16 * 256 + sizeof(B2MolDev) * H.mols.size() + sizeof(long long) * H.row_off.size() +
+  std::vector<B2gSuper> su;
+  std::vector<B2gsMol> su_mol;
+  std::vector<long long> su_off;
+  b2_su_host(H, su, su_mol, su_off);
+  for (int k = 0; k < B2_SU_NOFF; ++k) P->su.n_task[k] = su_off[k * (nmol + 1ll) + nmol];
+  P->su.n_pair = P->su.n_task[B2_SU_PAIRS];
+  size_t need = 20 * 256 + sizeof(B2gSuper) * su.size() + sizeof(B2gsMol) * su_mol.size() +
+                sizeof(long long) * su_off.size() + sizeof(B2MolDev) * H.mols.size() + sizeof(long long) * H.row_off.size() +
                 sizeof(B2Shell) * H.shells.size() + sizeof(int) * H.ao2sh.size() +
                 sizeof(double) * H.atom_xyz.size() + sizeof(int) * H.atom_z.size() +
                 sizeof(double) * tab.size() + sizeof(float) * tab32.size() +
@@ -221,6 +228,8 @@ int b2_plan_create(int nmol, const int *natm, const int *nbas, const int *atm, c
       (rc = b2_upload(&P->shells, H.shells, &u)) || (rc = b2_upload(&P->ao2sh, H.ao2sh, &u)) ||
       (rc = b2_upload(&P->atom_xyz, H.atom_xyz, &u)) || (rc = b2_upload(&P->atom_z, H.atom_z, &u)) ||
       (rc = b2_upload(&P->boys, tab, &u)) || (rc = b2_upload(&P->boys32, tab32, &u)) ||
+      (rc = b2_upload(&P->su.su, su, &u)) || (rc = b2_upload(&P->su.mol, su_mol, &u)) ||
+      (rc = b2_upload(&P->su.off, su_off, &u)) ||
       (rc = b2_set_jk_chunk(P, 0, &u)) || (rc = b2_build_pairs(*P, u.st)) || (rc = b2_set_sv(P, &u))) {
     cudaStreamSynchronize(u.st);
     cudaStreamDestroy(u.st);

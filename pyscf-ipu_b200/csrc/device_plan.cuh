@@ -3,6 +3,7 @@
 #include "plan_host.hpp"
 #include "boys.cuh"
 #include "eri_sq.cuh"
+#include "super.cuh"
 
 // number of kernels this library has launched (monotonic; read with b2_launch_count)
 void b2_count_launches(long long n);
@@ -35,18 +36,31 @@ struct B2SubsetDev {           // compacted work tables for a subset of the batc
   std::vector<long long> xq_off_h;
 };
 
+// super-shell tables (super.cuh): prefixes over molecules, B2_SU_NOFF arrays of nmol + 1 back to
+// back: tasks of the six integral classes, pairs, tasks of the six gradient classes, slices
+#define B2_SU_PAIRS 6
+#define B2_SU_GRAD 7
+#define B2_SU_GRAD1 13
+#define B2_SU_NOFF 14
+struct B2SuDev {
+  B2gSuper *su = nullptr;
+  B2gsMol *mol = nullptr;
+  long long *off = nullptr;
+  B2gPrim *pr64 = nullptr;                // nine slots per pair: float64 and gradient primitives
+  B2gPrim32 *pr32 = nullptr;
+  B2gCount *pn = nullptr;                 // per pair: float32 / float64 / gradient primitives
+  long long n_pair = 0, n_task[B2_SU_NOFF] = {};
+};
+
 struct B2PlanDev {
   B2PlanHost h;
   B2MolDev *mols = nullptr;
   long long *row_off = nullptr;
   B2Shell *shells = nullptr;
   B2PairInfo *pinfo = nullptr;
-  B2PairPrim<double> *pp64 = nullptr;
-  B2PairPrim<float> *pp32 = nullptr;
-  unsigned char *pp32_n = nullptr;        // per shell pair: surviving float32 primitive pairs
+  B2SuDev su;
   int *ao2sh = nullptr;
-  int *cls_list = nullptr;
-  int *cls_cnt = nullptr;
+  int *cls_list = nullptr;                // shell-pair class lists (allocation-free entry only)
   double *atom_xyz = nullptr;
   int *atom_z = nullptr;
   double *boys = nullptr;
@@ -57,8 +71,6 @@ struct B2PlanDev {
   int device = 0;
   long long h2d_bytes = 0;                // bytes copied host -> device by plan creation
   B2GridDev g;
-  B2EriTask *eri_tasks32 = nullptr, *eri_tasks64 = nullptr;
-  std::vector<long long> eri_goff32, eri_goff64;   // task group (class combination) starts
   std::vector<long long> jk_off_h;                 // host copy of jk_chunk_off
   B2SubsetDev sub;
   int xc_impl = 0;             // float32 XC: 0 = tensor-core kernel, 1 = SIMT kernel
@@ -76,9 +88,10 @@ struct B2PlanDev {
 };
 
 int b2_launch_eri_s8(B2PlanDev &P, int precision, void *out, cudaStream_t st);
-// the ERI work list of `precision` (32: canonical shell quartets grouped by class combination,
-// up to 32 kets per task; 64: p-shell bras split by component), built once per plan
-int b2_eri_tasks_ready(B2PlanDev &P, int precision, cudaStream_t st);
+void b2_su_host(const B2PlanHost &h, std::vector<B2gSuper> &su, std::vector<B2gsMol> &gm,
+                std::vector<long long> &off);
+// bra and ket types of the six gradient classes, in launch order
+static const int b2gs_tb[6] = {2, 2, 2, 1, 1, 0}, b2gs_tk[6] = {2, 1, 0, 1, 0, 0};
 int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const double *mo_energy,
                    const double *coords, const double *weights, double *D, double *W, double *grad,
                    cudaStream_t st);

@@ -3,18 +3,13 @@
 // (direct.py:584-707), and writes straight into the tril-of-tril s8 layout of
 // ``mol.intor('int2e_sph', aosym='s8')`` (nanoDFT.py:285).
 //
-// Decomposition: a task list (built on the device from the plan's class counts, or on the host
-// for the allocation-free single-molecule entry) assigns each warp one bra shell pair IJ of one
-// molecule and a chunk of ket shell pairs KL of a single angular class (ss, ps, sp, pp), all
-// with KL <= (I,I) (32 kets per task for batch plans, 128 for the single-molecule entry; 4 tasks
-// per CTA); the bra's primitive pairs are staged in the warp's shared-memory slot.  Batch plans
-// run the float32 classes with at most 27 components in the flattened kernel k_eri_fl (lanes
-// over the chunk's (ket, ket primitive pair) entries); otherwise (k_eri_sq) every lane evaluates
-// all components of one shell quartet (float32) or of one bra component (float64, p bras split
-// over 3 lanes), looping over the chunk's kets.  Every s8 entry is written exactly once, by the
-// warp whose bra shell pair owns its row ij.
+// Batch plans: super-shell pairs (super.cuh, eri_su.cuh).  A class is a bra slice type and a ket
+// pair type; a warp task is one bra slice x 32 ket pairs of one molecule, found from prefix sums
+// of the molecules' task counts (no work list in memory).  The allocation-free single-molecule
+// entry at the end of this file keeps the shell-pair kernels k_eri_sq and their host work list.
 #include <type_traits>
 #include "eri_sq.cuh"
+#include "eri_su.cuh"
 #include "device_plan.cuh"
 #include "devmem.cuh"
 #include "eri_flops.h"
@@ -49,121 +44,233 @@ k_eri_sq(const B2EriTask *__restrict__ tasks, long long ntask, const B2MolDev *_
   }
 }
 
-// Flattened form for the float32 classes with at most 27 components per shell quartet: the
-// warp's (ket, ket primitive pair) entries are packed over the lanes (a ket's primitive pairs
-// survive screening in numbers 0..9, so one ket per lane left the warp waiting for its
-// largest ket); each lane sums its entry over the bra's primitive pairs, a same-ket segmented
-// shuffle scan (segments <= 9 lanes, 4 steps) combines the entries of each ket in a fixed
-// order, and the segment's last lane adds the sum to the ket's accumulator in shared memory.
-// component block <-> flat list (unrolled: constant indices, registers only)
-template <typename S>
-__device__ __forceinline__ void b2_fl_flatten(const float (&acc)[S::NI][S::NJ][S::NK][S::NL], float *v) {
-  int t = 0;
-#pragma unroll
-  for (int a = 0; a < S::NI; ++a)
-#pragma unroll
-    for (int b = 0; b < S::NJ; ++b)
-#pragma unroll
-      for (int c = 0; c < S::NK; ++c)
-#pragma unroll
-        for (int d = 0; d < S::NL; ++d) v[t++] = acc[a][b][c][d];
-}
-template <typename S>
-__device__ __forceinline__ void b2_fl_unflatten(const float *v, float (&acc)[S::NI][S::NJ][S::NK][S::NL]) {
-  int t = 0;
-#pragma unroll
-  for (int a = 0; a < S::NI; ++a)
-#pragma unroll
-    for (int b = 0; b < S::NJ; ++b)
-#pragma unroll
-      for (int c = 0; c < S::NK; ++c)
-#pragma unroll
-        for (int d = 0; d < S::NL; ++d) acc[a][b][c][d] = v[t++];
+// ------------------------------------------------------------------ batch plans
+template <typename T> struct B2EriPrimOf { using type = B2gPrim; };
+template <> struct B2EriPrimOf<float> { using type = B2gPrim32; };
+__device__ __forceinline__ int b2_eri_n(const B2gCount &n, const B2gPrim *) { return n.y; }
+__device__ __forceinline__ int b2_eri_n(const B2gCount &n, const B2gPrim32 *) { return n.x; }
+
+__device__ __forceinline__ int b2_eri_find(const long long *__restrict__ off, int n, long long x) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (off[mid] <= x) lo = mid; else hi = mid - 1;
+  }
+  return lo;
 }
 
-template <int LI, int LJ, int LK, int LL>
+// one warp task: the bra slice's data and its ket range
+struct B2EriTaskSu {
+  int m, pair, f, cnt, k0, A, B;
+};
+template <int TB, int TK>
+__device__ __forceinline__ bool b2_eri_task(const long long *__restrict__ toff, int nmol,
+                                            const B2gsMol *__restrict__ gms, long long task, B2gsMol &g,
+                                            B2EriTaskSu &t) {
+  t.m = b2_eri_find(toff, nmol, task);
+  g = gms[t.m];
+  const int nch = (b2es_npair(g.ns, g.np, TK) + 31) >> 5;
+  const int r0 = (int)(task - toff[t.m]), i = r0 / nch;
+  int limit;
+  b2es_bra_of(g.ns, g.np, TB, TK, i, t.pair, limit);
+  t.f = TB == 2 ? i - 3 * (i / 3) : 0;
+  t.k0 = (r0 - i * nch) * 32;
+  t.cnt = min(32, limit - t.k0);
+  if (t.cnt <= 0) return false;
+  b2gs_pair(g.ns, g.np, t.pair, t.A, t.B);
+  return true;
+}
+
+// (ss|ss) pairs: lanes over the chunk's (ket, ket primitive) entries packed by a prefix sum of the
+// kets' surviving primitives; each lane sums its entry over the bra's primitives, a same-ket
+// segmented scan (segments <= 9 lanes) combines the entries of a ket.
+template <typename T>
 __global__ void __launch_bounds__(128)
-k_eri_fl(const B2EriTask *__restrict__ tasks, long long ntask, const B2MolDev *__restrict__ mols,
-         const B2PairInfo *__restrict__ pinfo, const B2PairPrim<float> *__restrict__ pp,
-         const unsigned char *__restrict__ ppn, const int *__restrict__ cls_list, const float *__restrict__ btab,
-         float *__restrict__ out) {
-  using S = B2Sq<float, LI, LJ, LK, LL, -1>;
-  constexpr int NC = S::NI * S::NJ * S::NK * S::NL;
-  static_assert(NC <= 27, "flattened ERI form: at most 27 components");
-  __shared__ B2PairPrim<float> sbra[4][B2_MAXPP];
-  __shared__ int s_nb[4];
-  __shared__ int s_off[4][32], s_kl[4][32];
+k_eri_ss(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
+         const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su,
+         const typename B2EriPrimOf<T>::type *__restrict__ pr, const B2gCount *__restrict__ pn,
+         const T *__restrict__ btab, T *__restrict__ out) {
+  using S = B2Es<T, 0, 0>;
+  __shared__ B2EriBra<T> sbra[4][B2_MAXPP];
+  __shared__ int s_off[4][32];
   __shared__ unsigned char s_map[4][32 * B2_MAXPP];
-  __shared__ float s_acc[4][32][NC];
+  __shared__ T s_acc[4][32];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long long ti = (long long)blockIdx.x * 4 + w;
-  if (ti >= ntask) return;                        // whole warp
-  const B2EriTask tk = tasks[ti];
-  const B2MolDev md = mols[tk.mol];
-  const B2PairInfo bp = pinfo[md.sp_off + tk.IJ];
-  if (lane == 0) {
-    const B2PairPrim<float> *src = pp + (size_t)(md.sp_off + tk.IJ) * B2_MAXPP;
-    int nb = 0;
-    for (int x = 0; x < B2_MAXPP; ++x)
-      if (src[x].K != 0.f) sbra[w][nb++] = src[x];
-    s_nb[w] = nb;
-  }
-  // this lane's ket (tasks of batch plans hold at most 32 kets) and its surviving primitive pairs
-  int KL = 0, nq = 0;
-  if (lane < tk.count) {
-    KL = cls_list[md.sp_off + md.cls_start[tk.cls] + tk.start + lane];
-    nq = ppn[md.sp_off + KL];
-  }
-  int inc = nq;
+  const long long ntask = toff[nmol];
+  for (long long task = (long long)blockIdx.x * 4 + w; task < ntask; task += (long long)gridDim.x * 4) {
+    B2gsMol g;
+    B2EriTaskSu t;
+    if (!b2_eri_task<0, 0>(toff, nmol, gms, task, g, t)) continue;   // whole warp: beyond the diagonal
+    const long long p0 = g.pr_off;
+    const int nb = b2_eri_n(pn[p0 + t.pair], pr);
+    __syncwarp();                                    // the previous task's shared memory is consumed
+    const double zero[3] = {0, 0, 0};
+    if (lane < nb) b2es_bra(pr[(p0 + t.pair) * B2_MAXPP + lane], false, 0, zero, sbra[w][lane]);
+    const int nq = lane < t.cnt ? b2_eri_n(pn[p0 + t.k0 + lane], pr) : 0;
+    int inc = nq;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += y;
-  }
-  const int E = __shfl_sync(0xffffffffu, inc, 31), exc = inc - nq;
-  s_off[w][lane] = exc;
-  s_kl[w][lane] = KL;
-  for (int j = 0; j < nq; ++j) s_map[w][exc + j] = (unsigned char)lane;
-#pragma unroll
-  for (int c = 0; c < NC; ++c) s_acc[w][lane][c] = 0.f;
-  __syncwarp();
-  const int nb = s_nb[w];
-  const B2PairPrim<float> *ppm = pp + (size_t)md.sp_off * B2_MAXPP;
-  for (int e0 = 0; e0 < E; e0 += 32) {
-    const int e = e0 + lane;
-    const bool valid = e < E;
-    const int k = valid ? (int)s_map[w][e] : -1 - lane;   // entries past the end: unique keys
-    float acc[S::NI][S::NJ][S::NK][S::NL];
-    S::zero(acc);
-    if (valid) {
-      const B2PairPrim<float> Q = ppm[(size_t)s_kl[w][k] * B2_MAXPP + (e - s_off[w][k])];
-      for (int p = 0; p < nb; ++p) S::quartet(sbra[w][p], Q, btab, acc);
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
     }
-    float a[NC];
-    b2_fl_flatten<S>(acc, a);
+    const int E = __shfl_sync(0xffffffffu, inc, 31);
+    s_off[w][lane] = inc - nq;
+    for (int j = 0; j < nq; ++j) s_map[w][inc - nq + j] = (unsigned char)lane;
+    s_acc[w][lane] = (T)0;
+    __syncwarp();
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane;
+      const bool valid = e < E;
+      const int k = valid ? (int)s_map[w][e] : -1 - lane;   // entries past the end: unique keys
+      T a = (T)0;
+      if (valid) {
+        B2EriKet<T> q;
+        b2es_ket(pr[(p0 + t.k0 + k) * B2_MAXPP + (e - s_off[w][k])], 0, zero, q);
+        T phi[1][1] = {{(T)0}};
+        for (int p = 0; p < nb; ++p) S::quartet(sbra[w][p], q, btab, phi);
+        S::ket(q, phi[0], &a);
+      }
 #pragma unroll
-    for (int o = 1; o < 16; o <<= 1) {                     // same-ket inclusive scan
-      const int ko = __shfl_up_sync(0xffffffffu, k, o);
-      const bool take = lane >= o && ko == k;
+      for (int o = 1; o < 16; o <<= 1) {                     // same-ket inclusive scan
+        const int ko = __shfl_up_sync(0xffffffffu, k, o);
+        const T y = __shfl_up_sync(0xffffffffu, a, o);
+        if (lane >= o && ko == k) a += y;
+      }
+      const int kn = __shfl_down_sync(0xffffffffu, k, 1);
+      if (valid && (lane == 31 || kn != k)) s_acc[w][k] += a;
+      __syncwarp();
+    }
+    if (lane < t.cnt) {
+      int c, d;
+      b2gs_pair(g.ns, g.np, t.k0 + lane, c, d);
+      const B2gSuper *sm = su + g.su_off;
+      b2es_put(out + mols[t.m].eri_off, sm[t.A].ao_s, sm[t.B].ao_s, sm[c].ao_s, sm[d].ao_s, t.A == t.B, c == d,
+               t.pair == t.k0 + lane, s_acc[w][lane]);
+    }
+  }
+}
+
+// The other classes: 4 lanes per ket pair, 8 kets at a time; a lane takes every fourth of its
+// ket's primitives and sums, over the bra's primitives (shared memory), the derivatives Phi of the
+// class (up to 40 values in registers).  The ket's polynomial turns them into up to 16 integrals
+// per bra function, which a two-step transposing butterfly sums over the ket's lanes: lane li
+// ends with the integrals of ket function li, in registers until the ket is done.
+// Bound by FP32 issue (float32) and by the chain of a quartet at 8 warps per SM (float64, 242
+// registers).  Before: 16 kernels, one per l class over the unmerged shells, every integral
+// accumulated per primitive quartet: 2.2 times the quartets, each with its own Boys evaluation.
+// All classes and the exchange list, 2048 molecules float32: 67.6 -> 38.2 ms; 50 molecules float64:
+// 5.21 -> 2.07 ms.
+template <typename T> struct __align__(16) B2EriWarp {
+  B2EriBra<T> bra[B2_MAXPP];
+  double CD[32][3];
+  int ao[32][4];
+  unsigned char n[32], same[32];
+};
+template <typename T, int TB, int TK>
+__global__ void __launch_bounds__(128)
+k_eri_su(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
+         const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su,
+         const typename B2EriPrimOf<T>::type *__restrict__ pr, const B2gCount *__restrict__ pn,
+         const T *__restrict__ btab, T *__restrict__ out) {
+  using S = B2Es<T, TB, TK>;
+  constexpr int NB = S::NB, NO = TK == 2 ? 4 : 1;      // integrals a lane ends with per bra function
+  extern __shared__ __align__(16) unsigned char es_smem[];
+  T *tab = reinterpret_cast<T *>(es_smem);
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, qd = lane >> 2, li = lane & 3;
+  B2EriWarp<T> &W = reinterpret_cast<B2EriWarp<T> *>(es_smem + sizeof(T) * B2_BOYS_NT * B2_BOYS_NM)[w];
+  for (int e = threadIdx.x; e < B2_BOYS_NT * B2_BOYS_NM; e += blockDim.x) tab[e] = btab[e];
+  __syncthreads();
+  const long long ntask = toff[nmol];
+  for (long long task = (long long)blockIdx.x * 4 + w; task < ntask; task += (long long)gridDim.x * 4) {
+    B2gsMol g;
+    B2EriTaskSu t;
+    if (!b2_eri_task<TB, TK>(toff, nmol, gms, task, g, t)) continue;
+    const B2gSuper *sm = su + g.su_off;
+    const long long p0 = g.pr_off;
+    const int nb = b2_eri_n(pn[p0 + t.pair], pr), kf = b2es_first(g.ns, g.np, TK) + t.k0;
+    __syncwarp();                                    // the previous task's shared memory is consumed
+    if (lane < nb) {
+      double AB[3];
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float y = __shfl_up_sync(0xffffffffu, a[c], o);
-        if (take) a[c] += y;
+      for (int x = 0; x < 3; ++x) AB[x] = sm[t.A].R[x] - sm[t.B].R[x];
+      b2es_bra(pr[(p0 + t.pair) * B2_MAXPP + lane], TB == 2, t.f, AB, W.bra[lane]);
+    }
+    W.n[lane] = 0;
+    if (lane < t.cnt) {
+      int c, d;
+      b2gs_pair(g.ns, g.np, kf + lane, c, d);
+      W.n[lane] = (unsigned char)b2_eri_n(pn[p0 + kf + lane], pr);
+      W.same[lane] = (unsigned char)((c == d) + 2 * (t.pair == kf + lane));
+      W.ao[lane][0] = sm[c].ao_s; W.ao[lane][1] = sm[c].ao_p; W.ao[lane][2] = sm[d].ao_s; W.ao[lane][3] = sm[d].ao_p;
+#pragma unroll
+      for (int x = 0; x < 3; ++x) W.CD[lane][x] = sm[c].R[x] - sm[d].R[x];
+    }
+    const int F = TB == 2 ? (sm[t.A].ao_p < 0 ? -1 : sm[t.A].ao_p + t.f) : sm[t.A].ao_s;
+    const int bs = sm[t.B].ao_s, bp = sm[t.B].ao_p;
+    T *o = out + mols[t.m].eri_off;
+    __syncwarp();
+    auto perm = [&](int x) { return t.f + x >= 3 ? t.f + x - 3 : t.f + x; };
+#pragma unroll 1
+    for (int k8 = 0; k8 < t.cnt; k8 += 8) {
+      const int kk = k8 + qd, n = W.n[kk];
+      const int npass = (__reduce_max_sync(0xffffffffu, n) + 3) >> 2;
+      T acc[NB][NO];
+#pragma unroll
+      for (int b = 0; b < NB; ++b)
+#pragma unroll
+        for (int e = 0; e < NO; ++e) acc[b][e] = (T)0;
+#pragma unroll 1
+      for (int ps = 0; ps < npass; ++ps) {
+        const int j = 4 * ps + li;
+        const bool act = j < n;
+        T phi[NB][S::NP];
+        S::zero(phi);
+        B2EriKet<T> q;
+        if (act) {
+          b2es_ket(pr[(p0 + kf + kk) * B2_MAXPP + j], t.f, W.CD[kk], q);
+#pragma unroll 1
+          for (int p = 0; p < nb; ++p) S::quartet(W.bra[p], q, tab, phi);
+        }
+        const bool hi = li & 2, od = li & 1;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          T v[S::NK];
+#pragma unroll
+          for (int e = 0; e < S::NK; ++e) v[e] = (T)0;
+          if (act) S::ket(q, phi[b], v);
+          T h[S::NK / 2];
+#pragma unroll
+          for (int e = 0; e < S::NK / 2; ++e) {
+            const T keep = hi ? v[S::NK / 2 + e] : v[e];
+            h[e] = keep + __shfl_xor_sync(0xffffffffu, hi ? v[e] : v[S::NK / 2 + e], 2);
+          }
+#pragma unroll
+          for (int e = 0; e < NO; ++e) {
+            const T keep = od ? h[NO + e] : h[e];
+            acc[b][e] += keep + __shfl_xor_sync(0xffffffffu, od ? h[e] : h[NO + e], 1);
+          }
+        }
+      }
+      if (kk < t.cnt) {
+        const int cs = W.ao[kk][0], cp = W.ao[kk][1], ds = W.ao[kk][2], dp = W.ao[kk][3];
+        const bool same2 = W.same[kk] & 1, same = W.same[kk] & 2;
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+          const int jb = b == 0 ? bs : (bp < 0 ? -1 : bp + perm(b - 1));
+          if constexpr (TK == 1) {
+            const int l = li == 0 ? ds : (dp < 0 ? -1 : dp + perm(li - 1));
+            b2es_put(o, F, jb, cs, l, t.A == t.B, same2, same, acc[b][0]);
+          } else {
+            const int k = li == 0 ? cs : (cp < 0 ? -1 : cp + perm(li - 1));
+#pragma unroll
+            for (int d = 0; d < 4; ++d) {
+              const int l = d == 0 ? ds : (dp < 0 ? -1 : dp + perm(d - 1));
+              b2es_put(o, F, jb, k, l, t.A == t.B, same2, same, acc[b][d]);
+            }
+          }
+        }
       }
     }
-    const int kn = __shfl_down_sync(0xffffffffu, k, 1);
-    if (valid && (lane == 31 || kn != k))
-#pragma unroll
-      for (int c = 0; c < NC; ++c) s_acc[w][k][c] += a[c];
-    __syncwarp();
-  }
-  if (lane < tk.count) {
-    const B2PairInfo kp = pinfo[md.sp_off + KL];
-    float acc[S::NI][S::NJ][S::NK][S::NL], a[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) a[c] = s_acc[w][lane][c];
-    b2_fl_unflatten<S>(a, acc);
-    S::template store<float>(out + md.eri_off, bp, kp, acc);
   }
 }
 
@@ -183,242 +290,102 @@ static void b2_eri_group(const B2PlanDev &P, const B2EriTask *tasks, long long n
   }
 }
 
-// batch plans: the float32 classes with at most 27 components take the flattened kernel
-template <typename T, int LI, int LJ, int LK, int LL>
-static void b2_eri_group_batch(const B2PlanDev &P, const B2EriTask *tasks, long long n,
-                               const B2PairPrim<T> *pp, T *out, cudaStream_t st) {
-  constexpr int NC = (LI ? 3 : 1) * (LJ ? 3 : 1) * (LK ? 3 : 1) * (LL ? 3 : 1);
-  if constexpr (std::is_same<T, float>::value && NC <= 27) {
-    const long long maxg = 4 * ((1ll << 31) - 1);
-    for (long long t0 = 0; t0 < n; t0 += maxg) {
-      const long long nt = std::min(maxg, n - t0);
-      k_eri_fl<LI, LJ, LK, LL><<<(unsigned)((nt + 3) / 4), 128, 0, st>>>(
-          tasks + t0, nt, P.mols, P.pinfo, pp, P.pp32_n, P.cls_list, P.boys32, out);
-      b2_count_launches(1);
-    }
+// The six class kernels write disjoint entries of the s8 lists, so they run side by side on the
+// plan's bucket streams (forked from and joined back to `st` with events), the largest first.
+template <typename T, int TB, int TK>
+static int b2_eri_class(const B2PlanDev &P, int cls, const typename B2EriPrimOf<T>::type *pr, T *out, cudaStream_t st) {
+  const long long n = P.su.n_task[cls];
+  if (n <= 0) return B2_OK;
+  const unsigned nb = (unsigned)std::min<long long>((n + 3) / 4, 148ll * 8);
+  const long long *off = P.su.off + cls * (P.h.nmol + 1ll);
+  if constexpr (TB == 0 && TK == 0) {
+    k_eri_ss<T><<<nb, 128, 0, st>>>(off, P.h.nmol, P.su.mol, P.mols, P.su.su, pr, P.su.pn, b2_boys_table<T>(P), out);
   } else {
-    b2_eri_group<T, LI, LJ, LK, LL>(P, tasks, n, pp, out, st);
+    const size_t sm = sizeof(T) * B2_BOYS_NT * B2_BOYS_NM + 4 * sizeof(B2EriWarp<T>);
+    B2_CUDA_TRY(cudaFuncSetAttribute(k_eri_su<T, TB, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_eri_su<T, TB, TK><<<nb, 128, sm, st>>>(off, P.h.nmol, P.su.mol, P.mols, P.su.su, pr, P.su.pn,
+                                             b2_boys_table<T>(P), out);
   }
-}
-
-// The 16 class kernels write disjoint entries of the s8 lists, so they run side by side: each on
-// one of the plan's bucket streams (round robin, forked from and joined back to `st` with
-// events), which fills the GPU across the tails of the individual launches.
-template <typename T>
-static void b2_eri_all(const B2PlanDev &P, const B2EriTask *tasks, const std::vector<long long> &g,
-                       const B2PairPrim<T> *pp, T *out, cudaStream_t st) {
-  const bool fork = P.bkt_stream[0] != nullptr;
-  if (fork) cudaEventRecord(P.bkt_ev[B2_NBKT], st);
-  int k = 0;
-  auto sk = [&]() -> cudaStream_t {
-    if (!fork) return st;
-    cudaStream_t s = P.bkt_stream[k % B2_NBKT];
-    if (k < B2_NBKT) cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0);
-    ++k;
-    return s;
-  };
-#define B2_G(grp, LI, LJ, LK, LL)                                                            \
-  if (g[grp + 1] > g[grp])                                                                   \
-    b2_eri_group_batch<T, LI, LJ, LK, LL>(P, tasks + g[grp], g[grp + 1] - g[grp], pp, out, sk());
-  B2_G(0, 0, 0, 0, 0) B2_G(1, 0, 0, 1, 0) B2_G(2, 0, 0, 0, 1) B2_G(3, 0, 0, 1, 1)
-  B2_G(4, 1, 0, 0, 0) B2_G(5, 1, 0, 1, 0) B2_G(6, 1, 0, 0, 1) B2_G(7, 1, 0, 1, 1)
-  B2_G(8, 0, 1, 0, 0) B2_G(9, 0, 1, 1, 0) B2_G(10, 0, 1, 0, 1) B2_G(11, 0, 1, 1, 1)
-  B2_G(12, 1, 1, 0, 0) B2_G(13, 1, 1, 1, 0) B2_G(14, 1, 1, 0, 1) B2_G(15, 1, 1, 1, 1)
-#undef B2_G
-  if (fork)
-    for (int b = 0; b < B2_NBKT && b < k; ++b) {
-      cudaEventRecord(P.bkt_ev[b], P.bkt_stream[b]);
-      cudaStreamWaitEvent(st, P.bkt_ev[b], 0);
-    }
-}
-
-// Work list on the device.  Item it = 4 sp + c (sp: global bra shell pair, c: ket class) owns
-// ceil(cnt / chunk) x nsub tasks, cnt = class-c kets KL <= (I,I); tasks are grouped by
-// (bra class, c) and within a group ordered by item (the order of b2_eri_tasks).  Three passes
-// over tiles of B2_TT items: per-tile group sums, an exclusive scan of each group over the
-// tiles (group totals to the host, which sizes the list), then each tile writes its tasks.
-// A 4096-molecule batch has ~6e6 items and ~1.7e7 tasks.
-#define B2_TT 1024                 // items per tile: 256 threads x 4 consecutive items
-
-__device__ __forceinline__ void b2_task_item(const B2MolDev *__restrict__ mols, int nmol,
-                                             const B2PairInfo *__restrict__ pinfo,
-                                             const int *__restrict__ cls_cnt, long long it, long long n_items,
-                                             int chunk, int split_p, int &grp, int &n, int &mol, int &IJ,
-                                             int &cnt, int &nsub) {
-  grp = 0; n = 0; mol = 0; IJ = 0; cnt = 0; nsub = 1;
-  if (it >= n_items) return;
-  const long long sp = it >> 2;
-  const int c = (int)(it & 3);
-  int lo = 0, hi = nmol - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (mols[mid].sp_off <= sp) lo = mid; else hi = mid - 1;
-  }
-  const B2MolDev &md = mols[lo];
-  const B2PairInfo pi = pinfo[sp];
-  const int spcut = (int)b2_tri(pi.I) + pi.I;
-  mol = lo;
-  IJ = (int)(sp - md.sp_off);
-  cnt = cls_cnt[4ll * md.sp_off + (long long)c * md.nsp + spcut];
-  nsub = (split_p && pi.lI) ? 3 : 1;
-  grp = (pi.lI + 2 * pi.lJ) * 4 + c;
-  n = (cnt + chunk - 1) / chunk * nsub;
-}
-
-__global__ void __launch_bounds__(256)
-k_task_tile_sums(const B2MolDev *__restrict__ mols, int nmol, const B2PairInfo *__restrict__ pinfo,
-                 const int *__restrict__ cls_cnt, long long n_items, int chunk, int split_p,
-                 long long *__restrict__ tile_sum) {
-  __shared__ int s[16];
-  if (threadIdx.x < 16) s[threadIdx.x] = 0;
-  __syncthreads();
-  const long long i0 = (long long)blockIdx.x * B2_TT + 4 * threadIdx.x;
-  for (int k = 0; k < 4; ++k) {
-    int grp, n, mol, IJ, cnt, nsub;
-    b2_task_item(mols, nmol, pinfo, cls_cnt, i0 + k, n_items, chunk, split_p, grp, n, mol, IJ, cnt, nsub);
-    if (n) atomicAdd(&s[grp], n);
-  }
-  __syncthreads();
-  if (threadIdx.x < 16) tile_sum[(long long)blockIdx.x * 16 + threadIdx.x] = s[threadIdx.x];
-}
-
-// one CTA per group: exclusive scan of the group's tile sums in place; total -> gtot[group]
-__global__ void __launch_bounds__(1024)
-k_task_scan(long long *__restrict__ tile_sum, long long ntile, long long *__restrict__ gtot) {
-  __shared__ long long wsum[32];
-  const int g = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  long long carry = 0;
-  for (long long t0 = 0; t0 < ntile; t0 += 1024) {
-    const long long t = t0 + threadIdx.x;
-    const long long v = t < ntile ? tile_sum[t * 16 + g] : 0;
-    long long x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const long long y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w] = x;
-    __syncthreads();
-    if (w == 0) {
-      long long z = wsum[lane];
-      for (int o = 1; o < 32; o <<= 1) {
-        const long long y = __shfl_up_sync(0xffffffffu, z, o);
-        if (lane >= o) z += y;
-      }
-      wsum[lane] = z;                                    // inclusive over warps
-    }
-    __syncthreads();
-    const long long excl = carry + (w ? wsum[w - 1] : 0) + x - v;
-    if (t < ntile) tile_sum[t * 16 + g] = excl;
-    carry += wsum[31];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) gtot[g] = carry;
-}
-
-__global__ void __launch_bounds__(256)
-k_task_write(const B2MolDev *__restrict__ mols, int nmol, const B2PairInfo *__restrict__ pinfo,
-             const int *__restrict__ cls_cnt, long long n_items, int chunk, int split_p,
-             const long long *__restrict__ tile_base, const long long *__restrict__ goff,
-             B2EriTask *__restrict__ tasks) {
-  __shared__ long long wsum[8][16];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const long long i0 = (long long)blockIdx.x * B2_TT + 4 * threadIdx.x;
-  int grp[4], n[4], mol[4], IJ[4], cnt[4], nsub[4];
-  for (int k = 0; k < 4; ++k)
-    b2_task_item(mols, nmol, pinfo, cls_cnt, i0 + k, n_items, chunk, split_p, grp[k], n[k], mol[k], IJ[k],
-                 cnt[k], nsub[k]);
-  // per group: exclusive prefix of this thread's task counts over the CTA (warp scans + warp sums)
-  long long off[4];
-  for (int g = 0; g < 16; ++g) {
-    int v = 0;
-    for (int k = 0; k < 4; ++k) v += grp[k] == g ? n[k] : 0;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
-    }
-    if (lane == 31) wsum[w][g] = x;
-    int run = x - v;                                     // exclusive within the warp
-    for (int k = 0; k < 4; ++k)
-      if (grp[k] == g) { off[k] = run; run += n[k]; }
-  }
-  __syncthreads();
-  for (int k = 0; k < 4; ++k) {
-    if (!n[k]) continue;
-    const int g = grp[k];
-    long long o = goff[g] + tile_base[(long long)blockIdx.x * 16 + g] + off[k];
-    for (int v = 0; v < w; ++v) o += wsum[v][g];
-    const int c = (int)((i0 + k) & 3);
-    for (int s0 = 0; s0 < cnt[k]; s0 += chunk)
-      for (int sub = 0; sub < nsub[k]; ++sub)
-        tasks[o++] = B2EriTask{mol[k], IJ[k], c, s0, min(chunk, cnt[k] - s0), nsub[k] > 1 ? sub : -1};
-  }
-}
-
-static int b2_eri_task_upload(B2PlanDev &P, int precision, cudaStream_t st) {
-  B2EriTask *&dst = precision == 64 ? P.eri_tasks64 : P.eri_tasks32;
-  std::vector<long long> &goff = precision == 64 ? P.eri_goff64 : P.eri_goff32;
-  if (dst) return B2_OK;
-  const int chunk = 32;                          // kets per warp task
-  const int split_p = precision == 64 ? 1 : 0;
-  const long long n_items = 4ll * P.h.n_sp;
-  const long long ntile = std::max(1ll, (n_items + B2_TT - 1) / B2_TT);
-  long long *scratch = nullptr;                  // tile sums (16 per tile), group totals, group starts
-  B2_CUDA_TRY(b2_dmalloc_t(&scratch, sizeof(long long) * (size_t)(16 * ntile + 32), st));
-  long long *gtot = scratch + 16 * ntile, *dgoff = gtot + 16;
-  std::vector<long long> tot(16, 0);
-  int rc = B2_OK;
-  if (n_items > 0) {
-    k_task_tile_sums<<<(unsigned)ntile, 256, 0, st>>>(P.mols, P.h.nmol, P.pinfo, P.cls_cnt, n_items, chunk,
-                                                      split_p, scratch);
-    k_task_scan<<<16, 1024, 0, st>>>(scratch, ntile, gtot);
-    b2_count_launches(2);
-    if (cudaMemcpyAsync(tot.data(), gtot, sizeof(long long) * 16, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-      rc = B2_ERR_CUDA;
-  }
-  std::vector<long long> g(17, 0);
-  for (int k = 0; k < 16; ++k) g[k + 1] = g[k] + tot[k];
-  if (!rc && g[16] >= (1ll << 31)) rc = B2_ERR_SIZE;
-  if (!rc && b2_dmalloc_t(&dst, sizeof(B2EriTask) * std::max<size_t>(1, (size_t)g[16]), st) != cudaSuccess) {
-    dst = nullptr;
-    rc = B2_ERR_CUDA;
-  }
-  if (!rc && n_items > 0) {
-    if (cudaMemcpyAsync(dgoff, g.data(), sizeof(long long) * 16, cudaMemcpyHostToDevice, st) != cudaSuccess)
-      rc = B2_ERR_CUDA;
-    else {
-      k_task_write<<<(unsigned)ntile, 256, 0, st>>>(P.mols, P.h.nmol, P.pinfo, P.cls_cnt, n_items, chunk,
-                                                    split_p, scratch, dgoff, dst);
-      b2_count_launches(1);
-      if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) rc = B2_ERR_CUDA;
-    }
-  }
-  b2_dfree(scratch, st);
-  if (rc) {
-    b2_dfree(dst, st);
-    dst = nullptr;
-    return rc;
-  }
-  goff = g;
+  b2_count_launches(1);
+  B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
 }
 
-int b2_eri_tasks_ready(B2PlanDev &P, int precision, cudaStream_t st) {
-  if (precision != 64 && precision != 32) return B2_ERR_ARG;
-  return b2_eri_task_upload(P, precision, st);
+template <typename T>
+static int b2_eri_all(const B2PlanDev &P, const typename B2EriPrimOf<T>::type *pr, T *out, cudaStream_t st) {
+  cudaStream_t s[B2_NBKT];
+  const bool fork = P.bkt_stream[0] != nullptr;
+  if (fork) B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
+  for (int b = 0; b < B2_NBKT; ++b) {
+    s[b] = fork ? P.bkt_stream[b] : st;
+    if (fork) B2_CUDA_TRY(cudaStreamWaitEvent(s[b], P.bkt_ev[B2_NBKT], 0));
+  }
+  int rc = b2_eri_class<T, 1, 2>(P, 4, pr, out, s[0]);
+  if (!rc) rc = b2_eri_class<T, 0, 1>(P, 1, pr, out, s[1]);
+  if (!rc) rc = b2_eri_class<T, 1, 1>(P, 2, pr, out, s[2]);
+  if (!rc) rc = b2_eri_class<T, 0, 0>(P, 0, pr, out, s[3]);
+  if (!rc) rc = b2_eri_class<T, 2, 2>(P, 5, pr, out, s[4]);
+  if (!rc) rc = b2_eri_class<T, 0, 2>(P, 3, pr, out, s[4]);
+  if (fork)
+    for (int b = 0; b < B2_NBKT; ++b) {
+      cudaEventRecord(P.bkt_ev[b], s[b]);
+      cudaStreamWaitEvent(st, P.bkt_ev[b], 0);
+    }
+  return rc;
 }
 
 int b2_launch_eri_s8(B2PlanDev &P, int precision, void *out, cudaStream_t st) {
-  if (precision != 64 && precision != 32) return B2_ERR_ARG;
-  int rc = b2_eri_task_upload(P, precision, st);
-  if (rc) return rc;
-  if (precision == 64)
-    b2_eri_all<double>(P, P.eri_tasks64, P.eri_goff64, P.pp64, (double *)out, st);
-  else
-    b2_eri_all<float>(P, P.eri_tasks32, P.eri_goff32, P.pp32, (float *)out, st);
-  B2_CUDA_TRY(cudaGetLastError());
-  return B2_OK;
+  if (precision == 64) return b2_eri_all<double>(P, P.su.pr64, (double *)out, st);
+  if (precision == 32) return b2_eri_all<float>(P, P.su.pr32, (float *)out, st);
+  return B2_ERR_ARG;
+}
+
+// ------------------------------------------------------------------ super-shell tables
+// primitive pairs of every super-shell pair, one thread per pair
+__global__ void __launch_bounds__(128)
+k_su_prims(const B2gsMol *__restrict__ gm, const long long *__restrict__ poff, int nmol,
+           const B2gSuper *__restrict__ su, B2gPrim *__restrict__ pr64, B2gPrim32 *__restrict__ pr32,
+           B2gCount *__restrict__ pn) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= poff[nmol]) return;
+  const int m = b2_eri_find(poff, nmol, t);
+  const B2gsMol g = gm[m];
+  int A, B;
+  b2gs_pair(g.ns, g.np, (int)(t - g.pr_off), A, B);
+  pn[t] = b2gs_pair_prims(su[g.su_off + A], su[g.su_off + B], pr64 + t * B2_MAXPP, pr32 + t * B2_MAXPP);
+}
+
+// host tables: super shells, molecules, and the prefixes over molecules of the tasks of the six
+// integral classes, of the pairs, of the six gradient classes' tasks and of the one-electron
+// gradient's slices
+static const int b2_eri_tb[6] = {0, 0, 1, 0, 1, 2}, b2_eri_tk[6] = {0, 1, 1, 2, 2, 2};
+
+void b2_su_host(const B2PlanHost &h, std::vector<B2gSuper> &su, std::vector<B2gsMol> &gm,
+                std::vector<long long> &off) {
+  const int nmol = h.nmol;
+  gm.resize(nmol);
+  off.assign((size_t)B2_SU_NOFF * (nmol + 1), 0);
+  su.clear();
+  su.reserve(h.n_sh);
+  std::vector<B2gSuper> tmp(std::max(1, h.max_nbas));
+  for (int m = 0; m < nmol; ++m) {
+    const B2MolDev &md = h.mols[m];
+    int nt = 0;
+    const int ns = b2gs_supers(h.shells.data() + md.sh_off, md.nbas, tmp.data(), &nt), np = nt - ns;
+    auto add = [&](int k, long long n) {
+      long long *o = off.data() + k * (nmol + 1ll) + m;
+      o[1] = o[0] + n;
+      return o[0];
+    };
+    for (int c = 0; c < 6; ++c)
+      add(c, (long long)b2es_nbra(ns, np, b2_eri_tb[c], b2_eri_tk[c]) * ((b2es_npair(ns, np, b2_eri_tk[c]) + 31) / 32));
+    const long long pr0 = add(B2_SU_PAIRS, b2gs_npair(ns, np));
+    for (int c = 0; c < 6; ++c)
+      add(B2_SU_GRAD + c, (long long)b2gs_nslice(ns, np, b2gs_tb[c]) * ((b2gs_nket(ns, np, b2gs_tk[c]) + 31) / 32));
+    add(B2_SU_GRAD1, b2gs_nslice(ns, np, 0) + b2gs_nslice(ns, np, 1) + b2gs_nslice(ns, np, 2));
+    gm[m] = B2gsMol{ns, np, (int)su.size(), 0, pr0};
+    su.insert(su.end(), tmp.begin(), tmp.begin() + nt);
+  }
 }
 
 // ============================================================================================
@@ -590,72 +557,31 @@ extern "C" int b2_int2e_sph_s8_noalloc(const int *atm, int natm, const int *bas,
   return B2_OK;
 }
 
-// primitive-pair tables of every shell pair of the batch (float64 and float32 copies, screened
-// and packed), one thread per shell pair; same code as the host test build
-__global__ void k_pair_prims(const B2MolDev *__restrict__ mols, int nmol, const B2Shell *__restrict__ shells,
-                             const B2PairInfo *__restrict__ pinfo, long long n_sp,
-                             B2PairPrim<double> *__restrict__ pp64, B2PairPrim<float> *__restrict__ pp32,
-                             unsigned char *__restrict__ pp32_n) {
-  const long long gp = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (gp >= n_sp) return;
-  int lo = 0, hi = nmol - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (mols[mid].sp_off <= gp) lo = mid; else hi = mid - 1;
-  }
-  const B2PairInfo pi = pinfo[gp];
-  const int sh = mols[lo].sh_off;
-  int n32 = 0;
-  b2_pair_prims_packed(shells[sh + pi.I], shells[sh + pi.J], pp64 + gp * B2_MAXPP, pp32 + gp * B2_MAXPP, &n32);
-  pp32_n[gp] = (unsigned char)n32;
-}
-
-// shell-pair tables of every molecule, one warp per molecule: pair info, the class lists
-// (pairs of each angular class in ascending order, from cls_start) and the inclusive class
-// prefix counts cls_cnt[4 sp_off + c nsp + sp] = #{class-c pairs <= sp}; the host test build
-// fills the same tables (b2_plan_build with pair tables)
+// shell pairs (I >= J) of every molecule, one warp per molecule (the one-electron kernel's order)
 __global__ void __launch_bounds__(256)
 k_plan_pairs(const B2MolDev *__restrict__ mols, int nmol, const B2Shell *__restrict__ shells,
-             B2PairInfo *__restrict__ pinfo, int *__restrict__ cls_list, int *__restrict__ cls_cnt) {
+             B2PairInfo *__restrict__ pinfo) {
   const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
   if (m >= nmol) return;                           // whole warp
   const B2MolDev md = mols[m];
   const B2Shell *S = shells + md.sh_off;
-  const unsigned le = (2u << lane) - 1u;           // lanes <= this one (lane 31: all)
-  int run[4] = {0, 0, 0, 0};
-  for (int base = 0; base < md.nsp; base += 32) {
-    const int sp = base + lane;
-    int c = -1;
-    if (sp < md.nsp) {
-      const int I = (int)b2_untri(sp), J = sp - (int)b2_tri(I);
-      const int lI = S[I].l, lJ = S[J].l;
-      pinfo[md.sp_off + sp] = B2PairInfo{I, J, lI, lJ, S[I].ao0, S[J].ao0, S[I].nprim * S[J].nprim, 0};
-      c = b2_class(lI, lJ);
-    }
-    for (int cc = 0; cc < 4; ++cc) {
-      const unsigned mk = __ballot_sync(0xffffffffu, c == cc);
-      const int incl = run[cc] + __popc(mk & le);
-      if (sp < md.nsp) cls_cnt[4ll * md.sp_off + (long long)cc * md.nsp + sp] = incl;
-      if (c == cc) cls_list[md.sp_off + md.cls_start[cc] + incl - 1] = sp;
-      run[cc] += __popc(mk);
-    }
+  for (int sp = threadIdx.x & 31; sp < md.nsp; sp += 32) {
+    const int I = (int)b2_untri(sp), J = sp - (int)b2_tri(I);
+    pinfo[md.sp_off + sp] = B2PairInfo{I, J, S[I].l, S[J].l, S[I].ao0, S[J].ao0, S[I].nprim * S[J].nprim, 0};
   }
 }
 
+// device tables of a plan that kernels build: shell pairs and the super-shell pairs' primitives
 int b2_build_pairs(B2PlanDev &P, cudaStream_t st) {
-  const long long nsp = P.h.n_sp, n = nsp * B2_MAXPP;
+  const long long nsp = P.h.n_sp, np = P.su.n_pair;
   B2_CUDA_TRY(b2_dmalloc_t(&P.pinfo, sizeof(B2PairInfo) * (size_t)std::max(1ll, nsp), st));
-  B2_CUDA_TRY(b2_dmalloc_t(&P.cls_list, sizeof(int) * (size_t)std::max(1ll, nsp), st));
-  B2_CUDA_TRY(b2_dmalloc_t(&P.cls_cnt, sizeof(int) * (size_t)std::max(1ll, 4 * nsp), st));
-  B2_CUDA_TRY(b2_dmalloc_t(&P.pp64, sizeof(B2PairPrim<double>) * (size_t)std::max(1ll, n), st));
-  B2_CUDA_TRY(b2_dmalloc_t(&P.pp32, sizeof(B2PairPrim<float>) * (size_t)std::max(1ll, n), st));
-  B2_CUDA_TRY(b2_dmalloc_t(&P.pp32_n, (size_t)std::max(1ll, nsp), st));
-  if (n > 0) {
-    k_plan_pairs<<<(unsigned)((P.h.nmol + 7) / 8), 256, 0, st>>>(P.mols, P.h.nmol, P.shells, P.pinfo,
-                                                                 P.cls_list, P.cls_cnt);
-    k_pair_prims<<<(unsigned)((nsp + 127) / 128), 128, 0, st>>>(P.mols, P.h.nmol, P.shells, P.pinfo,
-                                                               nsp, P.pp64, P.pp32, P.pp32_n);
+  B2_CUDA_TRY(b2_dmalloc_t(&P.su.pr64, sizeof(B2gPrim) * B2_MAXPP * (size_t)std::max(1ll, np), st));
+  B2_CUDA_TRY(b2_dmalloc_t(&P.su.pr32, sizeof(B2gPrim32) * B2_MAXPP * (size_t)std::max(1ll, np), st));
+  B2_CUDA_TRY(b2_dmalloc_t(&P.su.pn, sizeof(B2gCount) * (size_t)std::max(1ll, np), st));
+  if (nsp > 0 && np > 0) {
+    k_plan_pairs<<<(unsigned)((P.h.nmol + 7) / 8), 256, 0, st>>>(P.mols, P.h.nmol, P.shells, P.pinfo);
+    k_su_prims<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(P.su.mol, P.su.off + B2_SU_PAIRS * (P.h.nmol + 1ll),
+                                                             P.h.nmol, P.su.su, P.su.pr64, P.su.pr32, P.su.pn);
     b2_count_launches(2);
     B2_CUDA_TRY(cudaGetLastError());
   }
@@ -663,24 +589,24 @@ int b2_build_pairs(B2PlanDev &P, cudaStream_t st) {
 }
 
 // Work the float32 ERI kernels do for a plan: primitive quartets evaluated (bra survivors x ket
-// survivors of every shell quartet of the task list) and their arithmetic by the per-class
-// counts of eri_flops.h (generated from eri_sq.cuh by eri_flops_count.cu).  One thread per task.
+// survivors of every slice quartet) and their arithmetic by the per-class counts of eri_flops.h
+// (generated from eri_su.cuh by eri_flops_count.cu): per primitive quartet, and per bra slice and
+// ket primitive for the ket's polynomial.  One thread per task.
+template <int TB, int TK>
 __global__ void __launch_bounds__(256)
-k_eri_count(const B2EriTask *__restrict__ tasks, long long n, const B2MolDev *__restrict__ mols,
-            const int *__restrict__ cls_list, const unsigned char *__restrict__ ppn, double fl, double sp,
-            double *__restrict__ out) {
+k_eri_count(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
+            const B2gCount *__restrict__ pn, double fl, double sp, double kf, double *__restrict__ out) {
   __shared__ double red[3][8];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double q = 0;
-  if (t < n) {
-    const B2EriTask tk = tasks[t];
-    const B2MolDev md = mols[tk.mol];
-    const double nb = ppn[md.sp_off + tk.IJ];
-    int nq = 0;
-    for (int k = 0; k < tk.count; ++k) nq += ppn[md.sp_off + cls_list[md.sp_off + md.cls_start[tk.cls] + tk.start + k]];
-    q = nb * nq;
+  double q = 0, e = 0;
+  B2gsMol g;
+  B2EriTaskSu tk;
+  if (t < toff[nmol] && b2_eri_task<TB, TK>(toff, nmol, gms, t, g, tk)) {
+    const int k0 = b2es_first(g.ns, g.np, TK) + tk.k0;
+    for (int k = 0; k < tk.cnt; ++k) e += pn[g.pr_off + k0 + k].x;
+    q = e * pn[g.pr_off + tk.pair].x;
   }
-  double v[3] = {q, q * fl, q * sp};
+  double v[3] = {q, q * fl + e * kf, q * sp};
   for (int c = 0; c < 3; ++c)
     for (int o = 16; o > 0; o >>= 1) v[c] += __shfl_down_sync(0xffffffffu, v[c], o);
   if ((threadIdx.x & 31) == 0)
@@ -693,21 +619,25 @@ k_eri_count(const B2EriTask *__restrict__ tasks, long long n, const B2MolDev *__
   }
 }
 
+template <int C>
+static void b2_eri_count_class(const B2PlanDev &P, double *d) {
+  constexpr int TB = C == 5 ? 2 : (C == 2 || C == 4 ? 1 : 0), TK = C == 0 ? 0 : (C <= 2 ? 1 : 2);
+  const long long n = P.su.n_task[C];
+  if (n > 0) {
+    k_eri_count<TB, TK><<<(unsigned)((n + 255) / 256), 256>>>(
+        P.su.off + C * (P.h.nmol + 1ll), P.h.nmol, P.su.mol, P.su.pn, (double)B2_ERI_FLOPS[C],
+        (double)B2_ERI_SPECIAL[C], (double)B2_ERI_KET_FLOPS[C], d);
+    b2_count_launches(1);
+  }
+  if constexpr (C < 5) b2_eri_count_class<C + 1>(P, d);
+}
+
 int b2_launch_eri_count(B2PlanDev &P, double *host_out) {
-  int rc = b2_eri_task_upload(P, 32, nullptr);
-  if (rc) return rc;
   double *d = nullptr;
   B2_CUDA_TRY(b2_dmalloc_t(&d, 3 * sizeof(double)));
   B2_CUDA_TRY(cudaMemset(d, 0, 3 * sizeof(double)));
-  const std::vector<long long> &g = P.eri_goff32;
-  for (int grp = 0; grp < 16; ++grp) {
-    const long long n = g[grp + 1] - g[grp];
-    if (n <= 0) continue;
-    k_eri_count<<<(unsigned)((n + 255) / 256), 256>>>(P.eri_tasks32 + g[grp], n, P.mols, P.cls_list, P.pp32_n,
-                                                       (double)B2_ERI_FLOPS[grp], (double)B2_ERI_SPECIAL[grp], d);
-    b2_count_launches(1);
-  }
-  rc = cudaMemcpy(host_out, d, 3 * sizeof(double), cudaMemcpyDeviceToHost) == cudaSuccess ? B2_OK : B2_ERR_CUDA;
+  b2_eri_count_class<0>(P, d);
+  const int rc = cudaMemcpy(host_out, d, 3 * sizeof(double), cudaMemcpyDeviceToHost) == cudaSuccess ? B2_OK : B2_ERR_CUDA;
   b2_dfree(d);
   return rc;
 }

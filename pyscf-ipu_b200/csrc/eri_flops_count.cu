@@ -1,6 +1,6 @@
 // Per-class arithmetic of one primitive quartet of the float32 ERI kernels, counted on the host
-// by running the kernels' own shell-quartet code (eri_sq.cuh, B2Sq<T,...>::quartet with its Boys
-// evaluation) on a counting number type.  Writes eri_flops.h, which bench.py's ERI roofline uses:
+// by running the kernels' own code (eri_su.cuh, B2Es<T,...>::quartet with its Boys evaluation and
+// B2Es<T,...>::ket) on a counting number type.  Writes eri_flops.h, which bench.py's ERI roofline uses:
 //
 //   nvcc -std=c++17 -I. -I../../include -x cu eri_flops_count.cu -o /tmp/eri_flops && /tmp/eri_flops > eri_flops.h
 //
@@ -12,7 +12,7 @@
 // F_0 alone on its error-function branch (erf counts as one special function).
 #include <cstdio>
 #include <cmath>
-#include "eri_sq.cuh"
+#include "eri_su.cuh"
 
 static long long g_flops = 0, g_special = 0;
 
@@ -65,9 +65,9 @@ inline CF erf(CF a) { if (!a.k) ++g_special; CF c = a; c.v = std::erf(a.v); retu
 template <> struct B2BoysTerms<CF> { static constexpr int n = B2BoysTerms<float>::n; };
 template <> struct B2BoysErfF0<CF> { static constexpr bool value = B2BoysErfF0<float>::value; };
 
-template <int LI, int LJ, int LK, int LL>
-static void count(long long &fl, long long &sp) {
-  using S = B2Sq<CF, LI, LJ, LK, LL, -1>;
+template <int TB, int TK>
+static void count(long long &fl, long long &sp, long long &kf) {
+  using S = B2Es<CF, TB, TK>;
   static CF tab[B2_BOYS_NT * B2_BOYS_NM];
   static bool filled = false;
   if (!filled) {
@@ -76,40 +76,43 @@ static void count(long long &fl, long long &sp) {
     for (int i = 0; i < B2_BOYS_NT * B2_BOYS_NM; ++i) tab[i] = CF::var(t64[i]);
     filled = true;
   }
-  B2PairPrim<CF> A, B;
+  B2EriBra<CF> A;
+  B2EriKet<CF> B;
   const double a[12] = {1.3, 0.4, 0.2, -0.1, 0.3, 0.25, -0.2, 0.1, 0.9, 0.35, 0.7, 0.6};
-  CF *pa = &A.zeta, *pb = &B.zeta;             // the struct is a run of T fields
-  for (int i = 0; i < (int)(sizeof(A) / sizeof(CF)); ++i) {
-    pa[i] = CF::var(a[i % 12] + 0.01 * i);
-    pb[i] = CF::var(a[(i + 5) % 12] - 0.02 * i);
-  }
-  CF acc[S::NI][S::NJ][S::NK][S::NL];
-  S::zero(acc);
-  for (int x = 0; x < S::NI; ++x)
-    for (int y = 0; y < S::NJ; ++y)
-      for (int z = 0; z < S::NK; ++z)
-        for (int w = 0; w < S::NL; ++w) acc[x][y][z][w] = CF::var(0.0);
+  CF *pa = &A.kS, *pb = &B.z;                  // the structs are runs of T fields
+  for (int i = 0; i < (int)(sizeof(A) / sizeof(CF)); ++i) pa[i] = CF::var(a[i % 12] + 0.01 * i);
+  for (int i = 0; i < (int)(sizeof(B) / sizeof(CF)); ++i) pb[i] = CF::var(a[(i + 5) % 12] + 0.02 * i);
+  CF phi[S::NB][S::NP], out[S::NK];
+  for (int b = 0; b < S::NB; ++b)
+    for (int k = 0; k < S::NP; ++k) phi[b][k] = CF::var(0.0);
   g_flops = g_special = 0;
-  S::quartet(A, B, tab, acc);
+  S::quartet(A, B, tab, phi);
   fl = g_flops;
   sp = g_special;
+  g_flops = 0;
+  for (int b = 0; b < S::NB; ++b) S::ket(B, phi[b], out);
+  kf = g_flops;
 }
 
 int main() {
-  long long f[16], s[16];
-#define C(g, LI, LJ, LK, LL) count<LI, LJ, LK, LL>(f[g], s[g]);
-  C(0, 0, 0, 0, 0) C(1, 0, 0, 1, 0) C(2, 0, 0, 0, 1) C(3, 0, 0, 1, 1)
-  C(4, 1, 0, 0, 0) C(5, 1, 0, 1, 0) C(6, 1, 0, 0, 1) C(7, 1, 0, 1, 1)
-  C(8, 0, 1, 0, 0) C(9, 0, 1, 1, 0) C(10, 0, 1, 0, 1) C(11, 0, 1, 1, 1)
-  C(12, 1, 1, 0, 0) C(13, 1, 1, 1, 0) C(14, 1, 1, 0, 1) C(15, 1, 1, 1, 1)
-#undef C
-  printf("// Generated by eri_flops_count.cu from eri_sq.cuh: arithmetic of one primitive quartet of the\n");
-  printf("// float32 ERI kernels per class combination g = (lI + 2 lJ) * 4 + (lK + 2 lL) (flops: +, -, *, /;\n");
-  printf("// special: sqrt, exp, reciprocal square root), constants folded as the compiler folds them.\n");
+  long long f[6], s[6], k[6];
+  count<0, 0>(f[0], s[0], k[0]);
+  count<0, 1>(f[1], s[1], k[1]);
+  count<1, 1>(f[2], s[2], k[2]);
+  count<0, 2>(f[3], s[3], k[3]);
+  count<1, 2>(f[4], s[4], k[4]);
+  count<2, 2>(f[5], s[5], k[5]);
+  printf("// Generated by eri_flops_count.cu from eri_su.cuh: arithmetic of one primitive quartet of the\n");
+  printf("// float32 ERI kernels per class (bra slice type, ket pair type) = (0,0) (0,1) (1,1) (0,2) (1,2) (2,2)\n");
+  printf("// (flops: +, -, *, /; special: sqrt, exp, erf, reciprocal square root), and of the ket's polynomial\n");
+  printf("// per bra slice and ket primitive, constants folded as the compiler folds them.\n");
   printf("#pragma once\n");
-  printf("static const int B2_ERI_FLOPS[16] = {");
-  for (int g = 0; g < 16; ++g) printf("%lld%s", f[g], g < 15 ? ", " : "};\n");
-  printf("static const int B2_ERI_SPECIAL[16] = {");
-  for (int g = 0; g < 16; ++g) printf("%lld%s", s[g], g < 15 ? ", " : "};\n");
+  auto row = [](const char *name, const long long *v) {
+    printf("static const int %s[6] = {", name);
+    for (int g = 0; g < 6; ++g) printf("%lld%s", v[g], g < 5 ? ", " : "};\n");
+  };
+  row("B2_ERI_FLOPS", f);
+  row("B2_ERI_SPECIAL", s);
+  row("B2_ERI_KET_FLOPS", k);
   return 0;
 }

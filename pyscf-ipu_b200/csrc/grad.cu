@@ -17,7 +17,6 @@
 // The per-term math is grad_sp.cuh and grad_math.cuh, the same code the host-check build tests
 // against the finite-difference oracle.
 #include <algorithm>
-#include <cstring>
 #include <vector>
 #include "device_plan.cuh"
 #include "devmem.cuh"
@@ -50,13 +49,7 @@ k_grad_dm(const B2MolDev *__restrict__ mols, const double *__restrict__ C, const
 
 // ---- two-electron and one-electron parts: super-shell slices (grad_sp.cuh)
 //
-// Tables of a call, in one scratch block: per molecule the super-shell and pair ranges, the super
-// shells (host), the screened primitive pairs of every super-shell pair (k_gs_prims), and the
-// task prefix of each kernel.
-struct B2gsMol {
-  int ns, np, su_off, pad;         // s-only and sp super shells, first super shell
-  long long pr_off;                // first super-shell pair
-};
+// The tables (super shells, screened primitive pairs, task prefixes) are the plan's.
 #define B2GS_TABLE (B2_BOYS_NT * B2_BOYS_NM)
 
 __device__ __forceinline__ int b2gs_find(const long long *__restrict__ off, int n, long long x) {
@@ -66,27 +59,6 @@ __device__ __forceinline__ int b2gs_find(const long long *__restrict__ off, int 
     if (off[mid] <= x) lo = mid; else hi = mid - 1;
   }
   return lo;
-}
-
-// primitive pairs of every super-shell pair, one thread per pair: the surviving ones packed
-// (nine slots per pair), their number in pn
-__global__ void __launch_bounds__(128)
-k_gs_prims(const B2gsMol *__restrict__ gm, const long long *__restrict__ poff, int nmol,
-           const B2gSuper *__restrict__ su, B2gPrim *__restrict__ pr, unsigned char *__restrict__ pn) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= poff[nmol]) return;
-  const int m = b2gs_find(poff, nmol, t);
-  const B2gsMol g = gm[m];
-  int A, B;
-  b2gs_pair(g.ns, g.np, (int)(t - g.pr_off), A, B);
-  const B2gSuper a = su[g.su_off + A], b = su[g.su_off + B];
-  int n = 0;
-  for (int p = 0; p < a.nprim; ++p)
-    for (int q = 0; q < b.nprim; ++q) {
-      B2gPrim r;
-      if (b2gs_prim(a, b, p, q, r)) pr[t * B2_MAXPP + n++] = r;
-    }
-  pn[t] = (unsigned char)n;
 }
 
 // per-warp shared memory of the two-electron kernel
@@ -157,7 +129,7 @@ template <int TB, int TK>
 __global__ void __launch_bounds__(128)
 k_grad_sp(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
           const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su, const B2gPrim *__restrict__ pr,
-          const unsigned char *__restrict__ pn, const double *__restrict__ btab, const double *__restrict__ D,
+          const B2gCount *__restrict__ pn, const double *__restrict__ btab, const double *__restrict__ D,
           double hyb, double *__restrict__ grad) {
   extern __shared__ __align__(16) unsigned char gs_smem[];
   double *tab = reinterpret_cast<double *>(gs_smem);
@@ -190,7 +162,7 @@ k_grad_sp(const long long *__restrict__ toff, int nmol, const B2gsMol *__restric
       AB[x] = sm[A].R[px] - sm[B].R[px];
       if (TB && sm[B].ao_p >= 0) bi[1 + x] = sm[B].ao_p + px;
     }
-    const int nb = pn[g.pr_off + pb];
+    const int nb = pn[g.pr_off + pb].z;
     __syncwarp();                                  // the previous task's shared memory is consumed
     if (lane < nb) b2gs_bra(pr[(g.pr_off + pb) * B2_MAXPP + lane], TB, f, AB, W.bra[lane]);
     int nq = 0, ca = 0, da = 0;
@@ -199,7 +171,7 @@ k_grad_sp(const long long *__restrict__ toff, int nmol, const B2gsMol *__restric
       const int pk = b2gs_ket_pair(g.ns, g.np, TK, k0 + lane);
       b2gs_pair(g.ns, g.np, pk, c, d);
       const B2gSuper &sc = sm[c], &sd = sm[d];
-      nq = pn[g.pr_off + pk];
+      nq = pn[g.pr_off + pk].z;
       ca = sc.atom;
       da = sd.atom;
       W.pair[lane] = pk;
@@ -287,7 +259,7 @@ k_grad_sp(const long long *__restrict__ toff, int nmol, const B2gsMol *__restric
 // primitive pairs and nuclei in its local-memory recursion tables, one CTA per molecule.
 template <int TB>
 __device__ __forceinline__ void b2gs_one(const B2gsMol &g, int i, const B2MolDev &md, const B2gSuper *__restrict__ sm,
-                                         const B2gPrim *__restrict__ prm, const unsigned char *__restrict__ pnm,
+                                         const B2gPrim *__restrict__ prm, const B2gCount *__restrict__ pnm,
                                          const double *__restrict__ xyz, const int *__restrict__ Z,
                                          const double *tab, const double *__restrict__ Dm,
                                          const double *__restrict__ Wm, double *__restrict__ gm, int lane) {
@@ -309,7 +281,7 @@ __device__ __forceinline__ void b2gs_one(const B2gsMol &g, int i, const B2MolDev
   }
 #pragma unroll
   for (int x = 0; x < 3; ++x) AB[x] = sa.R[(f + x) % 3] - sb.R[(f + x) % 3];
-  const int nb = pnm[pb];
+  const int nb = pnm[pb].z;
   double gA[3] = {0, 0, 0}, gB[3] = {0, 0, 0};
   if (lane < nb) {
     B2gBraRec r;
@@ -365,7 +337,7 @@ __device__ __forceinline__ void b2gs_one(const B2gsMol &g, int i, const B2MolDev
 __global__ void __launch_bounds__(128)
 k_grad_1e(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict__ gms,
           const B2MolDev *__restrict__ mols, const B2gSuper *__restrict__ su, const B2gPrim *__restrict__ pr,
-          const unsigned char *__restrict__ pn, const double *__restrict__ atom_xyz, const int *__restrict__ atom_z,
+          const B2gCount *__restrict__ pn, const double *__restrict__ atom_xyz, const int *__restrict__ atom_z,
           const double *__restrict__ btab, const double *__restrict__ D, const double *__restrict__ Wd,
           double *__restrict__ grad) {
   extern __shared__ __align__(16) unsigned char gs_smem[];
@@ -382,7 +354,7 @@ k_grad_1e(const long long *__restrict__ toff, int nmol, const B2gsMol *__restric
     const int n0 = b2gs_nslice(g.ns, g.np, 0), n1 = b2gs_nslice(g.ns, g.np, 1);
     const B2gSuper *sm = su + g.su_off;
     const B2gPrim *prm = pr + g.pr_off * B2_MAXPP;
-    const unsigned char *pnm = pn + g.pr_off;
+    const B2gCount *pnm = pn + g.pr_off;
     const double *xyz = atom_xyz + 3ll * md.atm_off, *Dm = D + md.mat_off, *Wm = Wd + md.mat_off;
     const int *Z = atom_z + md.atm_off;
     double *gm = grad + 3ll * md.atm_off;
@@ -531,83 +503,19 @@ k_grad_nuc(const B2MolDev *__restrict__ mols, const double *__restrict__ atom_xy
   }
 }
 
-// host tables of the slice kernels and their device copies (one scratch block, freed in stream
-// order): super shells, molecules, prefixes of the pairs, of the six two-electron classes' tasks
-// (order as launched) and of the one-electron slices
-struct B2gsTables {
-  void *block = nullptr;
-  const B2gSuper *su = nullptr;
-  const B2gsMol *gm = nullptr;
-  const long long *off = nullptr;                 // [8][nmol + 1]
-  B2gPrim *pr = nullptr;
-  unsigned char *pn = nullptr;
-  long long n[8];                                 // totals: pairs, classes 0..5, one-electron
-};
-static const int b2gs_tb[6] = {2, 2, 2, 1, 1, 0}, b2gs_tk[6] = {2, 1, 0, 1, 0, 0};
-
-static int b2gs_tables(const B2PlanDev &P, B2gsTables &T, cudaStream_t st) {
-  const int nmol = P.h.nmol;
-  std::vector<B2gSuper> su;
-  std::vector<B2gsMol> gm(nmol);
-  std::vector<long long> off(8ll * (nmol + 1), 0);
-  su.reserve(P.h.n_sh);
-  std::vector<B2gSuper> tmp(std::max(1, P.h.max_nbas));
-  for (int m = 0; m < nmol; ++m) {
-    const B2MolDev &md = P.h.mols[m];
-    int nt = 0;
-    const int ns = b2gs_supers(P.h.shells.data() + md.sh_off, md.nbas, tmp.data(), &nt), np = nt - ns;
-    gm[m] = B2gsMol{ns, np, (int)su.size(), 0, off[m]};
-    su.insert(su.end(), tmp.begin(), tmp.begin() + nt);
-    long long *o = off.data() + m;
-    o[1] = o[0] + b2gs_npair(ns, np);
-    int all = 0;
-    for (int t = 0; t < 3; ++t) all += b2gs_nslice(ns, np, t);
-    for (int c = 0; c < 6; ++c) {
-      long long *q = o + (c + 1) * (nmol + 1ll);
-      q[1] = q[0] + (long long)b2gs_nslice(ns, np, b2gs_tb[c]) * ((b2gs_nket(ns, np, b2gs_tk[c]) + 31) / 32);
-    }
-    long long *q = o + 7 * (nmol + 1ll);
-    q[1] = q[0] + all;
-  }
-  for (int k = 0; k < 8; ++k) T.n[k] = off[k * (nmol + 1ll) + nmol];
-  auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t b0 = up(sizeof(B2gSuper) * su.size()), b1 = up(sizeof(B2gsMol) * gm.size()),
-               b2 = up(sizeof(long long) * off.size()), b3 = up(sizeof(B2gPrim) * B2_MAXPP * (size_t)T.n[0]);
-  unsigned char *d = nullptr;
-  B2_CUDA_TRY(b2_dmalloc_t(&d, b0 + b1 + b2 + b3 + (size_t)T.n[0], st));
-  T.block = d;
-  T.su = reinterpret_cast<B2gSuper *>(d);
-  T.gm = reinterpret_cast<B2gsMol *>(d + b0);
-  T.off = reinterpret_cast<long long *>(d + b0 + b1);
-  T.pr = reinterpret_cast<B2gPrim *>(d + b0 + b1 + b2);
-  T.pn = d + b0 + b1 + b2 + b3;
-  std::vector<unsigned char> h(b0 + b1 + b2);
-  std::memcpy(h.data(), su.data(), sizeof(B2gSuper) * su.size());
-  std::memcpy(h.data() + b0, gm.data(), sizeof(B2gsMol) * gm.size());
-  std::memcpy(h.data() + b0 + b1, off.data(), sizeof(long long) * off.size());
-  // pageable source: the call returns once the data is staged, so h may go out of scope
-  B2_CUDA_TRY(cudaMemcpyAsync(d, h.data(), h.size(), cudaMemcpyHostToDevice, st));
-  if (T.n[0] > 0) {
-    k_gs_prims<<<(unsigned)((T.n[0] + 127) / 128), 128, 0, st>>>(T.gm, T.off, nmol, T.su, T.pr, T.pn);
-    b2_count_launches(1);
-  }
-  B2_CUDA_TRY(cudaGetLastError());
-  return B2_OK;
-}
-
 // resident CTAs of 4 warps, tasks strided over them
 static unsigned b2gs_grid(long long ntask) { return (unsigned)std::min<long long>((ntask + 3) / 4, 148ll * 8); }
 
 template <int C>
-static int b2gs_launch_2e(const B2PlanDev &P, const B2gsTables &T, const double *D, double hyb, double *grad,
-                          cudaStream_t st) {
+static int b2gs_launch_2e(const B2PlanDev &P, const double *D, double hyb, double *grad, cudaStream_t st) {
   constexpr int TB = C < 3 ? 2 : (C < 5 ? 1 : 0), TK = C == 0 ? 2 : (C == 1 || C == 3 ? 1 : 0);
-  const long long n = T.n[C + 1];
+  const long long n = P.su.n_task[B2_SU_GRAD + C];
   if (n > 0) {
     const size_t smem = sizeof(double) * B2GS_TABLE + 4 * sizeof(B2gsWarp);
     B2_CUDA_TRY(cudaFuncSetAttribute(k_grad_sp<TB, TK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_grad_sp<TB, TK><<<b2gs_grid(n), 128, smem, st>>>(T.off + (C + 1) * (P.h.nmol + 1ll), P.h.nmol, T.gm, P.mols,
-                                                        T.su, T.pr, T.pn, P.boys, D, hyb, grad);
+    k_grad_sp<TB, TK><<<b2gs_grid(n), 128, smem, st>>>(P.su.off + (B2_SU_GRAD + C) * (P.h.nmol + 1ll), P.h.nmol,
+                                                       P.su.mol, P.mols, P.su.su, P.su.pr64, P.su.pn, P.boys, D, hyb,
+                                                       grad);
     b2_count_launches(1);
   }
   return B2_OK;
@@ -615,7 +523,7 @@ static int b2gs_launch_2e(const B2PlanDev &P, const B2gsTables &T, const double 
 
 // the six two-electron classes and the one-electron part side by side on the plan's streams
 // (forked from and joined back to `st`): every kernel adds to grad with atomics
-static int b2gs_launch(const B2PlanDev &P, const B2gsTables &T, int parts, double hyb, const double *D,
+static int b2gs_launch(const B2PlanDev &P, int parts, double hyb, const double *D,
                        const double *W, double *grad, cudaStream_t st) {
   const bool fork = P.bkt_stream[0] != nullptr;
   cudaStream_t s[B2_NBKT];
@@ -626,17 +534,18 @@ static int b2gs_launch(const B2PlanDev &P, const B2gsTables &T, int parts, doubl
   }
   int rc = B2_OK;
   if (parts & 2) {
-    rc = b2gs_launch_2e<0>(P, T, D, hyb, grad, s[0]);
-    if (!rc) rc = b2gs_launch_2e<1>(P, T, D, hyb, grad, s[1]);
-    if (!rc) rc = b2gs_launch_2e<3>(P, T, D, hyb, grad, s[2]);
-    if (!rc) rc = b2gs_launch_2e<4>(P, T, D, hyb, grad, s[3]);
-    if (!rc) rc = b2gs_launch_2e<2>(P, T, D, hyb, grad, s[4]);
-    if (!rc) rc = b2gs_launch_2e<5>(P, T, D, hyb, grad, s[2]);
+    rc = b2gs_launch_2e<0>(P, D, hyb, grad, s[0]);
+    if (!rc) rc = b2gs_launch_2e<1>(P, D, hyb, grad, s[1]);
+    if (!rc) rc = b2gs_launch_2e<3>(P, D, hyb, grad, s[2]);
+    if (!rc) rc = b2gs_launch_2e<4>(P, D, hyb, grad, s[3]);
+    if (!rc) rc = b2gs_launch_2e<2>(P, D, hyb, grad, s[4]);
+    if (!rc) rc = b2gs_launch_2e<5>(P, D, hyb, grad, s[2]);
   }
-  if (!rc && (parts & 1) && T.n[7] > 0) {
-    k_grad_1e<<<b2gs_grid(T.n[7]), 128, sizeof(double) * B2GS_TABLE, s[0]>>>(
-        T.off + 7 * (P.h.nmol + 1ll), P.h.nmol, T.gm, P.mols, T.su, T.pr, T.pn, P.atom_xyz, P.atom_z, P.boys, D, W,
-        grad);
+  const long long n1 = P.su.n_task[B2_SU_GRAD1];
+  if (!rc && (parts & 1) && n1 > 0) {
+    k_grad_1e<<<b2gs_grid(n1), 128, sizeof(double) * B2GS_TABLE, s[0]>>>(
+        P.su.off + B2_SU_GRAD1 * (P.h.nmol + 1ll), P.h.nmol, P.su.mol, P.mols, P.su.su, P.su.pr64, P.su.pn, P.atom_xyz,
+        P.atom_z, P.boys, D, W, grad);
     b2_count_launches(1);
   }
   if (fork)
@@ -662,10 +571,7 @@ int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const d
     b2_count_launches(1);
   }
   if (parts & 3) {
-    B2gsTables T;
-    int rc = b2gs_tables(P, T, st);
-    if (!rc) rc = b2gs_launch(P, T, parts, hyb, D, W, grad, st);
-    b2_dfree(T.block, st);
+    const int rc = b2gs_launch(P, parts, hyb, D, W, grad, st);
     if (rc) return rc;
   }
   if (parts & 4) {

@@ -5,6 +5,7 @@
 #include "eri_sq.cuh"
 #include "grad_math.cuh"
 #include "grad_sp.cuh"
+#include "eri_su.cuh"
 #include "xc_math.cuh"
 #include <algorithm>
 #include <vector>
@@ -177,12 +178,9 @@ template <int TB, int TK>
 static void b2hc_gs_class(const std::vector<B2gSuper> &S, int ns, int np, const double *D, int N, double hyb,
                           const double *tab, double *g) {
   auto prims = [&](const B2gSuper &a, const B2gSuper &b) {
-    std::vector<B2gPrim> v;
-    for (int p = 0; p < a.nprim; ++p)
-      for (int q = 0; q < b.nprim; ++q) {
-        B2gPrim r;
-        if (b2gs_prim(a, b, p, q, r)) v.push_back(r);
-      }
+    std::vector<B2gPrim> v(B2_MAXPP);
+    B2gPrim32 f[B2_MAXPP];
+    v.resize(b2gs_pair_prims(a, b, v.data(), f).z);
     return v;
   };
   for (int i = 0; i < b2gs_nslice(ns, np, TB); ++i) {
@@ -238,10 +236,11 @@ static void b2hc_gs_one(const B2PlanHost &P, const std::vector<B2gSuper> &S, int
       wg[k] = -(A == B ? 1.0 : 2.0) * W[F * N + bb];
     }
     for (int k = 0; k < 3; ++k) AB[k] = a.R[(f + k) % 3] - b.R[(f + k) % 3];
-    for (int p = 0; p < a.nprim; ++p)
-      for (int q = 0; q < b.nprim; ++q) {
-        B2gPrim pr;
-        if (!b2gs_prim(a, b, p, q, pr)) continue;
+    B2gPrim v64[B2_MAXPP];
+    B2gPrim32 v32[B2_MAXPP];
+    const B2gCount cnt = b2gs_pair_prims(a, b, v64, v32);
+    for (int p = 0; p < cnt.z; ++p) {
+        const B2gPrim &pr = v64[p];
         B2gBraRec r;
         b2gs_bra(pr, TB, f, AB, r);
         double gk[3];
@@ -264,6 +263,59 @@ static void b2hc_gs_one(const B2PlanHost &P, const std::vector<B2gSuper> &S, int
       g[3 * b.atom + (f + k) % 3] += gB[k];
     }
   }
+}
+
+// The super-shell integrals (eri_su.cuh) on the host: every class's slice quartets in the GPU
+// kernels' enumeration, summed over primitives by the code the kernels run.
+static int b2hc_n(const B2gCount &n, const B2gPrim *) { return n.y; }
+static int b2hc_n(const B2gCount &n, const B2gPrim32 *) { return n.x; }
+template <typename T, typename PR, int TB, int TK>
+static void b2hc_es_class(const std::vector<B2gSuper> &S, int ns, int np, const std::vector<PR> &pr,
+                          const std::vector<B2gCount> &cn, const T *tab, T *out) {
+  using E = B2Es<T, TB, TK>;
+  for (int i = 0; i < b2es_nbra(ns, np, TB, TK); ++i) {
+    int bp, lim, A, B;
+    b2es_bra_of(ns, np, TB, TK, i, bp, lim);
+    b2gs_pair(ns, np, bp, A, B);
+    const int f = TB == 2 ? i - 3 * (i / 3) : 0, F = TB == 2 ? (S[A].ao_p < 0 ? -1 : S[A].ao_p + f) : S[A].ao_s;
+    const double AB[3] = {S[A].R[0] - S[B].R[0], S[A].R[1] - S[B].R[1], S[A].R[2] - S[B].R[2]};
+    const int nb = b2hc_n(cn[bp], pr.data());
+    B2EriBra<T> bra[B2_MAXPP];
+    for (int p = 0; p < nb; ++p) b2es_bra(pr[bp * B2_MAXPP + p], TB == 2, f, AB, bra[p]);
+    for (int k = 0; k < lim; ++k) {
+      const int kp = b2es_first(ns, np, TK) + k;
+      int c, d;
+      b2gs_pair(ns, np, kp, c, d);
+      const double CD[3] = {S[c].R[0] - S[d].R[0], S[c].R[1] - S[d].R[1], S[c].R[2] - S[d].R[2]};
+      T v[E::NB][E::NK] = {};
+      for (int j = 0; j < b2hc_n(cn[kp], pr.data()); ++j) {
+        B2EriKet<T> q;
+        b2es_ket(pr[kp * B2_MAXPP + j], f, CD, q);
+        T phi[E::NB][E::NP], w[E::NK];
+        E::zero(phi);
+        for (int p = 0; p < nb; ++p) E::quartet(bra[p], q, tab, phi);
+        for (int b = 0; b < E::NB; ++b) {
+          E::ket(q, phi[b], w);
+          for (int e = 0; e < E::NK; ++e) v[b][e] += w[e];
+        }
+      }
+      auto ao = [&](const B2gSuper &s, int x) { return x == 0 ? s.ao_s : (s.ao_p < 0 ? -1 : s.ao_p + (f + x - 1) % 3); };
+      for (int b = 0; b < E::NB; ++b)
+        for (int e = 0; e < E::NK; ++e)
+          b2es_put(out, F, ao(S[B], b), ao(S[c], TK == 2 ? e / 4 : 0), ao(S[d], TK == 2 ? e % 4 : e), A == B, c == d,
+                   bp == kp, v[b][e]);
+    }
+  }
+}
+template <typename T, typename PR>
+static void b2hc_es_all(const std::vector<B2gSuper> &S, int ns, int np, const std::vector<PR> &pr,
+                        const std::vector<B2gCount> &cn, const T *tab, T *out) {
+  b2hc_es_class<T, PR, 0, 0>(S, ns, np, pr, cn, tab, out);
+  b2hc_es_class<T, PR, 0, 1>(S, ns, np, pr, cn, tab, out);
+  b2hc_es_class<T, PR, 1, 1>(S, ns, np, pr, cn, tab, out);
+  b2hc_es_class<T, PR, 0, 2>(S, ns, np, pr, cn, tab, out);
+  b2hc_es_class<T, PR, 1, 2>(S, ns, np, pr, cn, tab, out);
+  b2hc_es_class<T, PR, 2, 2>(S, ns, np, pr, cn, tab, out);
 }
 
 extern "C" {
@@ -401,6 +453,36 @@ int b2hc_grad_2e_tasks(int nmol, const int *natm, const int *nbas, const int *at
   for (int i = 0; i < 3 * P.n_atm; ++i) g[i] = 0;
   *bad = 0;
   b2hc_2e_group<0>(P, tasks, goff, D, hyb, tab.data(), g, bad);
+  return 0;
+}
+
+// one molecule's s8 list by the super-shell integrals; precision 64 or 32 (out double either way,
+// entries no class writes keep their value)
+int b2hc_eri_super(int natm, int nbas, const int *atm, const int *bas, const double *env, int precision, double *out) {
+  B2PlanHost P;
+  const long long eo = 0;
+  int rc = b2_plan_build(P, 1, &natm, &nbas, atm, bas, env, &eo);
+  if (rc) return rc;
+  std::vector<double> tab(B2_BOYS_NT * B2_BOYS_NM);
+  b2_boys_fill_table(tab.data());
+  std::vector<B2gSuper> S(nbas);
+  int nt = 0;
+  const int ns = b2gs_supers(P.shells.data(), nbas, S.data(), &nt), np = nt - ns, n = b2gs_npair(ns, np);
+  std::vector<B2gPrim> p64((size_t)n * B2_MAXPP);
+  std::vector<B2gPrim32> p32((size_t)n * B2_MAXPP);
+  std::vector<B2gCount> cn(n);
+  for (int k = 0; k < n; ++k) {
+    int A, B;
+    b2gs_pair(ns, np, k, A, B);
+    cn[k] = b2gs_pair_prims(S[A], S[B], &p64[(size_t)k * B2_MAXPP], &p32[(size_t)k * B2_MAXPP]);
+  }
+  if (precision == 64) {
+    b2hc_es_all<double>(S, ns, np, p64, cn, tab.data(), out);
+  } else {
+    std::vector<float> tf(tab.begin(), tab.end()), o(out, out + P.mols[0].n4);
+    b2hc_es_all<float>(S, ns, np, p32, cn, tf.data(), o.data());
+    for (long long e = 0; e < P.mols[0].n4; ++e) out[e] = o[e];
+  }
   return 0;
 }
 

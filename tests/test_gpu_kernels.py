@@ -324,3 +324,27 @@ def test_xc_float64_sizes(cuda, heavy):
             else:
                 assert (eng.plan.unpack(V, k) == -7.0).all() and E[k] == -7.0
     eng.close()
+
+
+@pytest.mark.parametrize("prec, tol", [(64, 1e-11), (32, 5e-6)])
+def test_eri_batch_sizes(cuda, prec, tol):
+    """batched integrals at the edges of the super-shell kernels: s shells only, one sp shell, more
+    than one chunk of 32 kets in every class, shells off the STO-3G pattern; each entry written
+    and the padding between the lists left alone"""
+    from test_hostcheck import odd_shells
+    water = Mole("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7572 -0.4692")
+    rng = np.random.default_rng(17)
+    mols = [Mole("H 0 0 0; H 0 0 0.74"), water, odd_shells(water),
+            Mole("; ".join(f"H {0.9 * (k % 3)} {0.8 * (k // 3)} 0" for k in range(9)) + "; H 0 0 1.1"),
+            odd_shells(Mole(random_molecule(rng, 4))), Mole(random_molecule(rng, 9))]
+    P = Plan(mols)
+    dt = torch.float64 if prec == 64 else torch.float32
+    out = torch.full((P.n_eri,), float("nan"), dtype=dt, device=cuda)
+    check(lib().b2_eri_s8(P.h, prec, ptr(out), stream_handle()), "b2_eri_s8")
+    v = out.double().cpu().numpy()
+    ends = list(P.eri_off[1:]) + [P.n_eri]
+    for k, m in enumerate(mols):
+        ref, o = oeri.eri_s8(m), int(P.eri_off[k])
+        np.testing.assert_allclose(v[o:o + len(ref)], ref, atol=tol, rtol=0)
+        assert np.isnan(v[o + len(ref):ends[k]]).all()
+    P.close()

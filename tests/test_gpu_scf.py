@@ -248,3 +248,28 @@ def test_drop_in_setup_routes(cuda):
     with pytest.raises(np.linalg.LinAlgError):
         eng.setup_arrays()
     eng.close()
+
+
+@pytest.mark.parametrize("atoms", [
+    ["H 0 0 0; H 0 0 0.74"],                                          # two atoms: one block of four, half empty
+    ["; ".join(f"H {0.9 * (k % 4)} {0.8 * (k // 4 % 4)} {1.1 * (k // 16)}" for k in range(n)) for n in (16, 18, 32)],
+    ["F 0 0 0; C 0 0 1.38; H 1.02 0 1.74; H -0.51 0.88 1.74; H -0.51 -0.88 1.74"],
+])
+def test_device_setup_sizes(cuda, atoms):
+    """grid, one-electron matrices and E_nuc at the kernels' edges (blocks of four atoms, the
+    16 / 17-atom split, more pairs than one chunk) against the host formulas"""
+    mols = [Mole(a) for a in atoms]
+    eng = RKSEngine(mols, level=0, precision="fp64")
+    eng.device_setup()
+    P, coords, w = eng.plan, eng.coords.cpu().numpy().reshape(-1, 3), eng.weights.cpu().numpy()
+    for k, m in enumerate(mols):
+        hs = HostSetup(m, 0)
+        g = slice(P.grid_off[k], P.grid_off[k + 1])
+        np.testing.assert_allclose(coords[g], hs.coords, atol=1e-12)
+        np.testing.assert_allclose(w[g], hs.weights, rtol=1e-10, atol=1e-14)
+        for name, ref in (("S", hs.S), ("T", hs.T), ("V", hs.V)):
+            got = P.unpack(getattr(eng, name).cpu().numpy(), k)
+            np.testing.assert_allclose(got, ref, atol=1e-11 * max(1.0, np.abs(ref).max()), err_msg=name)
+            assert (got == got.T).all()
+        assert abs(eng.enuc[k].item() - hs.E_nuc) <= 1e-12 * hs.E_nuc
+    eng.close()

@@ -332,3 +332,24 @@ def test_gradient_super_shell_form(atom, odd, counts):
     assert hc.b2hc_grad_1e(*a, _p(g, ctypes.c_double)) == 0
     assert hc.b2hc_grad_1e_super(*a, _p(gs, ctypes.c_double)) == 0
     np.testing.assert_allclose(gs, g, atol=1e-12 * max(1.0, np.abs(g).max()), rtol=0)
+
+
+@pytest.mark.parametrize("atom, odd", [
+    ("H 0 0 0; H 0 0.1 0.74", False),
+    ("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7532 -0.4792", False),
+    ("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7532 -0.4792", True),
+    ("N 0 0 0; C 0 0 1.4; H 0.9 0.2 -0.4; H -0.6 0.7 -0.3; H 0.8 0.6 1.8", True),
+])
+def test_eri_super_shell_form(atom, odd):
+    """the GPU's super-shell integrals (eri_su.cuh: every class, merged and unmerged shells, one to
+    three primitives) against the oracle: every s8 entry written, float64 to rounding plus the
+    primitive screening (1e-12), float32 to the kernels' tolerance"""
+    hc = _hc()
+    mol = Mole(atom)
+    mol = odd_shells(mol) if odd else mol
+    ref = eri.eri_s8(mol)
+    keep, a = _gs_args(mol)
+    for prec, tol in ((64, 1e-12), (32, 5e-6)):
+        v = np.full(len(ref), np.nan)
+        assert hc.b2hc_eri_super(*a, prec, _p(v, ctypes.c_double)) == 0
+        np.testing.assert_allclose(v, ref, atol=tol, rtol=0)
