@@ -15,17 +15,9 @@
 #include "device_plan.cuh"
 #include "xc_math.cuh"
 #include "xc.cuh"
+#include "xc_f64.cuh"
 
 #define B2_XD_MAXSH 48
-
-__device__ __forceinline__ int b2_findx(const long long *off, int n, long long x) {
-  int lo = 0, hi = n - 1;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= x) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
 
 template <typename T, int PT, int Q>
 __device__ __forceinline__ void b2_xd_body(const B2MolDev &md, const B2Shell *sh, T *sD, T *sA,
@@ -171,7 +163,7 @@ k_xc_direct(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shell
   __shared__ T sRt[PT][4];
   __shared__ double sC[PT * 3];
   __shared__ double red[8];
-  const int lo = b2_findx(xblk_off, nmol, blockIdx.x);
+  const int lo = b2_xf_find(xblk_off, nmol, blockIdx.x);
   const int m = mol_map ? mol_map[lo] : lo;
   if (active && !active[m]) return;
   const B2MolDev md = mols[m];
@@ -208,63 +200,42 @@ k_xc_direct(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shell
 }
 
 // ------------------------------------------------------------------ float64 form
-// Per tile of 32 points (8 warps, lane = point wherever work is per point):
-//   AO values + gradients -> sA[c][orbital][36]      (warp = shell, so no divergence in l / nprim)
-//   X = AO0^T D by m16n8k8 float64 MMA, rho_c = sum_n X AO_c reduced from the accumulators
-//   B3LYP: Slater + B88, VWN and LYP on three warps, one point per lane
-//   Y = sum_c AO_c rt_c (over plane 1), V += AO0 Y^T by MMA into registers over the CTA's tiles
-// The strides 36 and NB + 4 (4 or 12 modulo 16 doubles) keep every fragment load free of bank
-// conflicts.  Products run over the molecule's orbitals rounded up to 8, not the bucket's 16 Q.
-// What bounded the form before (CUDA-core products, one 134 KB CTA per SM whatever the molecule,
-// B3LYP serially on one lane in 16): the functional on 16 lanes of 256 and the products'
-// shared-memory loads, 1117 us per evaluation of 272 000 points x 62 orbitals against 610 us now.
-// One launch per orbital bucket sizes shared memory for that bucket (2 CTAs per SM at 64
-// orbitals, 3 at 48, 4 below).
-__device__ __forceinline__ void b2_dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
-
-#define B2_XF_LDP 36
-template <int Q> struct B2Xf {
-  static constexpr int NB = 16 * Q, LDD = NB + 4, NX = (2 * Q + 3) / 4, NV = (2 * Q * Q + 7) / 8;
-  static constexpr size_t SMEM = sizeof(double) * (NB * LDD + 4 * NB * B2_XF_LDP + 16 * 32 + 9 * 32);
-};
-
+// Per tile of 32 points (xc_f64.cuh): AO values, X = AO0^T D by float64 MMA with rho reduced from
+// the accumulators, B3LYP on three warps, Y = sum_c AO_c rt_c over plane 1, V += AO0 Y^T by MMA
+// into registers over the CTA's tiles.  One launch per orbital bucket sizes shared memory for
+// that bucket (2 CTAs per SM at 64 orbitals, 4 up to 32).
+// 272 000 points x 62 orbitals: 1117 us per evaluation with CUDA-core products in one 134 KB CTA
+// per SM and the functional on one lane in 16; 610 us with MMA products, one CTA per SM resident
+// and every l shell's own exponentials; 436 us now.
 template <int Q>
-__global__ void __launch_bounds__(256, Q <= 2 ? 4 : (Q == 3 ? 3 : (Q == 4 ? 2 : 1)))
-k_xc_f64(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
+__global__ void __launch_bounds__(256, B2_XF_CTAS(Q))
+k_xc_f64(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, const B2gSuper *__restrict__ su,
          const long long *__restrict__ xblk_off, const long long *__restrict__ grid_off, int nmol, int tpc,
          const int *__restrict__ active, const double *__restrict__ coords, const double *__restrict__ wt,
          const double *__restrict__ D, double *__restrict__ V, double *__restrict__ exc,
          const int *__restrict__ mol_map) {
   using X = B2Xf<Q>;
-  constexpr int NB = X::NB, LDD = X::LDD, LDP = B2_XF_LDP, PL = NB * LDP;
+  constexpr int NB = X::NB, LDD = X::LDD, LDP = B2_XF_LDP, PL = X::PL, NV = (2 * Q * Q + 7) / 8;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ B2Shell sh[B2_XD_MAXSH];
-  const int lo = b2_findx(xblk_off, nmol, blockIdx.x);
+  const int lo = b2_xf_find(xblk_off, nmol, blockIdx.x);
   const int m = mol_map ? mol_map[lo] : lo;
   const B2MolDev md = mols[m];
-  const int N = md.nao, nbas = md.nbas;
+  const int N = md.nao;
   if ((N + 15) / 16 != Q || (active && !active[m])) return;
-  double *sD = reinterpret_cast<double *>(smem_raw);          // [NB][LDD]
-  double *sA = sD + NB * LDD;                                  // [4][NB][LDP]
-  double *sR = sA + 4 * PL;                                    // [4 warp pairs][4][32] partial rho
-  double *sF = sR + 16 * 32;                                   // [3 parts][exc, vrho, vgamma][32]
+  const B2gsMol gm = gms[m];
+  double *sD = reinterpret_cast<double *>(smem_raw), *sA = sD + NB * LDD, *sR = sA + 4 * PL, *sF = sR + 16 * 32;
   const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   for (int e = tid; e < NB * LDD; e += 256) {
     const int a = e / LDD, b = e - (e / LDD) * LDD;
     sD[e] = (a < N && b < N) ? D[md.mat_off + a * N + b] : 0.0;
   }
   for (int e = tid; e < 4 * PL; e += 256) sA[e] = 0.0;         // rows beyond N stay zero
-  for (int s = tid; s < nbas; s += 256) sh[s] = shells[md.sh_off + s];
   const long long G = grid_off[m + 1] - grid_off[m], t0 = (blockIdx.x - xblk_off[lo]) * (long long)tpc;
   const double *cm = coords + 3 * grid_off[m], *wm = wt + grid_off[m];
-  const int n8 = (N + 7) >> 3, m16 = (n8 + 1) >> 1;
-  double vacc[X::NV][4];
+  const int n8 = (N + 7) >> 3, m16 = (n8 + 1) >> 1, per = (m16 * n8 + 7) >> 3;
+  double vacc[NV][4];
 #pragma unroll
-  for (int j = 0; j < X::NV; ++j) vacc[j][0] = vacc[j][1] = vacc[j][2] = vacc[j][3] = 0.0;
+  for (int j = 0; j < NV; ++j) vacc[j][0] = vacc[j][1] = vacc[j][2] = vacc[j][3] = 0.0;
   double e_part = 0.0;
   for (int tt = 0; tt < tpc; ++tt) {
     const long long g0 = (t0 + tt) * 32;
@@ -276,132 +247,50 @@ k_xc_f64(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
       wg = wm[g0 + lane];
     }
     __syncthreads();                                           // tables filled / previous tile consumed
-    for (int s = w; s < nbas; s += 8) {
-      const B2Shell &S = sh[s];
-      const double dx = px - S.R[0], dy = py - S.R[1], dz = pz - S.R[2], r2 = dx * dx + dy * dy + dz * dz;
-      double ga = 0, gb = 0;
-      for (int k = 0; k < S.nprim; ++k) {
-        const double ax = S.exp[k] * r2;
-        if (!pt || ax > 60.0) continue;
-        const double ev = S.coef[k] * exp(-ax);
-        ga += ev;
-        gb += -2.0 * S.exp[k] * ev;
-      }
-      double *o = sA + S.ao0 * LDP + lane;
-      if (S.l == 0) {
-        o[0] = ga;
-        o[PL] = gb * dx;
-        o[2 * PL] = gb * dy;
-        o[3 * PL] = gb * dz;
-      } else {
-        const double dd[3] = {dx, dy, dz};
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          o[c * LDP] = dd[c] * ga;
-#pragma unroll
-          for (int k = 0; k < 3; ++k) o[(1 + k) * PL + c * LDP] = (c == k ? ga : 0.0) + dd[c] * dd[k] * gb;
-        }
-      }
-    }
+    b2_xf_ao<PL>(su + gm.su_off, gm.ns + gm.np, pt, px, py, pz, sA);
     __syncthreads();
     {
-      const int r0 = 16 * (w & 1), j0 = w >> 1;
       double x[X::NX][4];
-#pragma unroll
-      for (int i = 0; i < X::NX; ++i) x[i][0] = x[i][1] = x[i][2] = x[i][3] = 0.0;
-      for (int k0 = 0; k0 < 8 * n8; k0 += 8) {
-        double a[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[i] = sA[(k0 + t + 4 * (i >> 1)) * LDP + r0 + g + 8 * (i & 1)];
-#pragma unroll
-        for (int i = 0; i < X::NX; ++i) {
-          const int j = j0 + 4 * i;
-          if (j < n8) {
-            const double b[2] = {sD[(k0 + t) * LDD + 8 * j + g], sD[(k0 + t + 4) * LDD + 8 * j + g]};
-            b2_dmma(x[i], a, b);
-          }
-        }
-      }
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        double s0 = 0, s1 = 0;
-#pragma unroll
-        for (int i = 0; i < X::NX; ++i) {
-          const int j = j0 + 4 * i;
-          if (j < n8) {
-            const double *o = sA + c * PL + (8 * j + 2 * t) * LDP + r0 + g;
-            s0 += x[i][0] * o[0] + x[i][1] * o[LDP];
-            s1 += x[i][2] * o[8] + x[i][3] * o[LDP + 8];
-          }
-        }
-        s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
-        s0 += __shfl_xor_sync(0xffffffffu, s0, 2);
-        s1 += __shfl_xor_sync(0xffffffffu, s1, 2);
-        if (t == 0) {
-          sR[(j0 * 4 + c) * 32 + r0 + g] = s0;
-          sR[(j0 * 4 + c) * 32 + r0 + g + 8] = s1;
-        }
-      }
+      b2_xf_mm<Q>(sA, sD, n8, x);
+      b2_xf_rho<Q>(sA, n8, x, sR);
     }
-    __syncthreads();
-    double rho[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-      rho[c] = (sR[c * 32 + lane] + sR[(4 + c) * 32 + lane]) + (sR[(8 + c) * 32 + lane] + sR[(12 + c) * 32 + lane]);
-    if (w < 3) {
-      const B2XcPoint<double> o = w == 0   ? b2_b3lyp_x<double>(rho[0], rho[1], rho[2], rho[3])
-                                  : w == 1 ? b2_b3lyp_vwn<double>(rho[0], rho[1], rho[2], rho[3])
-                                           : b2_b3lyp_lyp<double>(rho[0], rho[1], rho[2], rho[3]);
-      sF[(3 * w) * 32 + lane] = o.exc;
-      sF[(3 * w + 1) * 32 + lane] = o.vrho;
-      sF[(3 * w + 2) * 32 + lane] = o.vgamma;
-    }
-    __syncthreads();
+    B2XfPoint f;
+    b2_xf_func(sR, sF, f);
     {
-      const double fe = sF[lane] + sF[3 * 32 + lane] + sF[6 * 32 + lane];
-      const double fr = sF[32 + lane] + sF[4 * 32 + lane] + sF[7 * 32 + lane];
-      const double fg = sF[2 * 32 + lane] + sF[5 * 32 + lane] + sF[8 * 32 + lane];
-      if (w == 0 && pt) e_part += rho[0] * wg * fe;
-      const double f4 = 4.0 * fg * wg;                         // points beyond the grid add nothing
-      const double rt0 = pt ? fr * 0.5 * wg : 0.0, rt1 = pt ? f4 * rho[1] : 0.0, rt2 = pt ? f4 * rho[2] : 0.0,
-                   rt3 = pt ? f4 * rho[3] : 0.0;
+      if (w == 0 && pt) e_part += f.rho[0] * wg * f.exc;
+      const double f4 = 4.0 * f.vgamma * wg;                   // points beyond the grid add nothing
+      const double rt0 = pt ? f.vrho * 0.5 * wg : 0.0, rt1 = pt ? f4 * f.rho[1] : 0.0, rt2 = pt ? f4 * f.rho[2] : 0.0,
+                   rt3 = pt ? f4 * f.rho[3] : 0.0;
       for (int n = w; n < 8 * n8; n += 8) {
         double *o = sA + n * LDP + lane;
         o[PL] = o[0] * rt0 + o[PL] * rt1 + o[2 * PL] * rt2 + o[3 * PL] * rt3;
       }
     }
     __syncthreads();
-    {
-      const int per = (m16 * n8 + 7) >> 3;
 #pragma unroll
-      for (int k0 = 0; k0 < 32; k0 += 8) {
+    for (int k0 = 0; k0 < 32; k0 += 8) {
 #pragma unroll
-        for (int j = 0; j < X::NV; ++j) {
-          const int i = w * per + j;
-          if (j < per && i < m16 * n8) {
-            const int mi = i / n8, ni = i - (i / n8) * n8;
-            const double *oa = sA + (16 * mi + g) * LDP + k0 + t, *ob = sA + PL + (8 * ni + g) * LDP + k0 + t;
-            const double a[4] = {oa[0], oa[8 * LDP], oa[4], oa[8 * LDP + 4]};
-            const double b[2] = {ob[0], ob[4]};
-            b2_dmma(vacc[j], a, b);
-          }
+      for (int j = 0; j < NV; ++j) {
+        const int i = w * per + j;
+        if (j < per && i < m16 * n8) {
+          const int mi = i / n8, ni = i - (i / n8) * n8;
+          const double *oa = sA + (16 * mi + g) * LDP + k0 + t, *ob = sA + PL + (8 * ni + g) * LDP + k0 + t;
+          const double a[4] = {oa[0], oa[8 * LDP], oa[4], oa[8 * LDP + 4]};
+          const double b[2] = {ob[0], ob[4]};
+          b2_dmma(vacc[j], a, b);
         }
       }
     }
   }
-  {
-    const int per = (m16 * n8 + 7) >> 3;
 #pragma unroll
-    for (int j = 0; j < X::NV; ++j) {
-      const int i = w * per + j;
-      if (j < per && i < m16 * n8) {
-        const int mi = i / n8, ni = i - (i / n8) * n8;
+  for (int j = 0; j < NV; ++j) {
+    const int i = w * per + j;
+    if (j < per && i < m16 * n8) {
+      const int mi = i / n8, ni = i - (i / n8) * n8;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int a = 16 * mi + g + 8 * (c >> 1), b = 8 * ni + 2 * t + (c & 1);
-          if (a < N && b < N && vacc[j][c] != 0.0) atomicAdd(&V[md.mat_off + a * N + b], vacc[j][c]);
-        }
+      for (int c = 0; c < 4; ++c) {
+        const int a = 16 * mi + g + 8 * (c >> 1), b = 8 * ni + 2 * t + (c & 1);
+        if (a < N && b < N && vacc[j][c] != 0.0) atomicAdd(&V[md.mat_off + a * N + b], vacc[j][c]);
       }
     }
   }
@@ -462,7 +351,7 @@ static int b2_xf_bucket(const B2PlanDev &P, bool one, const int *active, const d
     if (!one) B2_CUDA_TRY(cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0));
     B2_CUDA_TRY(cudaFuncSetAttribute(k_xc_f64<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B2Xf<Q>::SMEM));
     k_xc_f64<Q><<<(unsigned)nblk, 256, B2Xf<Q>::SMEM, s>>>(
-        P.mols, P.shells, sub ? P.sub.x64 : P.g.xblk64, P.g.grid_off, sub ? P.sub.n : P.h.nmol, P.g.tpc64, active,
+        P.mols, P.su.mol, P.su.su, sub ? P.sub.x64 : P.g.xblk64, P.g.grid_off, sub ? P.sub.n : P.h.nmol, P.g.tpc64, active,
         coords, w, D, V, exc, sub ? P.sub.mol_map : nullptr);
     b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
