@@ -13,6 +13,7 @@
 // Jacobi ipu_eigh (nanoDFT.py:370-393).
 #include <type_traits>
 #include "device_plan.cuh"
+#include "dmma.cuh"
 #include "scf.cuh"
 
 __device__ double b2_block_sum(double v, double *red) {
@@ -39,27 +40,11 @@ __device__ double b2_block_max(double v, double *red) {
   return s;
 }
 
-// rotation (c, s) zeroing A_pq (Golub & Van Loan, sym.schur2)
-__device__ __host__ inline void b2_schur2(double app, double aqq, double apq, double &c, double &s) {
-  if (apq == 0.0) { c = 1.0; s = 0.0; return; }
-  const double tau = (aqq - app) / (2.0 * apq);
-  double t;
-  if (fabs(tau) > 1e150) t = 0.5 / tau;
-  else t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-  c = 1.0 / sqrt(1.0 + t * t);
-  s = t * c;
-}
-
 // ------------------------------------------------------------------ small dense products
 // Both SCF kernels run one molecule per CTA with 64 Q threads (2 Q warps) for the orbital bucket
 // N <= 16 Q.  acc += A B by float64 MMA (m16n8k8): warp w owns columns 8w..8w+7 and every 16-row
 // tile, so a B fragment serves Q products.  fa(r, k) and fb(k, c) return zero outside N.  The
 // inner products of the form before ran one output element per thread with two loads per FMA.
-__device__ __forceinline__ void b2_dmma(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
-               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
-}
 template <int Q, typename FA, typename FB>
 __device__ __forceinline__ void b2_mm(double (&acc)[Q][4], int N, int K, FA fa, FB fb) {
   const int w = threadIdx.x >> 5, g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
@@ -189,7 +174,9 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
 // eigenvectors.  Round-robin order: the five rotations of a round act on disjoint pairs, so lanes
 // 0..4 compute them and 25 lanes apply G_k A_kl G_l^T to the 2 x 2 blocks, nine rounds per sweep
 // (the serial order's 45 dependent rotations per sweep took 95 us per call, most of a small
-// molecule's iteration).
+// molecule's iteration; 61 us in round-robin order with the angle in float64, 48 us now).  The tangent is taken in float32, as in
+// b2_jacobi1; couplings below float32's range are far below the stopping norm (the border of B
+// holds ones).
 __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
   constexpr int n = 10;
   const int l = threadIdx.x & 31;
@@ -223,7 +210,13 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
         pair(l, p, q);
         double c = 1.0, s = 0.0;
         const double apq = A[p * n + q], app = A[p * n + p], aqq = A[q * n + q];
-        if (!(fabs(apq) <= 1e-300 || fabs(apq) < 1e-18 * sqrt(fabs(app * aqq)))) b2_schur2(app, aqq, apq, c, s);
+        if (fabs(apq) > 1e-36 && apq * apq > 1e-36 * fabs(app * aqq)) {
+          // tau = (aqq - app) / (2 apq), t = sign(tau) / (|tau| + sqrt(1 + tau^2)) (sym.schur2)
+          const float tau = fminf(fmaxf((float)(aqq - app) / (float)(2.0 * apq), -1e18f), 1e18f);
+          const double t = (double)(copysignf(1.0f, tau) / (fabsf(tau) + sqrtf(1.0f + tau * tau)));
+          c = rsqrt(1.0 + t * t);
+          s = t * c;
+        }
         rot[2 * l] = c;
         rot[2 * l + 1] = s;
       }
@@ -256,8 +249,8 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
 
 // ------------------------------------------------------------------ Fock + DIIS
 // ring layout per molecule (offset mat_off * 9): errs[9][N*N], hams[9][N*N]; B: 100 doubles
-// Bound by latency at one molecule per CTA; 62 orbitals, one molecule: 175 us per call before (two
-// products with one output element per thread, serial 10 x 10 Jacobi).
+// Bound by latency at one molecule per CTA; 62 orbitals, one molecule: 172 us per call before (two
+// products with one output element per thread, serial 10 x 10 Jacobi), 135 us now.
 template <int Q>
 __global__ void __launch_bounds__(64 * Q)
 k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
@@ -369,7 +362,9 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
   __syncthreads();
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     double s = 0;
-    for (int k = 0; k < nfill; ++k) s += sc[k + 1] * hr[(long long)k * NN + e];
+#pragma unroll
+    for (int k = 0; k < 9; ++k)                      // loads of the whole ring in flight at once
+      if (k < nfill) s += sc[k + 1] * hr[(long long)k * NN + e];
     H[mo + e] = s;
   }
 }
@@ -381,7 +376,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
 // and order of eigenvectors, which the density does not depend on.
 // Products: M = L^T W, T = H M, A = M^T T, W' = W V', C = L^T W', D = 2 C_occ C_occ^T, all by
 // float64 MMA; two matrices in shared memory (74 KB at 64 orbitals, 3 CTAs per SM).  62 orbitals,
-// one molecule: 430 us per call before.
+// one molecule: 428 us per call before, 168 us now.
 template <int Q>
 __global__ void __launch_bounds__(64 * Q)
 k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
