@@ -9,9 +9,8 @@
 //               lane (grad_sp.cuh);
 //   k_grad_1e   d/dR of <D, T + V_nuc> - <dme0, S> (h1aos and s1, nanoDFT.py:420-424): one warp
 //               per super-shell slice, lanes over nuclei;
-//   k_grad_xc   d/dR of E_xc at fixed density and grid (V_xc, nanoDFT.py:408-415): one CTA per
-//               32 grid points of one molecule, AO values, D-products and B3LYP staged in
-//               shared memory;
+//   k_grad_xc   d/dR of E_xc at fixed density and grid (V_xc, nanoDFT.py:408-415): tiles of 32
+//               points of one molecule, products with D by float64 MMA;
 //   k_grad_nuc  nuclear repulsion (grad_nuc, nanoDFT.py:428-438).
 //
 // The per-term math is grad_sp.cuh and grad_math.cuh, the same code the host-check build tests
@@ -19,12 +18,9 @@
 #include <algorithm>
 #include <vector>
 #include "device_plan.cuh"
-#include "devmem.cuh"
 #include "grad_math.cuh"
 #include "grad_sp.cuh"
-
-#define B2G_TP 32                  // grid points per XC tile (one warp's lanes)
-#define B2G_XC_THREADS 256
+#include "xc_f64.cuh"
 
 __global__ void __launch_bounds__(256)
 k_grad_dm(const B2MolDev *__restrict__ mols, const double *__restrict__ C, const double *__restrict__ eps,
@@ -122,7 +118,7 @@ __device__ __forceinline__ void b2gs_lane(const B2gsWarp &W, int nb, int k, cons
 // Boys table sits in shared memory (its rows are gathered at random: from global memory those
 // gathers took longer than the arithmetic of the small classes).
 // Bound by FP64 issue and latency (118-255 registers: 8-16 warps per SM); the whole gradient of
-// 160 uneven molecules takes 31 ms, of one molecule with 5 heavy atoms 0.26 ms.  Before (one warp
+// 160 uneven molecules takes 24 ms, of one molecule with 5 heavy atoms 0.24 ms.  Before (one warp
 // per shell quartet and l class in 16 kernels, contracted Obara-Saika [e0|f0] arrays through
 // shared memory and a horizontal recursion per quartet): 732 ms and 65 ms.
 template <int TB, int TK>
@@ -364,122 +360,144 @@ k_grad_1e(const long long *__restrict__ toff, int nmol, const B2gsMol *__restric
   }
 }
 
-// Exchange-correlation part on 32 grid points of one molecule (tile t of molecule m, tile_off:
-// per-molecule tile prefix).  With phi the AO values and u = D phi, U_k = D d_k phi:
-//   rho = phi.u, grad rho = 2 (d phi).u, and moving atom A moves its orbitals, so
-//   dE/dR_A,x = -2 sum_g w sum_{i on A} [vrho d_x phi_i u_i
-//                                        + 2 vgamma sum_k g_k (d_x d_k phi_i u_i + d_x phi_i U_k,i)].
-// Shared memory: D (N x N), phi and its gradient (4 x N x 32), u and U (4 x N x 32), the
-// points' weighted vrho / vgamma and grad rho, and the molecule's atom sums.
-__host__ __device__ inline long long b2g_xc_smem_doubles(int N, int natm) {
-  return (long long)N * N + 8ll * N * B2G_TP + 5 * B2G_TP + 3ll * natm;
-}
-
-__global__ void __launch_bounds__(B2G_XC_THREADS)
-k_grad_xc(const B2MolDev *__restrict__ mols, int nmol, const B2Shell *__restrict__ shells,
-          const long long *__restrict__ grid_off, const long long *__restrict__ tile_off,
+// Exchange-correlation part.  With phi the AO values, u = D phi and, per point, a = w vrho and
+// b = 2 w vgamma grad rho, moving atom A moves its orbitals (d phi_i / dR_A = -grad phi_i):
+//   dE/dR_A,x = -2 sum_g sum_{i on A} [d_x phi_i t_i + u_i sum_k b_k d_x d_k phi_i],
+//   t = D (a phi + sum_k b_k d_k phi).
+// So two products with D per tile (u and t; the form before made four, u and D d_k phi), by
+// float64 MMA in the phases of xc_f64.cuh; u and t replace the AO planes, and the last phase takes
+// the orbitals' derivatives from the radial sums again, one super shell per warp, its three sums
+// in registers over the CTA's tiles.  160 molecules, 1.45e6 points: 9.5 ms before (CUDA-core
+// products in 160 KB CTAs, the functional on one warp), 2.8 ms now.
+template <int Q>
+__global__ void __launch_bounds__(256, Q <= 4 ? 2 : 1)       // more registers than CTAs: the sums stay in them
+k_grad_xc(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, const B2gSuper *__restrict__ su,
+          const long long *__restrict__ xblk_off, const long long *__restrict__ grid_off, int nmol, int tpc,
           const double *__restrict__ coords, const double *__restrict__ weights, const double *__restrict__ D,
           double *__restrict__ grad) {
-  extern __shared__ double sm[];
-  const long long bt = blockIdx.x;
-  int lo = 0, hi = nmol - 1;                      // molecule: last m with tile_off[m] <= bt
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (tile_off[mid] <= bt) lo = mid; else hi = mid - 1;
-  }
-  const int m = lo;
+  using X = B2Xf<Q>;
+  constexpr int NB = X::NB, LDD = X::LDD, LDP = B2_XF_LDP, PL = X::PL;
+  constexpr int NS = 2 * Q + 1;                  // super shells per warp: at most 16 Q / 8, rounded up
+  extern __shared__ __align__(16) unsigned char gx_smem[];
+  const int m = b2_xf_find(xblk_off, nmol, blockIdx.x);
   const B2MolDev md = mols[m];
-  const int N = md.nao, nbas = md.nbas, natm = md.natm;
-  const long long p0 = grid_off[m] + (bt - tile_off[m]) * B2G_TP;
-  const int np = (int)min((long long)B2G_TP, grid_off[m + 1] - p0);
-  double *sD = sm;
-  double *phi = sD + N * N;                       // [4][N][TP]
-  double *u = phi + 4 * N * B2G_TP;               // [4][N][TP]
-  double *vr = u + 4 * N * B2G_TP, *vg = vr + B2G_TP, *gr = vg + B2G_TP;   // gr [3][TP]
-  double *sG = gr + 3 * B2G_TP;
-  const int tid = threadIdx.x, lane = tid & 31;
-  for (int e = tid; e < N * N; e += blockDim.x) sD[e] = D[md.mat_off + e];
-  for (int e = tid; e < 3 * natm; e += blockDim.x) sG[e] = 0.0;
-  // AO values and gradients; item = shell * 32 + point, so a warp shares one shell
-  for (int it = tid; it < nbas * B2G_TP; it += blockDim.x) {
-    const int s = it / B2G_TP, p = it - s * B2G_TP;
-    const B2Shell &S = shells[md.sh_off + s];
-    double f[3] = {0, 0, 0}, df[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, hf[3][6];
-    if (p < np) b2g_ao2<double>(S, coords + 3 * (p0 + p), f, df, hf);
-    for (int c = 0; c < 2 * S.l + 1; ++c) {
-      const int i = S.ao0 + c;
-      phi[i * B2G_TP + p] = f[c];
-      for (int x = 0; x < 3; ++x) phi[((1 + x) * N + i) * B2G_TP + p] = df[c][x];
-    }
+  const int N = md.nao;
+  if ((N + 15) / 16 != Q) return;
+  const B2gsMol gm = gms[m];
+  const B2gSuper *sm = su + gm.su_off;
+  const int nsu = gm.ns + gm.np;
+  double *sD = reinterpret_cast<double *>(gx_smem), *sA = sD + NB * LDD, *sR = sA + 4 * PL, *sF = sR + 16 * 32;
+  const int tid = threadIdx.x, w = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  for (int e = tid; e < NB * LDD; e += 256) {
+    const int a = e / LDD, b = e - (e / LDD) * LDD;
+    sD[e] = (a < N && b < N) ? D[md.mat_off + b * N + a] : 0.0;      // u_i = sum_j D_ij phi_j
   }
-  __syncthreads();
-  for (int it = tid; it < N * B2G_TP; it += blockDim.x) {
-    const int i = it / B2G_TP, p = it - i * B2G_TP;
-    double s0 = 0, s1 = 0, s2 = 0, s3 = 0;
-    for (int j = 0; j < N; ++j) {
-      const double dij = sD[i * N + j];
-      s0 += dij * phi[j * B2G_TP + p];
-      s1 += dij * phi[(N + j) * B2G_TP + p];
-      s2 += dij * phi[(2 * N + j) * B2G_TP + p];
-      s3 += dij * phi[(3 * N + j) * B2G_TP + p];
+  for (int e = tid; e < 4 * PL; e += 256) sA[e] = 0.0;         // rows beyond N stay zero
+  const long long G = grid_off[m + 1] - grid_off[m], t0 = (blockIdx.x - xblk_off[m]) * (long long)tpc;
+  const double *cm = coords + 3 * grid_off[m], *wm = weights + grid_off[m];
+  const int n8 = (N + 7) >> 3, r0 = 16 * (w & 1), j0 = w >> 1;
+  double acc[NS][3];
+#pragma unroll
+  for (int k = 0; k < NS; ++k) acc[k][0] = acc[k][1] = acc[k][2] = 0.0;
+  // a product's accumulators to a plane
+  auto put = [&](const double (&x)[X::NX][4], double *P) {
+#pragma unroll
+    for (int i = 0; i < X::NX; ++i) {
+      const int j = j0 + 4 * i;
+      if (j < n8) {
+        double *o = P + (8 * j + 2 * t) * LDP + r0 + g;
+        o[0] = x[i][0];
+        o[LDP] = x[i][1];
+        o[8] = x[i][2];
+        o[LDP + 8] = x[i][3];
+      }
     }
-    u[i * B2G_TP + p] = s0;
-    u[(N + i) * B2G_TP + p] = s1;
-    u[(2 * N + i) * B2G_TP + p] = s2;
-    u[(3 * N + i) * B2G_TP + p] = s3;
-  }
-  __syncthreads();
-  if (tid < B2G_TP) {
-    const int p = tid;
-    double rho = 0, r1[3] = {0, 0, 0};
-    for (int i = 0; i < N; ++i) {
-      const double ui = u[i * B2G_TP + p];
-      rho += phi[i * B2G_TP + p] * ui;
-      for (int x = 0; x < 3; ++x) r1[x] += phi[((1 + x) * N + i) * B2G_TP + p] * ui;
+  };
+  for (int tt = 0; tt < tpc; ++tt) {
+    const long long g0 = (t0 + tt) * 32;
+    if (g0 >= G) break;
+    const bool pt = g0 + lane < G;
+    double px = 0, py = 0, pz = 0, wg = 0;
+    if (pt) {
+      px = cm[3 * (g0 + lane)]; py = cm[3 * (g0 + lane) + 1]; pz = cm[3 * (g0 + lane) + 2];
+      wg = wm[g0 + lane];
     }
-    double a = 0, b = 0;
-    if (p < np) {
-      const B2XcPoint<double> o = b2_b3lyp_point<double>(rho, r1[0], r1[1], r1[2]);
-      const double wt = weights[p0 + p];
-      a = wt * o.vrho;
-      b = wt * o.vgamma;
+    __syncthreads();                                           // tables filled / previous tile consumed
+    b2_xf_ao<PL>(sm, nsu, pt, px, py, pz, sA);
+    __syncthreads();
+    double x[X::NX][4];
+    b2_xf_mm<Q>(sA, sD, n8, x);
+    b2_xf_rho<Q>(sA, n8, x, sR);
+    B2XfPoint f;
+    b2_xf_func(sR, sF, f);
+    // points beyond the grid add nothing; grad rho = 2 rho[1..3]
+    const double a = pt ? wg * f.vrho : 0.0;
+    const double b[3] = {pt ? 4.0 * wg * f.vgamma * f.rho[1] : 0.0, pt ? 4.0 * wg * f.vgamma * f.rho[2] : 0.0,
+                         pt ? 4.0 * wg * f.vgamma * f.rho[3] : 0.0};
+    for (int n = w; n < 8 * n8; n += 8) {
+      double *o = sA + n * LDP + lane;
+      o[PL] = a * o[0] + b[0] * o[PL] + b[1] * o[2 * PL] + b[2] * o[3 * PL];
     }
-    vr[p] = a;
-    vg[p] = b;
-    for (int x = 0; x < 3; ++x) gr[x * B2G_TP + p] = 2.0 * r1[x];
-  }
-  __syncthreads();
-  const int hidx[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
-  for (int it = tid; it < nbas * B2G_TP; it += blockDim.x) {    // warp-uniform shell
-    const int s = it / B2G_TP, p = it - s * B2G_TP;
-    const B2Shell &S = shells[md.sh_off + s];
-    double acc[3] = {0, 0, 0};
-    if (p < np) {
-      double f[3], df[3][3], hf[3][6];
-      b2g_ao2<double>(S, coords + 3 * (p0 + p), f, df, hf);
-      const double a = vr[p], b2 = 2.0 * vg[p];
-      const double g0 = gr[p], g1 = gr[B2G_TP + p], g2 = gr[2 * B2G_TP + p];
-      for (int c = 0; c < 2 * S.l + 1; ++c) {
-        const int i = S.ao0 + c;
-        const double u0 = u[i * B2G_TP + p];
-        const double uk[3] = {u[(N + i) * B2G_TP + p], u[(2 * N + i) * B2G_TP + p], u[(3 * N + i) * B2G_TP + p]};
-        const double gk[3] = {g0, g1, g2};
-        for (int x = 0; x < 3; ++x) {
-          double q = 0;
-          for (int k = 0; k < 3; ++k) q += gk[k] * (hf[c][hidx[x][k]] * u0 + df[c][x] * uk[k]);
-          acc[x] += a * df[c][x] * u0 + b2 * q;
+    __syncthreads();                                           // planes 2 and 3 are free now
+    put(x, sA + 2 * PL);
+    b2_xf_mm<Q>(sA + PL, sD, n8, x);
+    put(x, sA + 3 * PL);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NS; ++k) {
+      const int s = w + 8 * k;
+      if (s < nsu) {
+        const B2gSuper &S = sm[s];
+        const double d[3] = {px - S.R[0], py - S.R[1], pz - S.R[2]}, r2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+        double s1 = 0, s2 = 0, p0 = 0, p1 = 0, p2 = 0;         // sums of c e, -2 a c e, 4 a^2 c e
+        for (int q = 0; q < S.nprim; ++q) {
+          const double al = S.ex[q], ax = al * r2;
+          if (!pt || ax > 60.0) continue;
+          const double ev = exp(-ax), es = S.cs[q] * ev, ep = S.cp[q] * ev;
+          s1 -= 2.0 * al * es;
+          s2 += 4.0 * al * al * es;
+          p0 += ep;
+          p1 -= 2.0 * al * ep;
+          p2 += 4.0 * al * al * ep;
+        }
+        const double bd = b[0] * d[0] + b[1] * d[1] + b[2] * d[2];
+        if (S.ao_s >= 0) {
+          const double *o = sA + S.ao_s * LDP + lane;
+          const double ui = o[2 * PL], ti = o[3 * PL], c = s1 * ti + s2 * bd * ui;
+#pragma unroll
+          for (int y = 0; y < 3; ++y) acc[k][y] += c * d[y] + s1 * ui * b[y];
+        }
+        if (S.ao_p >= 0) {
+          const double *o = sA + S.ao_p * LDP + lane;
+          double ui[3], ti[3], T = 0, U = 0, bU = 0;
+#pragma unroll
+          for (int y = 0; y < 3; ++y) {
+            ui[y] = o[2 * PL + y * LDP];
+            ti[y] = o[3 * PL + y * LDP];
+            T += d[y] * ti[y];
+            U += d[y] * ui[y];
+            bU += b[y] * ui[y];
+          }
+          const double c = p1 * (T + bU) + p2 * bd * U;
+#pragma unroll
+          for (int y = 0; y < 3; ++y) acc[k][y] += p0 * ti[y] + p1 * bd * ui[y] + p1 * U * b[y] + c * d[y];
         }
       }
     }
-    for (int x = 0; x < 3; ++x) {
-      double v = acc[x];
+  }
 #pragma unroll
-      for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      if (lane == 0) atomicAdd(&sG[3 * S.atom + x], -2.0 * v);
+  for (int k = 0; k < NS; ++k) {
+    const int s = w + 8 * k;
+    if (s < nsu) {
+#pragma unroll
+      for (int y = 0; y < 3; ++y) {
+        double v = acc[k][y];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) atomicAdd(grad + 3ll * (md.atm_off + sm[s].atom) + y, -2.0 * v);
+      }
     }
   }
-  __syncthreads();
-  for (int e = tid; e < 3 * natm; e += blockDim.x) atomicAdd(grad + 3ll * md.atm_off + e, sG[e]);
 }
 
 // nuclear repulsion: g_a = -sum_{b != a} Z_a Z_b (R_a - R_b) / |R_a - R_b|^3 (coincident atoms
@@ -557,6 +575,26 @@ static int b2gs_launch(const B2PlanDev &P, int parts, double hyb, const double *
   return rc;
 }
 
+// one launch per orbital bucket that holds molecules, on the bucket streams; CTAs of other buckets'
+// molecules return at once
+template <int Q>
+static int b2g_launch_xc(const B2PlanDev &P, const double *coords, const double *weights, const double *D, double *grad,
+                         cudaStream_t st) {
+  if (P.bkt_off_h[Q] > P.bkt_off_h[Q - 1]) {
+    const cudaStream_t s = P.bkt_stream[Q - 1];
+    B2_CUDA_TRY(cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0));
+    B2_CUDA_TRY(cudaFuncSetAttribute(k_grad_xc<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B2Xf<Q>::SMEM));
+    k_grad_xc<Q><<<(unsigned)P.g.n_xblk64, 256, B2Xf<Q>::SMEM, s>>>(P.mols, P.su.mol, P.su.su, P.g.xblk64, P.g.grid_off,
+                                                                    P.h.nmol, P.g.tpc64, coords, weights, D, grad);
+    b2_count_launches(1);
+    B2_CUDA_TRY(cudaGetLastError());
+    B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[Q - 1], s));
+    B2_CUDA_TRY(cudaStreamWaitEvent(st, P.bkt_ev[Q - 1], 0));
+  }
+  if constexpr (Q > 1) return b2g_launch_xc<Q - 1>(P, coords, weights, D, grad, st);
+  return B2_OK;
+}
+
 int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const double *mo_energy,
                    const double *coords, const double *weights, double *D, double *W, double *grad,
                    cudaStream_t st) {
@@ -574,30 +612,11 @@ int b2_launch_grad(B2PlanDev &P, int parts, double hyb, const double *C, const d
     const int rc = b2gs_launch(P, parts, hyb, D, W, grad, st);
     if (rc) return rc;
   }
-  if (parts & 4) {
-    std::vector<long long> toff(nmol + 1, 0);
-    for (int m = 0; m < nmol; ++m) {
-      const long long G = P.g.grid_off_h[m + 1] - P.g.grid_off_h[m];
-      toff[m + 1] = toff[m] + (G + B2G_TP - 1) / B2G_TP;
-    }
-    if (toff[nmol] > 0) {
-      if (toff[nmol] >= (1ll << 31)) return B2_ERR_SIZE;
-      const size_t smem = sizeof(double) * (size_t)b2g_xc_smem_doubles(P.h.max_nao, P.h.max_natm);
-      B2_CUDA_TRY(cudaFuncSetAttribute(k_grad_xc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      long long *dtoff = nullptr;
-      B2_CUDA_TRY(b2_dmalloc_t(&dtoff, sizeof(long long) * (nmol + 1), st));
-      // pageable source: the call returns once the data is staged, so toff may go out of scope
-      cudaError_t e = cudaMemcpyAsync(dtoff, toff.data(), sizeof(long long) * (nmol + 1),
-                                      cudaMemcpyHostToDevice, st);
-      if (e == cudaSuccess) {
-        k_grad_xc<<<(unsigned)toff[nmol], B2G_XC_THREADS, smem, st>>>(P.mols, nmol, P.shells, P.g.grid_off,
-                                                                       dtoff, coords, weights, D, grad);
-        b2_count_launches(1);
-        e = cudaGetLastError();
-      }
-      b2_dfree(dtoff, st);
-      if (e != cudaSuccess) return B2_ERR_CUDA;
-    }
+  if ((parts & 4) && P.g.n_xblk64 > 0) {
+    if (P.g.n_xblk64 >= (1ll << 31)) return B2_ERR_SIZE;
+    B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
+    const int rc = b2g_launch_xc<B2_NBKT>(P, coords, weights, D, grad, st);
+    if (rc) return rc;
   }
   if (parts & 8) {
     k_grad_nuc<<<nmol, 128, 0, st>>>(P.mols, P.atom_xyz, P.atom_z, grad);
