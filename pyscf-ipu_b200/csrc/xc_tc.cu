@@ -573,10 +573,10 @@ int b2_launch_xc_tc(const B2PlanDev &P, const int *active, const double *coords,
 //   * persistent CTAs pull work items (molecule, block of tiles) from a device queue (one
 //     atomic counter per bucket, cleared before the launch) until it is empty; an item of an
 //     inactive molecule is skipped;
-//   * the radial factors ga = sum c e^{-a r^2} and gb = sum -2 a c e^{-a r^2} are evaluated once per
-//     shell and tile (consecutive shells with the same centre and exponents, the 2s/2p pair of
-//     STO-3G, share the exponentials); AO values go to the N and T tiles, AO gradients to tensor
-//     memory (three columns per orbital) for the rho and Y phases;
+//   * the tiles' columns are grouped by super shell (b2_xq_columns): the radial factors
+//     ga = sum c e^{-a r^2} and gb = sum -2 a c e^{-a r^2} share their exponentials between the s and
+//     p functions of a shell; AO values go to the N and T tiles, AO gradients to tensor memory
+//     (three columns per orbital) for the rho and Y phases;
 //   * the next tile's grid point is loaded one tile ahead;
 //   * the AO0^T tile holds NB rows: the M = 64 product's rows >= NB read whatever follows
 //     (the next point chunk, or a pad), which only reaches accumulator rows >= NB, never read;
@@ -597,9 +597,65 @@ template <int Q> __host__ __device__ constexpr uint32_t b2_xq_tmem_cols() {
          : (16 * Q > 64 ? 6 : 5) * 16 * Q <= 256 ? 256 : 512;
 }
 
+// Columns of a molecule's NB-column tiles: groups of four, a merged sp shell (s, px, py, pz) or four
+// functions of their own (s shells; p functions without an s partner), so a group's arithmetic is
+// straight-line code with one set of exponentials per shell.  The groups are dealt out to the four
+// thread quarters in turn (functions of their own first: they cost twice an sp group), Q slots
+// each; 4 ceil(N / 4) <= NB columns are used.  Before, columns were the AOs in order with a table
+// look-up, type selects and a float64 displacement per orbital: 6.87 -> 5.72 ms per evaluation of
+// 2048 uneven molecules (the kernel is issue-bound, and these phases were 38% of its instructions).
+template <int Q>
+__device__ void b2_xq_columns(const B2gsMol &g, const B2gSuper *__restrict__ su, float (*sGrp)[64], int *sTy, int *sMap) {
+  constexpr int NB = 16 * Q;
+  const B2gSuper *S = su + g.su_off;
+  for (int c = threadIdx.x; c < NB; c += blockDim.x) {
+    const int slot = c >> 2, u = c & 3;
+    const int k = (slot - (slot / Q) * Q) * 4 + slot / Q;       // order in which slots are dealt out
+    int lone = 0;                                               // p shells without an s partner
+    for (int j = 0; j < g.np; ++j) lone += S[g.ns + j].ao_s < 0;
+    const int n1 = g.ns + 3 * lone, a = (n1 + 3) >> 2;
+    int s = -1, comp = -1;
+    const bool sp = k >= a;
+    if (sp) {
+      int want = k - a;
+      for (int j = 0; j < g.np && s < 0; ++j)
+        if (S[g.ns + j].ao_s >= 0 && want-- == 0) s = g.ns + j;
+    } else if (4 * k + u < g.ns) {
+      s = 4 * k + u;
+    } else if (4 * k + u < n1) {
+      const int i = 4 * k + u - g.ns;
+      int want = i / 3;
+      comp = i - 3 * (i / 3);
+      for (int j = 0; j < g.np && s < 0; ++j)
+        if (S[g.ns + j].ao_s < 0 && want-- == 0) s = g.ns + j;
+    }
+    const bool group = sp && s >= 0;
+    sMap[c] = s < 0 ? -1 : (group ? (u == 0 ? S[s].ao_s : S[s].ao_p + u - 1) : (comp < 0 ? S[s].ao_s : S[s].ao_p + comp));
+    if (u == 0) sTy[slot] = group;
+    if (group && u > 0) continue;
+    float *o = sGrp[slot] + (group ? 0 : 16 * u);
+    for (int q = 0; q < 3; ++q) {
+      const bool has = s >= 0 && q < S[s].nprim;
+      const double al = has ? S[s].ex[q] : 0.0, R = s >= 0 ? S[s].R[q] : 0.0;
+      const double c1 = has ? (comp < 0 ? S[s].cs[q] : S[s].cp[q]) : 0.0;
+      o[q] = (float)R;
+      o[4 + q] = (float)(R - (double)o[q]);
+      o[8 + q] = (float)c1;
+      o[12 + q] = (float)(-2.0 * al * c1);
+      o[q == 0 ? 3 : (q == 1 ? 7 : 11)] = (float)(al * 1.4426950408889634);
+      if (group) {
+        o[16 + q] = (float)S[s].cp[q];
+        o[20 + q] = (float)(-2.0 * al * S[s].cp[q]);
+        if (!has) o[16 + q] = 0.f;
+      }
+    }
+    o[15] = (float)comp;
+  }
+}
+
 template <int Q>
 __global__ void __launch_bounds__(B2_XT_NT, Q <= 2 ? 2 : 1)
-k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
+k_xc_tq(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, const B2gSuper *__restrict__ su,
         const B2XtItem *__restrict__ items, int n_items, int *__restrict__ queue,
         const long long *__restrict__ grid_off, int tpc, const int *__restrict__ active,
         const double *__restrict__ coords, const double *__restrict__ w, const double *__restrict__ D,
@@ -609,8 +665,8 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
   constexpr uint32_t NCOL = b2_xq_tmem_cols<Q>();
   constexpr uint32_t colX = 0, colA = NB, colV = 4 * NB, colV2 = 5 * NB;
   extern __shared__ __align__(128) float smem_f[];
-  __shared__ B2XtOrb sOrb[NB];
-  __shared__ double sR[B2_XT_MAXSH][3];
+  __shared__ __align__(16) float sGrp[NB / 4][64];   // basis functions of each group of four columns
+  __shared__ int sTy[NB / 4], sMap[NB];              // group type (1: sp shell), AO of each column (-1: none)
   __shared__ float sRed[16 * B2_XT_PT];
   // NB = 80 leaves no room for a separate B3LYP exchange buffer: it reuses sRed (one more barrier)
   constexpr bool kAlias = Q >= 5;
@@ -666,36 +722,13 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
     const double *cm = coords + 3 * grid_off[m];
     const double *wm = w + grid_off[m];
     // the previous item's V product may still read the T / Y^T tiles, and its V flush already
-    // waited for it; here: orbital table, shell centres, D split into TF32 pieces
-    for (int s = tid; s < md.nbas; s += B2_XT_NT) {
-      const B2Shell &S = shells[md.sh_off + s];
-      sR[s][0] = S.R[0];
-      sR[s][1] = S.R[1];
-      sR[s][2] = S.R[2];
-      const int nc = S.l == 0 ? 1 : 3;
-      bool same = false;                            // same centre and exponents as shell s-1
-      if (s > 0) {
-        const B2Shell &P0 = shells[md.sh_off + s - 1];
-        same = P0.atom == S.atom && P0.nprim == S.nprim;
-        for (int k = 0; k < S.nprim && same; ++k) same = P0.exp[k] == S.exp[k];
-      }
-      for (int c = 0; c < nc; ++c) {
-        B2XtOrb o;
-        for (int k = 0; k < 3; ++k) {
-          const bool has = k < S.nprim;
-          o.e2[k] = has ? (float)(S.exp[k] * 1.4426950408889634) : 0.f;
-          o.c[k] = has ? (float)S.coef[k] : 0.f;
-          o.m2a[k] = has ? (float)(-2.0 * S.exp[k]) : 0.f;
-        }
-        o.s = (float)s;
-        o.comp = S.l == 0 ? -1.f : (float)c;
-        o.pad = same ? 1.f : 0.f;
-        sOrb[S.ao0 + c] = o;
-      }
-    }
+    // waited for it; here: column table, D split into TF32 pieces
+    b2_xq_columns<Q>(gms[m], su, sGrp, sTy, sMap);
+    __syncthreads();
     for (int e = tid; e < NB * NB; e += B2_XT_NT) {
       const int r = e / NB, k = e - r * NB;
-      const float v = (r < N && k < N) ? (float)D[md.mat_off + (long long)r * N + k] : 0.f;
+      const int ra = sMap[r], rk = sMap[k];
+      const float v = (ra >= 0 && rk >= 0) ? (float)D[md.mat_off + (long long)ra * N + rk] : 0.f;
       float d1, d2, t;
       b2_split_rn(v, d1, t);
       d2 = __uint_as_float((__float_as_uint(t) + 0x1000u) & 0xFFFFE000u);
@@ -703,8 +736,6 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
       sDh[idx] = d1;
       sDl[idx] = d2;
     }
-    // the orbital table and shell centres are read by every thread from the first tile on
-    __syncthreads();
     double e_part = 0.0;
     bool first = true;
     // point of this thread in the next tile, loaded one tile ahead (the loads' latency overlaps
@@ -717,8 +748,7 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
     for (int tt = 0; tt < tpc; ++tt) {
       const long long g0 = ((long long)item.t0 + tt) * B2_XT_PT;
       if (g0 >= G) break;
-      const int np = (int)min((long long)B2_XT_PT, G - g0);
-      const bool valid = p < np;
+      const bool valid = g0 + p < G;
       const double px = qx, py = qy, pz = qz, wd = qw;     // zero for points past the grid
       {
         const long long g1 = g0 + B2_XT_PT + p;
@@ -726,56 +756,55 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
         if (tt + 1 < tpc && g1 < G) { qx = cm[3 * g1]; qy = cm[3 * g1 + 1]; qz = cm[3 * g1 + 2]; qw = wm[g1]; }
       }
       const float wp = (float)wd;
-      // ---- AO values (registers) and AO gradients (tensor memory) of this thread's orbitals
+      // ---- AO values (registers) and AO gradients (tensor memory) of this thread's orbitals.
+      // Coordinates as float pairs: (hi - hi) + (lo - lo) keeps the displacement to float32
+      // rounding without float64 arithmetic per shell.  Points past the grid (w = 0) are evaluated
+      // like the others: their weights zero what follows.
       float a0[4 * Q];
       {
-        int s_prev = -1;
-        float ev0 = 0, ev1 = 0, ev2 = 0, dx = 0, dy = 0, dz = 0, ga = 0, gb = 0;
+        const float ph[3] = {(float)px, (float)py, (float)pz};
+        const float pl[3] = {(float)(px - (double)ph[0]), (float)(py - (double)ph[1]), (float)(pz - (double)ph[2])};
 #pragma unroll
         for (int j4 = 0; j4 < Q; ++j4) {
+          const float4 *rec = reinterpret_cast<const float4 *>(sGrp[qq * Q + j4]);
           float a1[4], a2[4], a3[4];
+          if (sTy[qq * Q + j4]) {                      // s and p of one shell: shared exponentials
+            const float4 h = rec[0], l = rec[1], cs = rec[2], ms = rec[3], cp = rec[4], mp = rec[5];
+            const float dx = (ph[0] - h.x) + (pl[0] - l.x), dy = (ph[1] - h.y) + (pl[1] - l.y),
+                        dz = (ph[2] - h.z) + (pl[2] - l.z);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            const float ev0 = b2_ex2(-h.w * r2), ev1 = b2_ex2(-l.w * r2), ev2 = b2_ex2(-cs.w * r2);
+            const float gb = ms.x * ev0 + ms.y * ev1 + ms.z * ev2;
+            const float pa = cp.x * ev0 + cp.y * ev1 + cp.z * ev2, pb = mp.x * ev0 + mp.y * ev1 + mp.z * ev2;
+            const float tx = dx * pb, ty = dy * pb, tz = dz * pb;
+            a0[4 * j4] = cs.x * ev0 + cs.y * ev1 + cs.z * ev2;
+            a0[4 * j4 + 1] = dx * pa;
+            a0[4 * j4 + 2] = dy * pa;
+            a0[4 * j4 + 3] = dz * pa;
+            a1[0] = gb * dx; a1[1] = pa + tx * dx; a1[2] = ty * dx; a1[3] = tz * dx;
+            a2[0] = gb * dy; a2[1] = tx * dy; a2[2] = pa + ty * dy; a2[3] = tz * dy;
+            a3[0] = gb * dz; a3[1] = tx * dz; a3[2] = ty * dz; a3[3] = pa + tz * dz;
+          } else {                                     // four functions of their own
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int n = nq0 + 4 * j4 + u;
-            float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
-            if (n < N && valid) {
-              const float4 o0 = reinterpret_cast<const float4 *>(sOrb)[3 * n];
-              const float4 o1 = reinterpret_cast<const float4 *>(sOrb)[3 * n + 1];
-              const int sh = min(max((int)o0.w, 0), B2_XT_MAXSH - 1);   // table index (clamped)
-              if (sh != s_prev) {        // same for every lane of the warp
-                const float4 o2 = reinterpret_cast<const float4 *>(sOrb)[3 * n + 2];
-                if (!(o2.w != 0.f && sh == s_prev + 1 && s_prev >= 0)) {
-                  dx = (float)(px - sR[sh][0]);
-                  dy = (float)(py - sR[sh][1]);
-                  dz = (float)(pz - sR[sh][2]);
-                  const float r2 = dx * dx + dy * dy + dz * dz;
-                  ev0 = b2_ex2(-o0.x * r2);
-                  ev1 = b2_ex2(-o0.y * r2);
-                  ev2 = b2_ex2(-o0.z * r2);
-                }
-                s_prev = sh;
-                ga = o1.x * ev0 + o1.y * ev1 + o1.z * ev2;
-                gb = o2.x * o1.x * ev0 + o2.y * o1.y * ev1 + o2.z * o1.z * ev2;
-              }
-              const float comp = o1.w;
-              if (comp < 0.f) {          // s:   AO = ga, grad AO = gb d
-                v0 = ga;
-                v1 = gb * dx;
-                v2 = gb * dy;
-                v3 = gb * dz;
-              } else {                   // p_k: AO = d_k ga, grad AO = ga e_k + d_k gb d
-                const float dk = comp == 0.f ? dx : (comp == 1.f ? dy : dz);
-                const float t = dk * gb;
-                v0 = dk * ga;
-                v1 = (comp == 0.f ? ga : 0.f) + t * dx;
-                v2 = (comp == 1.f ? ga : 0.f) + t * dy;
-                v3 = (comp == 2.f ? ga : 0.f) + t * dz;
+            for (int u = 0; u < 4; ++u) {
+              const float4 h = rec[4 * u], l = rec[4 * u + 1], c = rec[4 * u + 2], m2 = rec[4 * u + 3];
+              const float dx = (ph[0] - h.x) + (pl[0] - l.x), dy = (ph[1] - h.y) + (pl[1] - l.y),
+                          dz = (ph[2] - h.z) + (pl[2] - l.z);
+              const float r2 = dx * dx + dy * dy + dz * dz;
+              const float ev0 = b2_ex2(-h.w * r2), ev1 = b2_ex2(-l.w * r2), ev2 = b2_ex2(-c.w * r2);
+              const float ga = c.x * ev0 + c.y * ev1 + c.z * ev2, gb = m2.x * ev0 + m2.y * ev1 + m2.z * ev2;
+              a0[4 * j4 + u] = ga;
+              a1[u] = gb * dx;
+              a2[u] = gb * dy;
+              a3[u] = gb * dz;
+              if (m2.w >= 0.f) {                       // a p function without an s partner
+                const float dk = m2.w == 0.f ? dx : (m2.w == 1.f ? dy : dz);
+                a0[4 * j4 + u] = dk * ga;
+                a1[u] = a1[u] * dk + (m2.w == 0.f ? ga : 0.f);
+                a2[u] = a2[u] * dk + (m2.w == 1.f ? ga : 0.f);
+                a3[u] = a3[u] * dk + (m2.w == 2.f ? ga : 0.f);
               }
             }
-            a0[4 * j4 + u] = v0;
-            a1[u] = v1;
-            a2[u] = v2;
-            a3[u] = v3;
           }
           b2_tmem_st4(tl + colA + nq0 + 4 * j4, a1[0], a1[1], a1[2], a1[3]);
           b2_tmem_st4(tl + colA + NB + nq0 + 4 * j4, a2[0], a2[1], a2[2], a2[3]);
@@ -878,8 +907,9 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
       }
       b2_bar_quarter(q4);                                           // [3]
       const float ex = sFn[0 * B2_XT_PT + p] + (sFn[3 * B2_XT_PT + p] + sFn[6 * B2_XT_PT + p]);
-      const float vrho = sFn[1 * B2_XT_PT + p] + (sFn[4 * B2_XT_PT + p] + sFn[7 * B2_XT_PT + p]);
-      const float vg = sFn[2 * B2_XT_PT + p] + (sFn[5 * B2_XT_PT + p] + sFn[8 * B2_XT_PT + p]);
+      float vrho = sFn[1 * B2_XT_PT + p] + (sFn[4 * B2_XT_PT + p] + sFn[7 * B2_XT_PT + p]);
+      float vg = sFn[2 * B2_XT_PT + p] + (sFn[5 * B2_XT_PT + p] + sFn[8 * B2_XT_PT + p]);
+      if (!valid) vrho = vg = 0.f;
       if (qq == 0 && valid) e_part += (double)rho[0] * wd * (double)ex;
       const float rt0 = vrho * 0.5f * wp, f4 = 4.f * vg * wp;
       const float rt1 = f4 * rho[1], rt2 = f4 * rho[2], rt3 = f4 * rho[3];
@@ -949,22 +979,24 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
         uint32_t v[4];
         b2_tmem_ld4(tl + colV + n0, v);
         b2_tmem_wait_ld();
-        if (lane < 16 && mu < N) {
+        if (lane < 16 && mu < NB && sMap[mu] >= 0) {
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const float f = __uint_as_float(v[u]);
-            if (n0 + u < N && f != 0.f) atomicAdd(&V[md.mat_off + (long long)mu * N + n0 + u], (double)f);
+            const int c = sMap[n0 + u];
+            if (c >= 0 && f != 0.f) atomicAdd(&V[md.mat_off + (long long)sMap[mu] * N + c], (double)f);
           }
         }
         if (NB > 64) {
           b2_tmem_ld4(tl + colV2 + n0, v);
           b2_tmem_wait_ld();
           const int mu2 = NB - 64 + mu;
-          if (lane < 16 && mu2 >= 64 && mu2 < N) {
+          if (lane < 16 && mu2 >= 64 && sMap[mu2] >= 0) {
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
               const float f = __uint_as_float(v[u]);
-              if (n0 + u < N && f != 0.f) atomicAdd(&V[md.mat_off + (long long)mu2 * N + n0 + u], (double)f);
+              const int c = sMap[n0 + u];
+              if (c >= 0 && f != 0.f) atomicAdd(&V[md.mat_off + (long long)sMap[mu2] * N + c], (double)f);
             }
           }
         }
@@ -1008,7 +1040,7 @@ static int b2_xq_launch(const B2PlanDev &P, const B2XtItem *items, int n_items, 
   }
   const int grid = std::min(n_items, occ[dev]);
   const int tpc = P.g.xq_tpc[Q - 1] > 0 ? P.g.xq_tpc[Q - 1] : std::max(1, P.g.tpc_tc);
-  k_xc_tq<Q><<<grid, B2_XT_NT, sm, st>>>(P.mols, P.shells, items, n_items, queue, P.g.grid_off,
+  k_xc_tq<Q><<<grid, B2_XT_NT, sm, st>>>(P.mols, P.su.mol, P.su.su, items, n_items, queue, P.g.grid_off,
                                           tpc, active, coords, w, D, V, exc);
   return B2_OK;
 }
