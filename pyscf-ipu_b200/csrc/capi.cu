@@ -108,7 +108,7 @@ static void b2_plan_free(B2PlanDev *P) {
   if (P->jk_stream) cudaStreamSynchronize(P->jk_stream);
   b2_subset_free(P);
   b2_grid_free(*P);
-  b2_dfree(P->mols); b2_dfree(P->row_off); b2_dfree(P->shells); b2_dfree(P->pinfo);
+  b2_dfree(P->mols); b2_dfree(P->row_off); b2_dfree(P->shells);
   b2_dfree(P->su.su); b2_dfree(P->su.mol); b2_dfree(P->su.off);
   b2_dfree(P->su.pr64); b2_dfree(P->su.pr32); b2_dfree(P->su.pn); b2_dfree(P->ao2sh);
   b2_dfree(P->atom_xyz); b2_dfree(P->atom_z); b2_dfree(P->boys); b2_dfree(P->boys32);

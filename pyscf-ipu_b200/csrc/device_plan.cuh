@@ -57,7 +57,7 @@ struct B2PlanDev {
   B2MolDev *mols = nullptr;
   long long *row_off = nullptr;
   B2Shell *shells = nullptr;
-  B2PairInfo *pinfo = nullptr;
+  B2PairInfo *pinfo = nullptr;            // shell pairs (allocation-free entry only)
   B2SuDev su;
   int *ao2sh = nullptr;
   int *cls_list = nullptr;                // shell-pair class lists (allocation-free entry only)

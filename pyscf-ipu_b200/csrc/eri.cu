@@ -557,32 +557,16 @@ extern "C" int b2_int2e_sph_s8_noalloc(const int *atm, int natm, const int *bas,
   return B2_OK;
 }
 
-// shell pairs (I >= J) of every molecule, one warp per molecule (the one-electron kernel's order)
-__global__ void __launch_bounds__(256)
-k_plan_pairs(const B2MolDev *__restrict__ mols, int nmol, const B2Shell *__restrict__ shells,
-             B2PairInfo *__restrict__ pinfo) {
-  const int m = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (m >= nmol) return;                           // whole warp
-  const B2MolDev md = mols[m];
-  const B2Shell *S = shells + md.sh_off;
-  for (int sp = threadIdx.x & 31; sp < md.nsp; sp += 32) {
-    const int I = (int)b2_untri(sp), J = sp - (int)b2_tri(I);
-    pinfo[md.sp_off + sp] = B2PairInfo{I, J, S[I].l, S[J].l, S[I].ao0, S[J].ao0, S[I].nprim * S[J].nprim, 0};
-  }
-}
-
-// device tables of a plan that kernels build: shell pairs and the super-shell pairs' primitives
+// device tables of a plan that kernels build: the super-shell pairs' primitives
 int b2_build_pairs(B2PlanDev &P, cudaStream_t st) {
-  const long long nsp = P.h.n_sp, np = P.su.n_pair;
-  B2_CUDA_TRY(b2_dmalloc_t(&P.pinfo, sizeof(B2PairInfo) * (size_t)std::max(1ll, nsp), st));
+  const long long np = P.su.n_pair;
   B2_CUDA_TRY(b2_dmalloc_t(&P.su.pr64, sizeof(B2gPrim) * B2_MAXPP * (size_t)std::max(1ll, np), st));
   B2_CUDA_TRY(b2_dmalloc_t(&P.su.pr32, sizeof(B2gPrim32) * B2_MAXPP * (size_t)std::max(1ll, np), st));
   B2_CUDA_TRY(b2_dmalloc_t(&P.su.pn, sizeof(B2gCount) * (size_t)std::max(1ll, np), st));
-  if (nsp > 0 && np > 0) {
-    k_plan_pairs<<<(unsigned)((P.h.nmol + 7) / 8), 256, 0, st>>>(P.mols, P.h.nmol, P.shells, P.pinfo);
+  if (np > 0) {
     k_su_prims<<<(unsigned)((np + 127) / 128), 128, 0, st>>>(P.su.mol, P.su.off + B2_SU_PAIRS * (P.h.nmol + 1ll),
                                                              P.h.nmol, P.su.su, P.su.pr64, P.su.pr32, P.su.pn);
-    b2_count_launches(2);
+    b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
   }
   return B2_OK;
