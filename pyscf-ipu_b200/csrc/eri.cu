@@ -150,21 +150,24 @@ k_eri_ss(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict
   }
 }
 
-// The other classes: 4 lanes per ket pair, 8 kets at a time; a lane takes every fourth of its
-// ket's primitives and sums, over the bra's primitives (shared memory), the derivatives Phi of the
-// class (up to 40 values in registers).  The ket's polynomial turns them into up to 16 integrals
-// per bra function, which a two-step transposing butterfly sums over the ket's lanes: lane li
-// ends with the integrals of ket function li, in registers until the ket is done.
+// The other classes: a ket pair's primitives are cut into units of four, one per lane of a group of
+// four lanes, and the task's units are packed over the warp's eight groups (with whole ket pairs per
+// group and as many passes as the longest pair of a pass needs, 19-21 of 32 lanes worked).  A lane
+// sums, over the bra's primitives (shared memory), the derivatives Phi of the class (up to 40 values
+// in registers).  The ket's polynomial turns them into up to 16 integrals per bra function, which a
+// two-step transposing butterfly sums over the group: lane li ends with the integrals of ket function
+// li.  A pair's further units (at most three in all) sit in the next groups, or at the next pass's
+// start: a segmented scan over groups and a carry combine them, and the pair's last group writes.
 // Bound by FP32 issue (float32) and by the chain of a quartet at 8 warps per SM (float64, 242
 // registers).  Before: 16 kernels, one per l class over the unmerged shells, every integral
 // accumulated per primitive quartet: 2.2 times the quartets, each with its own Boys evaluation.
-// All classes and the exchange list, 2048 molecules float32: 67.6 -> 38.2 ms; 50 molecules float64:
-// 5.21 -> 2.07 ms.
+// All classes and the exchange list, 2048 molecules float32: 67.6 -> 38.2 ms, 36.0 ms with the units
+// packed; 50 molecules float64: 5.21 -> 2.06 ms.
 template <typename T> struct __align__(16) B2EriWarp {
   B2EriBra<T> bra[B2_MAXPP];
   double CD[32][3];
   int ao[32][4];
-  unsigned char n[32], same[32];
+  unsigned char n[32], same[32], off[32], map[96];
 };
 template <typename T, int TB, int TK>
 __global__ void __launch_bounds__(128)
@@ -195,34 +198,42 @@ k_eri_su(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict
       for (int x = 0; x < 3; ++x) AB[x] = sm[t.A].R[x] - sm[t.B].R[x];
       b2es_bra(pr[(p0 + t.pair) * B2_MAXPP + lane], TB == 2, t.f, AB, W.bra[lane]);
     }
-    W.n[lane] = 0;
+    int nu = 0;                                      // units of this lane's ket (a pair without primitives has one)
     if (lane < t.cnt) {
       int c, d;
       b2gs_pair(g.ns, g.np, kf + lane, c, d);
-      W.n[lane] = (unsigned char)b2_eri_n(pn[p0 + kf + lane], pr);
+      const int n = b2_eri_n(pn[p0 + kf + lane], pr);
+      nu = max(1, (n + 3) >> 2);
+      W.n[lane] = (unsigned char)n;
       W.same[lane] = (unsigned char)((c == d) + 2 * (t.pair == kf + lane));
       W.ao[lane][0] = sm[c].ao_s; W.ao[lane][1] = sm[c].ao_p; W.ao[lane][2] = sm[d].ao_s; W.ao[lane][3] = sm[d].ao_p;
 #pragma unroll
       for (int x = 0; x < 3; ++x) W.CD[lane][x] = sm[c].R[x] - sm[d].R[x];
     }
+    int inc = nu;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    const int U = __shfl_sync(0xffffffffu, inc, 31);
+    W.off[lane] = (unsigned char)(inc - nu);
+    for (int j = 0; j < nu; ++j) W.map[inc - nu + j] = (unsigned char)lane;
     const int F = TB == 2 ? (sm[t.A].ao_p < 0 ? -1 : sm[t.A].ao_p + t.f) : sm[t.A].ao_s;
     const int bs = sm[t.B].ao_s, bp = sm[t.B].ao_p;
     T *o = out + mols[t.m].eri_off;
     __syncwarp();
     auto perm = [&](int x) { return t.f + x >= 3 ? t.f + x - 3 : t.f + x; };
+    T carry[NB][NO];
+    int kc = -1;                                     // ket of the last pass's last group
 #pragma unroll 1
-    for (int k8 = 0; k8 < t.cnt; k8 += 8) {
-      const int kk = k8 + qd, n = W.n[kk];
-      const int npass = (__reduce_max_sync(0xffffffffu, n) + 3) >> 2;
+    for (int u0 = 0; u0 < U; u0 += 8) {
+      const int u = u0 + qd;
+      const int kk = u < U ? (int)W.map[u] : -2 - qd;  // groups past the end: unique keys
+      const int sub = kk >= 0 ? u - (int)W.off[kk] : 0, j = 4 * sub + li;
+      const bool act = kk >= 0 && j < (int)W.n[max(kk, 0)];
       T acc[NB][NO];
-#pragma unroll
-      for (int b = 0; b < NB; ++b)
-#pragma unroll
-        for (int e = 0; e < NO; ++e) acc[b][e] = (T)0;
-#pragma unroll 1
-      for (int ps = 0; ps < npass; ++ps) {
-        const int j = 4 * ps + li;
-        const bool act = j < n;
+      {
         T phi[NB][S::NP];
         S::zero(phi);
         B2EriKet<T> q;
@@ -247,11 +258,35 @@ k_eri_su(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict
 #pragma unroll
           for (int e = 0; e < NO; ++e) {
             const T keep = od ? h[NO + e] : h[e];
-            acc[b][e] += keep + __shfl_xor_sync(0xffffffffu, od ? h[e] : h[NO + e], 1);
+            acc[b][e] = keep + __shfl_xor_sync(0xffffffffu, od ? h[e] : h[NO + e], 1);
           }
         }
       }
-      if (kk < t.cnt) {
+      // the carry, then an inclusive scan over the groups of one ket (at most three)
+      const bool cont = qd == 0 && kk == kc;
+      const bool s1 = __shfl_up_sync(0xffffffffu, kk, 4) == kk && qd >= 1;
+      const bool s2 = __shfl_up_sync(0xffffffffu, kk, 8) == kk && qd >= 2;
+      if (__any_sync(0xffffffffu, cont || s1)) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int e = 0; e < NO; ++e) {
+            if (cont) acc[b][e] += carry[b][e];
+            const T y = __shfl_up_sync(0xffffffffu, acc[b][e], 4);
+            if (s1) acc[b][e] += y;
+            const T z = __shfl_up_sync(0xffffffffu, acc[b][e], 8);
+            if (s2) acc[b][e] += z;
+          }
+      }
+      const bool last = kk >= 0 && 4 * (sub + 1) >= (int)W.n[max(kk, 0)];
+      kc = __shfl_sync(0xffffffffu, last ? -1 : kk, 28);   // a ket that goes on in the next pass
+      if (kc >= 0) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b)
+#pragma unroll
+          for (int e = 0; e < NO; ++e) carry[b][e] = __shfl_sync(0xffffffffu, acc[b][e], 28 + li);
+      }
+      if (last) {
         const int cs = W.ao[kk][0], cp = W.ao[kk][1], ds = W.ao[kk][2], dp = W.ao[kk][3];
         const bool same2 = W.same[kk] & 1, same = W.same[kk] & 2;
 #pragma unroll
