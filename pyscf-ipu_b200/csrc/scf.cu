@@ -170,16 +170,20 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
   return sweep;
 }
 
-// Jacobi on the 10 x 10 DIIS matrix A (shared memory, row-major) run by one warp; V <- the
-// eigenvectors.  Round-robin order: the five rotations of a round act on disjoint pairs, so lanes
-// 0..4 compute them and 25 lanes apply G_k A_kl G_l^T to the 2 x 2 blocks, nine rounds per sweep
-// (the serial order's 45 dependent rotations per sweep took 95 us per call, most of a small
-// molecule's iteration; 61 us in round-robin order with the angle in float64, 48 us now).  The tangent is taken in float32, as in
+// Jacobi on the leading ne rows and columns of the 10 x 10 DIIS matrix A (shared memory, row-major;
+// the border and the filled ring slots, rounded up to an even number; the others are zero, i.e.
+// decoupled) run by one warp; V <- the eigenvectors.  Round-robin order: the ne / 2 rotations of a
+// round act on disjoint pairs, so as many lanes compute them, and the pairs, and up to 25 lanes apply
+// G_k A_kl G_l^T to the 2 x 2 blocks.  What bounds it is the chain of rounds.  k_fock_diis per call at
+// 7 orbitals: 95 us in the serial order (45 dependent rotations per sweep), 61 us in rounds, 48 us with
+// the tangent in float32, 41 us over the leading rows alone.  The tangent is taken in float32, as in
 // b2_jacobi1; couplings below float32's range are far below the stopping norm (the border of B
 // holds ones).
-__device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
+__device__ void b2_jacobi_small_warp(double *A, double *V, double *rot, int *prs, int ne) {
   constexpr int n = 10;
-  const int l = threadIdx.x & 31;
+  const int l = threadIdx.x & 31, half = ne >> 1;
+  const int bk = l / half, bl = l - bk * half;            // this lane's block of pairs
+  const bool blk = l < half * half;
   for (int e = l; e < n * n; e += 32) V[e] = (e / n == e - (e / n) * n) ? 1.0 : 0.0;
   __syncwarp();
   for (int sweep = 0; sweep < 50; ++sweep) {
@@ -195,19 +199,15 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
       tot += __shfl_xor_sync(0xffffffffu, tot, o);
     }
     if (off <= 1e-28 * tot || off < 1e-300) break;
-    for (int r = 0; r < n - 1; ++r) {
-      auto pair = [&](int k, int &p, int &q) {
-        int a = k - 1 + r, b = n - 2 - k + r;
-        if (a >= n - 1) a -= n - 1;
-        if (b >= n - 1) b -= n - 1;
-        a = (k == 0) ? 0 : a + 1;
+    for (int r = 0; r < ne - 1; ++r) {
+      if (l < half) {
+        // round-robin pairs: index 0 fixed, the others rotate by r
+        int a = l - 1 + r, b = ne - 2 - l + r;
+        if (a >= ne - 1) a -= ne - 1;
+        if (b >= ne - 1) b -= ne - 1;
+        a = (l == 0) ? 0 : a + 1;
         b += 1;
-        p = min(a, b);
-        q = max(a, b);
-      };
-      if (l < 5) {
-        int p, q;
-        pair(l, p, q);
+        const int p = min(a, b), q = max(a, b);
         double c = 1.0, s = 0.0;
         const double apq = A[p * n + q], app = A[p * n + p], aqq = A[q * n + q];
         if (fabs(apq) > 1e-36 && apq * apq > 1e-36 * fabs(app * aqq)) {
@@ -219,28 +219,26 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot) {
         }
         rot[2 * l] = c;
         rot[2 * l + 1] = s;
+        prs[2 * l] = p;
+        prs[2 * l + 1] = q;
       }
       __syncwarp();
-      if (l < 25) {
-        const int bk = l / 5, bl = l - (l / 5) * 5;
-        int p, q, u, v;
-        pair(bk, p, q);
-        pair(bl, u, v);
+      if (blk) {
+        const int p = prs[2 * bk] * n, q = prs[2 * bk + 1] * n, u = prs[2 * bl], v = prs[2 * bl + 1];
         const double ck = rot[2 * bk], sk = rot[2 * bk + 1], cl = rot[2 * bl], sl = rot[2 * bl + 1];
-        const double a00 = A[p * n + u], a01 = A[p * n + v], a10 = A[q * n + u], a11 = A[q * n + v];
+        const double a00 = A[p + u], a01 = A[p + v], a10 = A[q + u], a11 = A[q + v];
+        double *v0 = V + 2 * bk * n, *v1 = v0 + n;         // V's rows 2 bk, 2 bk + 1, columns of pair bl
+        const double x0 = v0[u], y0 = v0[v], x1 = v1[u], y1 = v1[v];
         const double b00 = ck * a00 - sk * a10, b10 = sk * a00 + ck * a10;
         const double b01 = ck * a01 - sk * a11, b11 = sk * a01 + ck * a11;
-        A[p * n + u] = cl * b00 - sl * b01;
-        A[p * n + v] = sl * b00 + cl * b01;
-        A[q * n + u] = cl * b10 - sl * b11;
-        A[q * n + v] = sl * b10 + cl * b11;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {                   // V's rows 2 bk, 2 bk + 1, columns of pair bl
-          double *vr = V + (2 * bk + h) * n;
-          const double x = vr[u], y = vr[v];
-          vr[u] = cl * x - sl * y;
-          vr[v] = sl * x + cl * y;
-        }
+        A[p + u] = cl * b00 - sl * b01;
+        A[p + v] = sl * b00 + cl * b01;
+        A[q + u] = cl * b10 - sl * b11;
+        A[q + v] = sl * b10 + cl * b11;
+        v0[u] = cl * x0 - sl * y0;
+        v0[v] = sl * x0 + cl * y0;
+        v1[u] = cl * x1 - sl * y1;
+        v1[v] = sl * x1 + cl * y1;
       }
       __syncwarp();
     }
@@ -267,6 +265,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
   __shared__ double sc[10];
   __shared__ double stmp[9];
   __shared__ double sA[100], sV[100], sRot[10];
+  __shared__ int sPrs[10];
   const B2MolDev md = mols[m];
   const int N = md.nao, NN = N * N;
   const long long mo = md.mat_off;
@@ -344,7 +343,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
       sA[i] = keep ? B[i] : 0.0;
     }
     __syncwarp();
-    b2_jacobi_small_warp(sA, sV, sRot);
+    b2_jacobi_small_warp(sA, sV, sRot, sPrs, (nfill + 2) & ~1);
     __syncwarp();
     double smax = 0;
     for (int i = 0; i < 10; ++i) smax = fmax(smax, fabs(sA[i * 10 + i]));
@@ -600,16 +599,21 @@ static int b2_per_bucket(const B2PlanDev &P, cudaStream_t st, F launch) {
   const bool sub = P.sub.n > 0;
   const std::vector<int> &off = sub ? P.sub.bkt_off_h : P.bkt_off_h;
   const int *map = sub ? P.sub.bkt_map : P.bkt_map;
-  B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
+  int used = 0;
+  for (int b = 0; b < B2_NBKT; ++b) used += off[b + 1] > off[b];
+  if (used > 1) B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
   for (int b = B2_NBKT - 1; b >= 0; --b) {          // largest molecules first
     const int n = off[b + 1] - off[b];
     if (n <= 0) continue;
-    B2_CUDA_TRY(cudaStreamWaitEvent(P.bkt_stream[b], P.bkt_ev[B2_NBKT], 0));
-    B2_CUDA_TRY(launch(b + 1, n, map + off[b], P.bkt_stream[b]));
+    const cudaStream_t s = used > 1 ? P.bkt_stream[b] : st;   // one bucket: the caller's stream itself
+    if (used > 1) B2_CUDA_TRY(cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0));
+    B2_CUDA_TRY(launch(b + 1, n, map + off[b], s));
     b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
-    B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[b], P.bkt_stream[b]));
-    B2_CUDA_TRY(cudaStreamWaitEvent(st, P.bkt_ev[b], 0));
+    if (used > 1) {
+      B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[b], s));
+      B2_CUDA_TRY(cudaStreamWaitEvent(st, P.bkt_ev[b], 0));
+    }
   }
   return B2_OK;
 }
