@@ -226,16 +226,21 @@ __global__ void k_sym(const B2MolDev *__restrict__ mols, const int *__restrict__
   }
 }
 
+// slots > 0: runs that fill the rounds of that many resident CTAs (b2_xc_run).  The float64 kernel's
+// tiles are long (12 us at 62 orbitals, two CTAs per SM) and its CTAs few: 8500 tiles in runs of 7 took
+// 4.1 rounds, i.e. five, 443 us; 383 us as two rounds of runs of 15.
 static void b2_xc_split(const std::vector<long long> &goff, int nmol, int pt, int &tpc,
-                        std::vector<long long> &xblk, int tpc_fixed = 0) {
+                        std::vector<long long> &xblk, int tpc_fixed = 0, int slots = 0) {
+  std::vector<long long> nts(nmol);
   long long tiles = 0;
-  for (int m = 0; m < nmol; ++m) tiles += (goff[m + 1] - goff[m] + pt - 1) / pt;
+  for (int m = 0; m < nmol; ++m) tiles += nts[m] = (goff[m + 1] - goff[m] + pt - 1) / pt;
   // enough CTAs to fill the GPU several times over, each flushing V once
-  tpc = tpc_fixed > 0 ? tpc_fixed : (int)std::max(1ll, std::min(16ll, tiles / (8ll * 148ll)));
+  tpc = tpc_fixed > 0 ? tpc_fixed
+        : slots > 0   ? b2_xc_run(nts, slots, 1, 16)
+                      : (int)std::max(1ll, std::min(16ll, tiles / (8ll * 148ll)));
   xblk.assign(nmol + 1, 0);
   for (int m = 0; m < nmol; ++m) {
-    const long long nt = (goff[m + 1] - goff[m] + pt - 1) / pt;
-    xblk[m + 1] = xblk[m] + (nt + tpc - 1) / tpc;
+    xblk[m + 1] = xblk[m] + (nts[m] + tpc - 1) / tpc;
   }
 }
 
@@ -251,7 +256,7 @@ int b2_grid_setup(B2PlanDev &P, const long long *grid_off_host) {
     aoff[m + 1] = aoff[m] + 4 * G * P.h.mols[m].nao;
   }
   b2_xc_split(goff, nmol, 64, P.g.tpc32, x32);
-  b2_xc_split(goff, nmol, 32, P.g.tpc64, x64);
+  b2_xc_split(goff, nmol, 32, P.g.tpc64, x64, 0, 2 * 148);
   b2_xc_split(goff, nmol, 128, P.g.tpc_tc, xtc);
   P.g.n_points = goff[nmol];
   P.g.n_gblk = gblk[nmol];
@@ -288,6 +293,7 @@ int b2_grid_setup(B2PlanDev &P, const long long *grid_off_host) {
 int b2_xc_set_tpc(B2PlanDev &P, int tpc) {
   if (!P.g.grid_off || tpc < 0) return B2_ERR_ARG;
   for (int b = 0; b < B2_NBKT; ++b) P.g.xq_tpc[b] = 0;    // one value for every bucket
+  P.g.xq_exact = tpc > 0;
   std::vector<long long> xtc;
   b2_xc_split(P.g.grid_off_h, P.h.nmol, 128, P.g.tpc_tc, xtc, tpc);
   long long *d = nullptr;

@@ -206,7 +206,7 @@ k_xc_direct(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shell
 // that bucket (2 CTAs per SM at 64 orbitals, 4 up to 32).
 // 272 000 points x 62 orbitals: 1117 us per evaluation with CUDA-core products in one 134 KB CTA
 // per SM and the functional on one lane in 16; 610 us with MMA products, one CTA per SM resident
-// and every l shell's own exponentials; 436 us now.
+// and every l shell's own exponentials; 436 us before runs of tiles filled the rounds of CTAs, 383 us now.
 template <int Q>
 __global__ void __launch_bounds__(256, B2_XF_CTAS(Q))
 k_xc_f64(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, const B2gSuper *__restrict__ su,

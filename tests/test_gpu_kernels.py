@@ -326,6 +326,45 @@ def test_xc_float64_sizes(cuda, heavy):
     eng.close()
 
 
+@pytest.mark.parametrize("nmol", [1, 2, 5, 24])
+def test_xc_run_lengths(cuda, nmol):
+    """runs of tiles shortened to a small batch's share of the GPU (half the configured length and
+    more, with short last runs) against items of exactly one tile, whole batch and last molecule
+    alone.  float32 accumulators over at most 16 tiles: 1e-6 of E_xc, 1e-5 of
+    max|V|, as for the tile counts above."""
+    rng = np.random.default_rng(60 + nmol)
+    mols = [Mole(random_molecule(rng, int(k))) for k in rng.integers(1, 10, size=nmol)]
+    eng = RKSEngine(mols, level=0, precision="mixed", guess="minao", tuned=False)
+    eng.device_setup()
+    eng.D.copy_(eng.D0)
+    P, got = eng.plan, {}
+    for tiles in (16, 1):
+        if tiles > 1:
+            counts = np.full(5, tiles, np.int32)
+            check(lib().b2_plan_set_xc_bucket_tiles(P.h, ptr(counts)), "b2_plan_set_xc_bucket_tiles")
+        else:
+            check(lib().b2_plan_set_xc_tiles(P.h, tiles), "b2_plan_set_xc_tiles")
+        eng.xc()
+        torch.cuda.synchronize()
+        got[tiles] = (eng.exc.cpu().numpy().copy(), eng.Vxc.cpu().numpy().copy())
+        idx = np.array([nmol - 1], np.int32)
+        check(lib().b2_plan_set_subset(P.h, ptr(idx), 1), "b2_plan_set_subset")
+        act = torch.zeros(nmol, dtype=torch.int32, device=cuda)
+        act[nmol - 1] = 1
+        eng.xc(active=act)
+        torch.cuda.synchronize()
+        check(lib().b2_plan_set_subset(P.h, None, 0), "b2_plan_set_subset")
+        got[tiles] += (eng.exc.cpu().numpy().copy(), eng.Vxc.cpu().numpy().copy())
+    vmax = np.abs(got[1][1]).max()
+    for k in (0, 2):
+        np.testing.assert_allclose(got[16][k], got[1][k], rtol=1e-6)
+        np.testing.assert_allclose(got[16][k + 1], got[1][k + 1], atol=1e-5 * vmax)
+    st = ctypes.c_int(-1)
+    check(lib().b2_xc_tc_status(1, ctypes.byref(st)), "b2_xc_tc_status")
+    assert st.value == 0
+    eng.close()
+
+
 @pytest.mark.parametrize("prec, tol", [(64, 1e-11), (32, 5e-6)])
 def test_eri_batch_sizes(cuda, prec, tol):
     """batched integrals at the edges of the super-shell kernels: s shells only, one sp shell, more
