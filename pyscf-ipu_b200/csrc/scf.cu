@@ -76,6 +76,10 @@ __device__ __forceinline__ void b2_mm_out(const double (&acc)[Q][4], int N, F f)
     }
 }
 
+// CTAs per SM that the shared memory of the two kernels allows, kept within reach of the registers
+// (many molecules at once; a single one has the SM to itself)
+#define B2_SCF_CTAS(Q) ((Q) == 1 ? 10 : (Q) == 2 ? 6 : 7 - (Q))
+
 // ------------------------------------------------------------------ eigensolver
 // One-sided Jacobi (Hestenes) on the symmetric A: G = A / |A| + 2 I (|A| the largest row sum, so
 // the spectrum of G lies in [1, 3]), columns rotated pairwise until they are orthogonal; then
@@ -126,13 +130,15 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
       b += 1;
       double *cp = G + min(a, b) * LD, *cq = G + max(a, b) * LD;
       const double app = on ? nrm[min(a, b)] : 0.0, aqq = on ? nrm[max(a, b)] : 0.0;
-      double vp[RP], vq[RP], x = 0;
+      double vp[RP], vq[RP], x = 0, x1 = 0;          // two chains
 #pragma unroll
       for (int j = 0; j < RP; ++j) {
         vp[j] = on ? cp[li + 8 * j] : 0.0;
         vq[j] = on ? cq[li + 8 * j] : 0.0;
-        x += vp[j] * vq[j];
+        if (j & 1) x1 += vp[j] * vq[j];
+        else x += vp[j] * vq[j];
       }
+      x += x1;
       x += __shfl_xor_sync(0xffffffffu, x, 4);
       x += __shfl_xor_sync(0xffffffffu, x, 2);
       x += __shfl_xor_sync(0xffffffffu, x, 1);
@@ -141,9 +147,12 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
         big = big || x2 > 1e-17 * pq;
         // sym.schur2 (Golub & Van Loan): t = sign(d b) |b| / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 x
         const float d = (float)(aqq - app), bb = (float)(2.0 * x);
-        const float tf = copysignf(1.0f, d * bb) * fabsf(bb) / (fabsf(d) + sqrtf(d * d + bb * bb));
+        const float q2 = d * d + bb * bb;
+        const float tf = copysignf(1.0f, d * bb) * __fdividef(fabsf(bb), fabsf(d) + q2 * rsqrtf(q2));
         const double t = d == 0.0f ? (x > 0 ? 1.0 : -1.0) : (double)tf;
-        const double c = rsqrt(1.0 + t * t), s = t * c;
+        // 1 / sqrt(1 + t^2): float seed (e = 1 - u y^2 near 1e-7), one third-order step (Householder)
+        const double u = fma(t, t, 1.0), y = (double)rsqrtf((float)u), e = fma(-u * y, y, 1.0);
+        const double c = fma(y * e, fma(0.375, e, 0.5), y), s = t * c;
 #pragma unroll
         for (int j = 0; j < RP; ++j) {
           cp[li + 8 * j] = c * vp[j] - s * vq[j];
@@ -248,9 +257,10 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot, int *prs
 // ------------------------------------------------------------------ Fock + DIIS
 // ring layout per molecule (offset mat_off * 9): errs[9][N*N], hams[9][N*N]; B: 100 doubles
 // Bound by latency at one molecule per CTA; 62 orbitals, one molecule: 172 us per call before (two
-// products with one output element per thread, serial 10 x 10 Jacobi), 135 us now.
+// products with one output element per thread, serial 10 x 10 Jacobi), 139 us with element-wise
+// ring passes, 95 us with several elements' loads in flight.
 template <int Q>
-__global__ void __launch_bounds__(64 * Q)
+__global__ void __launch_bounds__(64 * Q, B2_SCF_CTAS(Q))
 k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
             const int *__restrict__ iter, double hyb, int use_diis, const double *__restrict__ Hcore,
             const double *__restrict__ S, const double *__restrict__ D, const double *__restrict__ J,
@@ -272,6 +282,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
   double *sH = sm, *sT = sH + 16 * Q * LD;
   for (int e = threadIdx.x; e < 2 * 16 * Q * LD; e += blockDim.x) sm[e] = 0.0;   // padding stays zero
   __syncthreads();
+#pragma unroll 4
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     const double djk = J[mo + e] - 0.5 * hyb * K[mo + e];
     diffJK[mo + e] = djk;
@@ -297,16 +308,28 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
   double emax = 0, s9[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) s9[k] = 0.0;
-  for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-    const int a = e / N, b = e - (e / N) * N;
-    const double v = sT[a * LD + b] - sT[b * LD + a];
-    emax = fmax(emax, fabs(v));
-    er[(long long)head * NN + e] = v;
-    hr[(long long)head * NN + e] = sH[a * LD + b];
-    // the nine dot products <err_k, err_new> in the same pass
+  // the nine dot products <err_k, err_new> in the same pass; two elements' ring loads in flight
+  for (int e0 = threadIdx.x; e0 < NN; e0 += 2 * blockDim.x) {
+    double r[2][9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k)
-      if (k < nfill) s9[k] += (k == head ? v : er[(long long)k * NN + e]) * v;
+    for (int h = 0; h < 2; ++h) {
+      const int e = e0 + h * (int)blockDim.x;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) r[h][k] = k < nfill && k != head && e < NN ? er[(long long)k * NN + e] : 0.0;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = e0 + h * (int)blockDim.x;
+      if (e >= NN) break;
+      const int a = e / N, b = e - (e / N) * N;
+      const double v = sT[a * LD + b] - sT[b * LD + a];
+      emax = fmax(emax, fabs(v));
+      er[(long long)head * NN + e] = v;
+      hr[(long long)head * NN + e] = sH[a * LD + b];
+#pragma unroll
+      for (int k = 0; k < 9; ++k)
+        if (k < nfill) s9[k] += (k == head ? v : r[h][k]) * v;
+    }
   }
   emax = b2_block_max(emax, red);
   {
@@ -359,6 +382,7 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
     if (l == 0) diis_err[m] = emax;
   }
   __syncthreads();
+#pragma unroll 4
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     double s = 0;
 #pragma unroll
@@ -375,9 +399,10 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
 // and order of eigenvectors, which the density does not depend on.
 // Products: M = L^T W, T = H M, A = M^T T, W' = W V', C = L^T W', D = 2 C_occ C_occ^T, all by
 // float64 MMA; two matrices in shared memory (74 KB at 64 orbitals, 3 CTAs per SM).  62 orbitals,
-// one molecule: 428 us per call before, 168 us now.
+// one molecule: 428 us per call before, 161 us now (168 us with one
+// dot-product chain and the library's reciprocal root).
 template <int Q>
-__global__ void __launch_bounds__(64 * Q)
+__global__ void __launch_bounds__(64 * Q, B2_SCF_CTAS(Q))
 k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
                const int *__restrict__ iter, const double *__restrict__ H,
                const double *__restrict__ Linv, double *__restrict__ D, double *__restrict__ mo_energy,
