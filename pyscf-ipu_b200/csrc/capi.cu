@@ -522,7 +522,7 @@ int b2_scf_iterate(void *plan, const b2_scf_state *S, void *stream) {
     if (!rc) rc = b2_note(cudaStreamWaitEvent(js, P.jk_ev[0], 0));
   }
   if (!rc) rc = S->ao ? b2_launch_xc(P, S->precision, a, S->ao, S->weights, S->D, S->Vxc, S->exc, st)
-                      : b2_launch_xc_direct(P, S->precision, a, S->coords, S->weights, S->D, S->Vxc, S->exc, st);
+                      : b2_launch_xc_direct(P, S->precision, a, S->coords, S->weights, S->D, S->Vxc, S->exc, st, false);
   if (!rc) rc = S->exch ? b2_launch_jk_symv(P, S->precision, a, S->eri, S->exch, S->D, S->J, S->K, P.sv_work, js)
                         : b2_launch_jk_s8(P, S->precision, a, S->eri, S->D, S->J, S->K, js);
   if (!rc && js != st) {
@@ -530,7 +530,7 @@ int b2_scf_iterate(void *plan, const b2_scf_state *S, void *stream) {
     if (!rc) rc = b2_note(cudaStreamWaitEvent(st, P.jk_ev[1], 0));
   }
   if (!rc) rc = b2_launch_energy_jk(P, a, S->D, S->Hcore, S->J, S->K, S->hyb, S->exc, S->enuc, S->diffJK,
-                                    S->energy, S->iter, st);
+                                    S->energy, S->iter, S->ao ? nullptr : S->Vxc, st);
   return rc;
 }
 

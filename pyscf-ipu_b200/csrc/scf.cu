@@ -528,12 +528,15 @@ __global__ void k_energy(const B2MolDev *__restrict__ mols, const int *__restric
 
 // end of one SCF iteration (nanoDFT.py:74-80): diff_JK = J - hyb/2 K of the new density
 // (get_JK, nanoDFT.py:125-139), the five energy terms (nanoDFT.py:20-38) and the molecule's
-// iteration counter advanced; inactive molecules are left untouched
+// iteration counter advanced; with Vsym also V <- V + V^T of the XC kernels; inactive molecules are
+// left untouched.  One launch fewer per iteration, and V + V^T runs where the matrices are read
+// anyway; launches and dependent round trips are what a small molecule's iteration consists of.
 __global__ void k_energy_jk(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
                             const double *__restrict__ D, const double *__restrict__ Hcore,
                             const double *__restrict__ J, const double *__restrict__ K, double hyb,
                             const double *__restrict__ exc, const double *__restrict__ enuc,
-                            double *__restrict__ diffJK, double *__restrict__ out, int *__restrict__ iter) {
+                            double *__restrict__ diffJK, double *__restrict__ out, int *__restrict__ iter,
+                            double *__restrict__ Vsym) {
   const int m = blockIdx.x;
   if (active && !active[m]) return;
   __shared__ double red[32];
@@ -547,6 +550,13 @@ __global__ void k_energy_jk(const B2MolDev *__restrict__ mols, const int *__rest
     diffJK[a] = djk;
     ec += d * Hcore[a];
     ej += d * djk;
+  }
+  if (Vsym) {                                      // V <- V + V^T
+    double *v = Vsym + md.mat_off;
+    for (int e = threadIdx.x; e < NN; e += blockDim.x) {
+      const int a = e / md.nao, b = e - (e / md.nao) * md.nao, t = b * md.nao + a;
+      if (a <= b) v[e] = v[t] = v[e] + v[t];
+    }
   }
   ec = b2_block_sum(ec, red);
   ej = b2_block_sum(ej, red);
@@ -563,8 +573,8 @@ __global__ void k_energy_jk(const B2MolDev *__restrict__ mols, const int *__rest
 
 int b2_launch_energy_jk(const B2PlanDev &P, const int *active, const double *D, const double *Hcore,
                         const double *J, const double *K, double hyb, const double *exc,
-                        const double *enuc, double *diffJK, double *out, int *iter, cudaStream_t st) {
-  k_energy_jk<<<P.h.nmol, 256, 0, st>>>(P.mols, active, D, Hcore, J, K, hyb, exc, enuc, diffJK, out, iter);
+                        const double *enuc, double *diffJK, double *out, int *iter, double *Vsym, cudaStream_t st) {
+  k_energy_jk<<<P.h.nmol, 256, 0, st>>>(P.mols, active, D, Hcore, J, K, hyb, exc, enuc, diffJK, out, iter, Vsym);
   b2_count_launches(1);
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;

@@ -300,9 +300,14 @@ k_xc_f64(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, con
   }
 }
 
-__global__ void k_zero_exc2(int nmol, const int *__restrict__ active, double *__restrict__ exc) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m < nmol && (!active || active[m])) exc[m] = 0.0;
+// V and E_xc of the active molecules (all without a mask) <- 0
+__global__ void k_zero_xc(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
+                          double *__restrict__ V, double *__restrict__ exc) {
+  const int m = blockIdx.x;
+  if (active && !active[m]) return;
+  const B2MolDev md = mols[m];
+  for (int e = threadIdx.x; e < md.nao * md.nao; e += blockDim.x) V[md.mat_off + e] = 0.0;
+  if (threadIdx.x == 0) exc[m] = 0.0;
 }
 
 __global__ void k_sym2(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
@@ -323,13 +328,12 @@ __global__ void k_sym2(const B2MolDev *__restrict__ mols, const int *__restrict_
   }
 }
 
-int b2_zero_exc(const B2PlanDev &P, const int *active, double *exc, cudaStream_t st) {
-  k_zero_exc2<<<(P.h.nmol + 255) / 256, 256, 0, st>>>(P.h.nmol, active, exc);
+int b2_zero_xc(const B2PlanDev &P, const int *active, double *V, double *exc, cudaStream_t st) {
+  k_zero_xc<<<P.h.nmol, 256, 0, st>>>(P.mols, active, V, exc);
   b2_count_launches(1);
   B2_CUDA_TRY(cudaGetLastError());
   return B2_OK;
 }
-
 int b2_sym_v(const B2PlanDev &P, const int *active, double *V, cudaStream_t st) {
   k_sym2<<<P.h.nmol, 256, 0, st>>>(P.mols, active, V);
   b2_count_launches(1);
@@ -366,17 +370,11 @@ static int b2_xf_bucket(const B2PlanDev &P, bool one, const int *active, const d
 
 static int b2_xcd_zero(const B2PlanDev &P, const int *active, double *V, double *exc, cudaStream_t st) {
   if (P.h.max_nbas > B2_XD_MAXSH) return B2_ERR_SIZE;
-  if (active) {
-    int rc = b2_zero_active(P, active, V, nullptr, st);
-    if (rc) return rc;
-  } else {
-    B2_CUDA_TRY(cudaMemsetAsync(V, 0, sizeof(double) * P.h.n_mat, st));
-  }
-  return b2_zero_exc(P, active, exc, st);
+  return b2_zero_xc(P, active, V, exc, st);
 }
 
 static int b2_xc_f64(const B2PlanDev &P, const int *active, const double *coords, const double *w, const double *D,
-                     double *V, double *exc, cudaStream_t st) {
+                     double *V, double *exc, cudaStream_t st, bool sym) {
   int rc = b2_xcd_zero(P, active, V, exc, st);
   if (rc) return rc;
   const std::vector<int> &off = P.sub.n > 0 ? P.sub.bkt_off_h : P.bkt_off_h;
@@ -384,12 +382,12 @@ static int b2_xc_f64(const B2PlanDev &P, const int *active, const double *coords
   for (int b = 0; b < B2_NBKT; ++b) used += off[b + 1] > off[b];
   if (used > 1) B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
   rc = b2_xf_bucket<B2_NBKT>(P, used <= 1, active, coords, w, D, V, exc, st);
-  return rc ? rc : b2_sym_v(P, active, V, st);
+  return rc || !sym ? rc : b2_sym_v(P, active, V, st);
 }
 
 // float32 on the CUDA cores (implementation 1)
 static int b2_xcd_f32(const B2PlanDev &P, const int *active, const double *coords, const double *w, const double *D,
-                      double *V, double *exc, cudaStream_t st) {
+                      double *V, double *exc, cudaStream_t st, bool sym) {
   constexpr int PT = 64, NBmax = 80;
   const bool sub = P.sub.n > 0;
   const long long nblk = sub ? P.sub.n_x32 : P.g.n_xblk32;
@@ -404,17 +402,18 @@ static int b2_xcd_f32(const B2PlanDev &P, const int *active, const double *coord
     b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
   }
-  return b2_sym_v(P, active, V, st);
+  return sym ? b2_sym_v(P, active, V, st) : B2_OK;
 }
 
 int b2_launch_xc_direct(const B2PlanDev &P, int precision, const int *active, const double *coords,
-                        const double *w, const double *D, double *V, double *exc, cudaStream_t st) {
+                        const double *w, const double *D, double *V, double *exc, cudaStream_t st,
+                        bool sym) {
   if (!P.g.grid_off) return B2_ERR_ARG;
-  if (precision == 64) return b2_xc_f64(P, active, coords, w, D, V, exc, st);
+  if (precision == 64) return b2_xc_f64(P, active, coords, w, D, V, exc, st, sym);
   if (precision == 32 && P.xc_impl == 0)
-    return b2_launch_xc_tq(P, active, coords, w, D, V, exc, st);
+    return b2_launch_xc_tq(P, active, coords, w, D, V, exc, st, sym);
   if (precision == 32 && P.xc_impl == 2)
-    return b2_launch_xc_tc(P, active, coords, w, D, V, exc, st);
-  if (precision == 32) return b2_xcd_f32(P, active, coords, w, D, V, exc, st);
+    return b2_launch_xc_tc(P, active, coords, w, D, V, exc, st, sym);
+  if (precision == 32) return b2_xcd_f32(P, active, coords, w, D, V, exc, st, sym);
   return B2_ERR_ARG;
 }

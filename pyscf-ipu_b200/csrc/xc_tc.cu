@@ -538,7 +538,7 @@ k_xc_tc(const B2MolDev *__restrict__ mols, const B2Shell *__restrict__ shells,
 }
 
 int b2_launch_xc_tc(const B2PlanDev &P, const int *active, const double *coords, const double *w,
-                    const double *D, double *V, double *exc, cudaStream_t st) {
+                    const double *D, double *V, double *exc, cudaStream_t st, bool sym) {
   const bool sub = P.sub.n > 0;
   const int nm = sub ? P.sub.n : P.h.nmol;
   const int *map = sub ? P.sub.mol_map : nullptr;
@@ -546,13 +546,7 @@ int b2_launch_xc_tc(const B2PlanDev &P, const int *active, const double *coords,
   const long long nblk = sub ? P.sub.n_xtc : P.g.n_xblk_tc;
   if (P.h.max_nbas > B2_XT_MAXSH || P.h.max_nao > 80) return B2_ERR_SIZE;
   if (!xblk) return B2_ERR_ARG;
-  if (active) {
-    int rc = b2_zero_active(P, active, V, nullptr, st);
-    if (rc) return rc;
-  } else {
-    B2_CUDA_TRY(cudaMemsetAsync(V, 0, sizeof(double) * P.h.n_mat, st));
-  }
-  int rc = b2_zero_exc(P, active, exc, st);
+  int rc = b2_zero_xc(P, active, V, exc, st);
   if (rc) return rc;
   const int NBmax = 16 * ((P.h.max_nao + 15) / 16);
   const size_t sm = sizeof(float) * (size_t)b2_xt_smem_floats(NBmax < 16 ? 16 : NBmax);
@@ -562,7 +556,7 @@ int b2_launch_xc_tc(const B2PlanDev &P, const int *active, const double *coords,
                                                   P.g.tpc_tc, active, coords, w, D, V, exc, map);
     b2_count_launches(1);
   }
-  return b2_sym_v(P, active, V, st);
+  return sym ? b2_sym_v(P, active, V, st) : B2_OK;
 }
 
 // ============================================================================================
@@ -1045,28 +1039,25 @@ static int b2_xq_launch(const B2PlanDev &P, const B2XtItem *items, int n_items, 
 }
 
 int b2_launch_xc_tq(const B2PlanDev &P, const int *active, const double *coords, const double *w,
-                    const double *D, double *V, double *exc, cudaStream_t st) {
+                    const double *D, double *V, double *exc, cudaStream_t st, bool sym) {
   const bool sub = P.sub.n > 0;
   const B2XtItem *items = (const B2XtItem *)(sub ? P.sub.xq_items : P.g.xq_items);
   const std::vector<long long> &off = sub ? P.sub.xq_off_h : P.g.xq_off_h;
   if (P.h.max_nbas > B2_XT_MAXSH || P.h.max_nao > 80) return B2_ERR_SIZE;
   if (!items || off.size() != B2_NBKT + 1 || !P.g.xq_queue) return B2_ERR_ARG;
-  if (active) {
-    int rc = b2_zero_active(P, active, V, nullptr, st);
-    if (rc) return rc;
-  } else {
-    B2_CUDA_TRY(cudaMemsetAsync(V, 0, sizeof(double) * P.h.n_mat, st));
-  }
-  int rc = b2_zero_exc(P, active, exc, st);
+  int rc = b2_zero_xc(P, active, V, exc, st);
   if (rc) return rc;
   B2_CUDA_TRY(cudaMemsetAsync(P.g.xq_queue, 0, sizeof(int) * B2_NBKT, st));
-  // one launch per bucket on the plan's bucket streams (forked from / joined to `st`)
-  B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
+  // one launch per bucket on the plan's bucket streams (forked from / joined to `st`); a single one
+  // runs on `st` itself
+  int used = 0;
+  for (int b = 0; b < B2_NBKT; ++b) used += off[b + 1] > off[b];
+  if (used > 1) B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[B2_NBKT], st));
   for (int b = B2_NBKT - 1; b >= 0; --b) {
     const int n = (int)(off[b + 1] - off[b]);
     if (n <= 0) continue;
-    cudaStream_t s = P.bkt_stream[b];
-    B2_CUDA_TRY(cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0));
+    const cudaStream_t s = used > 1 ? P.bkt_stream[b] : st;
+    if (used > 1) B2_CUDA_TRY(cudaStreamWaitEvent(s, P.bkt_ev[B2_NBKT], 0));
     const B2XtItem *it = items + off[b];
     int *q = P.g.xq_queue + b;
     switch (b) {
@@ -1079,10 +1070,12 @@ int b2_launch_xc_tq(const B2PlanDev &P, const int *active, const double *coords,
     if (rc) return rc;
     b2_count_launches(1);
     B2_CUDA_TRY(cudaGetLastError());
-    B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[b], s));
-    B2_CUDA_TRY(cudaStreamWaitEvent(st, P.bkt_ev[b], 0));
+    if (used > 1) {
+      B2_CUDA_TRY(cudaEventRecord(P.bkt_ev[b], s));
+      B2_CUDA_TRY(cudaStreamWaitEvent(st, P.bkt_ev[b], 0));
+    }
   }
-  return b2_sym_v(P, active, V, st);
+  return sym ? b2_sym_v(P, active, V, st) : B2_OK;
 }
 
 // Tiles per CTA (or per work item) for molecules of nt[...] tiles on `slots` resident CTAs: from
