@@ -543,6 +543,7 @@ __global__ void k_energy_jk(const B2MolDev *__restrict__ mols, const int *__rest
   const B2MolDev md = mols[m];
   const int NN = md.nao * md.nao;
   double ec = 0, ej = 0;
+#pragma unroll 4
   for (int e = threadIdx.x; e < NN; e += blockDim.x) {
     const long long a = md.mat_off + e;
     const double d = D[a];
@@ -551,11 +552,20 @@ __global__ void k_energy_jk(const B2MolDev *__restrict__ mols, const int *__rest
     ec += d * Hcore[a];
     ej += d * djk;
   }
-  if (Vsym) {                                      // V <- V + V^T
+  if (Vsym) {                                      // V <- V + V^T, four elements' loads in flight
     double *v = Vsym + md.mat_off;
-    for (int e = threadIdx.x; e < NN; e += blockDim.x) {
-      const int a = e / md.nao, b = e - (e / md.nao) * md.nao, t = b * md.nao + a;
-      if (a <= b) v[e] = v[t] = v[e] + v[t];
+    for (int e0 = threadIdx.x; e0 < NN; e0 += 4 * blockDim.x) {
+      double x[4];
+      int t[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int e = e0 + k * (int)blockDim.x, a = e / md.nao, b = e - (e / md.nao) * md.nao;
+        t[k] = e < NN && a <= b ? b * md.nao + a : -1;
+        x[k] = t[k] >= 0 ? v[e] + v[t[k]] : 0.0;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (t[k] >= 0) v[e0 + k * (int)blockDim.x] = v[t[k]] = x[k];
     }
   }
   ec = b2_block_sum(ec, red);
