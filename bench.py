@@ -129,7 +129,7 @@ def kernel_rooflines(eng, precision):
     quartets, prim = quartet_counts(eng.mols)
     prec = 64 if precision == "fp64" else 32
     eri_ms = _timed(lambda: check(lib().b2_eri_s8(P.h, prec, ptr(eng.eri), stream_handle()), "b2_eri_s8"), 3)
-    e = {"kernel": "k_eri_fl / k_eri_sq (16 class kernels)", "bound": "fp32 simt", "ms_per_launch": eri_ms,
+    e = {"kernel": "k_eri_ss / k_eri_su (6 class kernels)", "bound": "fp32 simt", "ms_per_launch": eri_ms,
          "shell_quartets_per_s": quartets / (eri_ms / 1e3), "shell_quartets": quartets,
          "primitive_quartets_unscreened": prim}
     if prec == 32:
