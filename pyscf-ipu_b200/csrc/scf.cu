@@ -90,8 +90,14 @@ __device__ __forceinline__ void b2_mm_out(const double (&acc)[Q][4], int N, F f)
 // and the eigenvectors, two barriers) took 2.2 us per round at 62 orbitals.
 // The angle's tangent is taken in float32 (the rotation itself is exactly orthogonal: cosine and
 // sine follow from that tangent in float64), which leaves 1e-7 of a coupling behind and shortens
-// the round's serial chain.  A sweep whose largest cosine between columns was below 3e-9 leaves
-// couplings at rounding level and is the last.
+// the round's serial chain.  A sweep is the last when its largest cosine was below 3e-9 and all its
+// angles below 1e-6: what such rotations mix into pairs already treated is at rounding level.  A
+// wide rotation may come from a cosine of any size where eigenvalues coincide, and carries the
+// couplings of one column over to the other, so another sweep follows it.  Within such a block a
+// cosine below 3e-15 is rounding (a dot product of 70 terms) and left alone, or its arbitrary angle
+// would undo the sweep's work again and again.  |C^T S C - 1| over 20 warm-started iterations of
+// CF4, cubane and neopentane: <= 2e-14, as the two-sided form had (3e-14); 7e-10 with the cosines
+// alone as the criterion.  Other molecules take 0-2 sweeps more over those iterations.
 // G: column-major, leading dimension LD = 16 Q + 8 (8 modulo 16 doubles: neighbouring groups on
 // different banks), rows and columns beyond N zero.  ev[i] <- eigenvalues, nv[i] <- 1 / |g_i|.
 template <int Q>
@@ -143,13 +149,18 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
       x += __shfl_xor_sync(0xffffffffu, x, 2);
       x += __shfl_xor_sync(0xffffffffu, x, 1);
       const double x2 = x * x, pq = app * aqq;
-      if (on && x2 > 1e-31 * pq) {
-        big = big || x2 > 1e-17 * pq;
+      const bool act = on && x2 > 1e-31 * pq;
+      double t = 0.0;
+      if (act) {
         // sym.schur2 (Golub & Van Loan): t = sign(d b) |b| / (|d| + sqrt(d^2 + b^2)), d = aqq - app, b = 2 x
         const float d = (float)(aqq - app), bb = (float)(2.0 * x);
         const float q2 = d * d + bb * bb;
         const float tf = copysignf(1.0f, d * bb) * __fdividef(fabsf(bb), fabsf(d) + q2 * rsqrtf(q2));
-        const double t = d == 0.0f ? (x > 0 ? 1.0 : -1.0) : (double)tf;
+        t = d == 0.0f ? (x > 0 ? 1.0 : -1.0) : (double)tf;
+      }
+      const bool wide = fabs(t) > 1e-6;
+      if (act && (!wide || x2 > 1e-29 * pq)) {
+        big = big || wide || x2 > 1e-17 * pq;
         // 1 / sqrt(1 + t^2): float seed (e = 1 - u y^2 near 1e-7), one third-order step (Householder)
         const double u = fma(t, t, 1.0), y = (double)rsqrtf((float)u), e = fma(-u * y, y, 1.0);
         const double c = fma(y * e, fma(0.375, e, 0.5), y), s = t * c;

@@ -273,3 +273,49 @@ def test_device_setup_sizes(cuda, atoms):
             assert (got == got.T).all()
         assert abs(eng.enuc[k].item() - hs.E_nuc) <= 1e-12 * hs.E_nuc
     eng.close()
+
+
+def _tetrahedral(centre, ligand, r):
+    d = r / 3 ** 0.5
+    return f"{centre} 0 0 0; " + "; ".join(f"{ligand} {d * x} {d * y} {d * z}"
+                                           for x, y, z in ((1, 1, 1), (-1, -1, 1), (-1, 1, -1), (1, -1, -1)))
+
+
+def _cubane():
+    c, h = 0.785, 0.785 + 1.09 / 3 ** 0.5
+    corners = [(x, y, z) for x in (1, -1) for y in (1, -1) for z in (1, -1)]
+    return "; ".join(f"{s} {a * x} {a * y} {a * z}" for s, a in (("C", c), ("H", h)) for x, y, z in corners)
+
+
+def _neopentane():
+    u = np.array([(1, 1, 1), (-1, -1, 1), (-1, 1, -1), (1, -1, -1)]) / 3 ** 0.5
+    atoms = [("C", np.zeros(3))] + [("C", 1.54 * a) for a in u]
+    atoms += [("H", 1.54 * a - 1.09 * b) for i, a in enumerate(u) for j, b in enumerate(u) if i != j]
+    return "; ".join(f"{s} {x:.15f} {y:.15f} {z:.15f}" for s, (x, y, z) in atoms)
+
+
+@pytest.mark.parametrize("atom", [
+    "H 0 0 0; H 0 0 0.74", _tetrahedral("C", "H", 1.09), _tetrahedral("C", "F", 1.32), _neopentane(), _cubane(),
+], ids=["h2", "ch4", "cf4", "neopentane", "cubane"])
+def test_eigh_density_coinciding_eigenvalues(cuda, atom):
+    """symmetric molecules, whose orbitals coincide in twos and threes: orbitals S-orthonormal and the
+    density and energies of LAPACK's eigenvectors, cold and then warm-started over 20 iterations.
+    Orthonormality: a product of N terms between columns orthogonal to 3e-15, N <= 48, through
+    L^T and back: 1e-12.  Density: rounding of A, 1e-14 of |A| ~ 50 Ha in float64, over the gap
+    between occupied and virtual orbitals, >= 0.2 Ha: 5e-12; energies: 2e-12."""
+    m = Mole(atom)
+    eng = RKSEngine([m], level=0, precision="fp64", guess="minao")
+    eng.prepare()
+    eng.initial()
+    N, nocc = m.nao, m.nelectron // 2
+    mat = lambda x: x[:N * N].cpu().numpy().reshape(N, N)
+    S, L = mat(eng.S), mat(eng.Linv)
+    for _ in range(20):
+        eng.step()
+        C, H = mat(eng.C), mat(eng.H)
+        w, v = np.linalg.eigh(L @ H @ L.T)
+        occ = L.T @ v[:, :nocc]
+        np.testing.assert_allclose(C.T @ S @ C, np.eye(N), atol=1e-12, rtol=0)
+        np.testing.assert_allclose(mat(eng.D), 2.0 * occ @ occ.T, atol=5e-12, rtol=0)
+        np.testing.assert_allclose(eng.mo_energy[:N].cpu().numpy(), w, atol=2e-12, rtol=0)
+    eng.close()
