@@ -18,7 +18,11 @@ import numpy as np
 from ._lib import lib, check, ptr
 
 NBKT = 5
-CANDIDATES = (1, 2, 4, 8, 16, 32, 64)
+# An item's length is the same in every batch (a molecule's V must not depend on its batch), and the
+# tensor cores' float32 sums over an item round towards zero, 1e-5 of V over 32 tiles.  Longer items
+# than 16 tiles are 2.2% faster on 4096 molecules (12.1 -> 11.8 ms) and cost a single molecule of 40
+# orbitals (73 tiles) 192 instead of 102 us per evaluation.
+CANDIDATES = (1, 2, 4, 8, 16)
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned.json")
 
 

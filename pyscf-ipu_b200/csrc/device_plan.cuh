@@ -22,8 +22,7 @@ struct B2GridDev {             // grid layout registered with b2_grid_set
   void *xq_items = nullptr;                         // per-bucket XC work items (molecule, tile)
   std::vector<long long> xq_off_h;                  // B2_NBKT + 1 bucket starts in xq_items
   int *xq_queue = nullptr;                          // B2_NBKT work-queue counters
-  int xq_tpc[B2_NBKT] = {0, 0, 0, 0, 0};            // most tiles per item per bucket (0: tpc_tc)
-  bool xq_exact = false;                            // tpc_tc was given: items of exactly that many tiles
+  int xq_tpc[B2_NBKT] = {0, 0, 0, 0, 0};            // tiles per item per bucket (0: tpc_tc)
 };
 
 struct B2SubsetDev {           // compacted work tables for a subset of the batch's molecules
@@ -107,8 +106,7 @@ int b2_launch_jk_s8(const B2PlanDev &P, int precision, const int *active, const 
                     const double *D, double *J, double *K, cudaStream_t st);
 int b2_zero_active(const B2PlanDev &P, const int *active, double *A, double *B, cudaStream_t st);
 // per-bucket work items of the tensor-core XC kernel for `mols` (device array in *items,
-// bucket starts in off), at most the configured tiles per item
-int b2_xc_run(const std::vector<long long> &nt, int slots, int least, int most);   // tiles per CTA (xc_tc.cu)
+// bucket starts in off), the configured tiles per item
 int b2_xq_build(const B2PlanDev &P, const std::vector<int> &mols, void **items, std::vector<long long> &off);
 // measurement and slot-refill helpers (eri.cu, blocks.cu)
 int b2_launch_eri_count(B2PlanDev &P, double *host_out);

@@ -226,6 +226,24 @@ __global__ void k_sym(const B2MolDev *__restrict__ mols, const int *__restrict__
   }
 }
 
+// Tiles per CTA for molecules of nt[...] tiles on `slots` resident CTAs: from `least` to `most`, and
+// the shortest run whose CTAs fit in as many rounds as runs of `most` need.  A CTA pays about one
+// tile's time for its tables, D and the V flush, so long runs are the better split while every slot
+// has several; with fewer tiles than that a run is a slot's share.  (Float64 sums only: the split moves
+// V by rounding.)
+static int b2_xc_run(const std::vector<long long> &nt, int slots, int least, int most) {
+  long long tiles = 0;
+  for (long long n : nt) tiles += n;
+  const long long cap = (long long)slots * most, fit = slots * std::max(1ll, (tiles + cap - 1) / cap);
+  int run = (int)std::max((long long)least, std::min((long long)most, (tiles + fit - 1) / fit));
+  for (; run < most; ++run) {                      // molecules' last runs may be short: count them
+    long long n = 0;
+    for (long long k : nt) n += (k + run - 1) / run;
+    if (n <= fit) break;
+  }
+  return run;
+}
+
 // slots > 0: runs that fill the rounds of that many resident CTAs (b2_xc_run).  The float64 kernel's
 // tiles are long (12 us at 62 orbitals, two CTAs per SM) and its CTAs few: 8500 tiles in runs of 7 took
 // 4.1 rounds, i.e. five, 443 us; 383 us as two rounds of runs of 15.
@@ -293,7 +311,6 @@ int b2_grid_setup(B2PlanDev &P, const long long *grid_off_host) {
 int b2_xc_set_tpc(B2PlanDev &P, int tpc) {
   if (!P.g.grid_off || tpc < 0) return B2_ERR_ARG;
   for (int b = 0; b < B2_NBKT; ++b) P.g.xq_tpc[b] = 0;    // one value for every bucket
-  P.g.xq_exact = tpc > 0;
   std::vector<long long> xtc;
   b2_xc_split(P.g.grid_off_h, P.h.nmol, 128, P.g.tpc_tc, xtc, tpc);
   long long *d = nullptr;

@@ -1078,47 +1078,21 @@ int b2_launch_xc_tq(const B2PlanDev &P, const int *active, const double *coords,
   return sym ? b2_sym_v(P, active, V, st) : B2_OK;
 }
 
-// Tiles per CTA (or per work item) for molecules of nt[...] tiles on `slots` resident CTAs: from
-// `least` to `most`, and the shortest run whose CTAs fit in as many rounds as runs of `most` need.  A
-// CTA pays about one tile's time for its tables, D and the V flush, so long runs are the better split
-// while every slot has several; with fewer tiles than that a run is a slot's share.
-int b2_xc_run(const std::vector<long long> &nt, int slots, int least, int most) {
-  long long tiles = 0;
-  for (long long n : nt) tiles += n;
-  const long long cap = (long long)slots * most, fit = slots * std::max(1ll, (tiles + cap - 1) / cap);
-  int run = (int)std::max((long long)least, std::min((long long)most, (tiles + fit - 1) / fit));
-  for (; run < most; ++run) {                      // molecules' last runs may be short: count them
-    long long n = 0;
-    for (long long k : nt) n += (k + run - 1) / run;
-    if (n <= fit) break;
-  }
-  return run;
-}
-
 // work items (molecule, first tile, tiles) of the per-bucket kernel for the molecules `mols`, grouped
-// by orbital bucket (off: B2_NBKT + 1 bucket starts).  The configured tiles per item (the tuned table's
-// per bucket, or `tpc`, which is taken as it is where the caller set it) come from thousands of
-// molecules; a batch that fills the GPU's slots less than once takes shorter items, down to half as
-// long: one molecule of 40 orbitals (73 tiles in runs of 32: three CTAs) 192 -> 102 us per
-// evaluation.  Not shorter, although single tiles took 22 us: the tensor cores' float32 sums round
-// towards zero, 1e-5 of V over 32 tiles, and a molecule's V should not depend on the batch it is in
-// by more than half of that.
+// by orbital bucket (off: B2_NBKT + 1 bucket starts), `tpc` or the bucket's configured tiles per item.
+// The length does not follow the batch: the tensor cores' float32 sums round towards zero, 1e-5 of V
+// over 32 tiles, so items cut to a batch's share of the GPU would make a molecule's V depend on the
+// batch it is in, and change it in the middle of an SCF where the active molecules are compacted.
 static void b2_xq_items(const B2PlanDev &P, const std::vector<int> &mols, int tpc, std::vector<B2XtItem> &items,
                         std::vector<long long> &off) {
   off.assign(B2_NBKT + 1, 0);
   std::vector<std::vector<B2XtItem>> per(B2_NBKT);
-  std::vector<long long> nt(mols.size());
-  for (size_t k = 0; k < mols.size(); ++k)
-    nt[k] = (P.g.grid_off_h[mols[k] + 1] - P.g.grid_off_h[mols[k]] + B2_XT_PT - 1) / B2_XT_PT;
-  int run[B2_NBKT];                                // the buckets' launches share the GPU: all tiles count
-  for (int b = 0; b < B2_NBKT; ++b) {
-    const int most = P.g.xq_tpc[b] > 0 ? P.g.xq_tpc[b] : tpc;
-    run[b] = P.g.xq_tpc[b] <= 0 && P.g.xq_exact ? tpc : b2_xc_run(nt, 148, (most + 1) / 2, most);
-  }
-  for (size_t k = 0; k < mols.size(); ++k) {
-    const int b = std::min(B2_NBKT - 1, (P.h.mols[mols[k]].nao - 1) / 16);
-    for (long long t = 0; t < nt[k]; t += run[b])
-      per[b].push_back(B2XtItem{mols[k], (int)t, (int)std::min((long long)run[b], nt[k] - t), 0});
+  for (int m : mols) {
+    const int b = std::min(B2_NBKT - 1, (P.h.mols[m].nao - 1) / 16);
+    const long long nt = (P.g.grid_off_h[m + 1] - P.g.grid_off_h[m] + B2_XT_PT - 1) / B2_XT_PT;
+    const int run = P.g.xq_tpc[b] > 0 ? P.g.xq_tpc[b] : tpc;
+    for (long long t = 0; t < nt; t += run)
+      per[b].push_back(B2XtItem{m, (int)t, (int)std::min((long long)run, nt - t), 0});
   }
   items.clear();
   for (int b = 0; b < B2_NBKT; ++b) {

@@ -387,3 +387,34 @@ def test_eri_batch_sizes(cuda, prec, tol):
         np.testing.assert_allclose(v[o:o + len(ref)], ref, atol=tol, rtol=0)
         assert np.isnan(v[o + len(ref):ends[k]]).all()
     P.close()
+
+
+@pytest.mark.parametrize("heavy", [1, 3, 5, 7, 9])
+def test_xc_float32_independent_of_batch(cuda, heavy):
+    """a molecule's float32 V and E_xc alone, in a batch that fills the GPU and with all but it
+    compacted away: its tiles are cut and summed the same way in all three, and only the order of
+    float64 additions of whole sums differs (N <= 5 per entry at 16 tiles or more: 1e-14 of max|V|,
+    1e-13 of E_xc over ~2e3 tiles' points)"""
+    rng = np.random.default_rng(70 + heavy)
+    one = Mole(random_molecule(rng, heavy))
+    got = []
+    for mols in ([one], [one] + [Mole(random_molecule(rng, int(k))) for k in rng.integers(1, 10, size=96)]):
+        eng = RKSEngine(mols, level=1, precision="mixed", guess="minao", tuned=False)
+        eng.device_setup()
+        P, counts = eng.plan, np.full(5, 32, np.int32)
+        check(lib().b2_plan_set_xc_bucket_tiles(P.h, ptr(counts)), "b2_plan_set_xc_bucket_tiles")
+        for subset in (0, 1):
+            act = None
+            if subset:
+                idx = np.zeros(1, np.int32)
+                check(lib().b2_plan_set_subset(P.h, ptr(idx), 1), "b2_plan_set_subset")
+                act = torch.zeros(len(mols), dtype=torch.int32, device=cuda)
+                act[0] = 1
+            eng.xc(eng.D0, active=act)
+            torch.cuda.synchronize()
+            got.append((eng.exc[0].item(), P.unpack(eng.Vxc.cpu().numpy(), 0).copy()))
+        check(lib().b2_plan_set_subset(P.h, None, 0), "b2_plan_set_subset")
+        eng.close()
+    for e, v in got[1:]:
+        assert abs(e - got[0][0]) <= 1e-13 * abs(e)
+        np.testing.assert_allclose(v, got[0][1], atol=1e-14 * np.abs(v).max(), rtol=0)
