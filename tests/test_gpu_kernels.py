@@ -418,3 +418,32 @@ def test_xc_float32_independent_of_batch(cuda, heavy):
     for e, v in got[1:]:
         assert abs(e - got[0][0]) <= 1e-13 * abs(e)
         np.testing.assert_allclose(v, got[0][1], atol=1e-14 * np.abs(v).max(), rtol=0)
+
+
+@pytest.fixture(scope="module")
+def both_precisions(cuda):
+    """float32 and float64 engines of 256 molecules, and the float64 path's converged densities"""
+    from b200dft.molgen import config3_batch
+    mols = [Mole(s) for s in config3_batch(256, seed=7)]
+    e64, e32 = (RKSEngine(mols, level=0, precision=p, guess="minao") for p in ("fp64", "mixed"))
+    e64.prepare()
+    assert bool(e64.run_converged()["converged"].all())
+    e32.prepare()
+    yield e64, e32, e64.D.clone()
+    e64.close()
+    e32.close()
+
+
+def test_eri_float32_error(both_precisions):
+    """float32 integrals no further from float64 than kernels that sum one l class at a time are,
+    over the same 256 molecules: 7.1e-7 at most, 9.0e-8 in the 2-norm (measured on those kernels)"""
+    e64, e32, _ = both_precisions
+    P, err, norm = e64.plan, 0.0, [0.0, 0.0]
+    for m in range(P.nmol):
+        o = int(P.eri_off[m])
+        ref = e64.eri[o:o + oeri.n_s8(int(P.nao[m]))]
+        d = e32.eri[o:o + len(ref)].double() - ref
+        err = max(err, d.abs().max().item())
+        norm[0] += d.pow(2).sum().item()
+        norm[1] += ref.pow(2).sum().item()
+    assert err <= 7.1e-7 and norm[0] ** 0.5 <= 9.0e-8 * norm[1] ** 0.5
