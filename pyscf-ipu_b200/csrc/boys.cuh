@@ -14,7 +14,7 @@
 #define B2_BOYS_INV_DT 8.0
 #define B2_BOYS_TMAX 40.0
 #define B2_BOYS_NT 322          // T_k = k*DT, k = 0..321 (covers TMAX + DT/2)
-#define B2_BOYS_NM 14           // m = 0..13 (L <= 4 plus 9 Taylor terms)
+#define B2_BOYS_NM 14           // m = 0..13 (L <= 5 plus 9 Taylor terms)
 
 // host: fill table[k*NM + m]
 static void b2_boys_fill_table(double *table) {
@@ -62,6 +62,19 @@ template <> __device__ __forceinline__ void b2_inv_rsqrt<float>(float t, float &
 template <typename T> struct B2BoysErfF0 { static constexpr bool value = false; };
 template <> struct B2BoysErfF0<float> { static constexpr bool value = true; };
 
+// x / (2 m + 1) of the downward recursion.  The float32 reciprocals of 3, 5, 7 and 9 are all too
+// large, by up to 4e-8 of their size; the error adds up with one sign over every integral (E_J of a
+// molecule was 7.4e-6 Ha too large on average, 0.9e-6 with it taken off), so float32 multiplies by
+// the reciprocal and by what its rounding left.
+template <typename T> struct B2BoysOddLow { static constexpr bool value = false; };
+template <> struct B2BoysOddLow<float> { static constexpr bool value = true; };
+template <typename T> B2_HD T b2_boys_odd(T x, int m) {
+  if (m == 0) return x;
+  const double r = 1.0 / (2 * m + 1);
+  if constexpr (B2BoysOddLow<T>::value) return x * (T)(float)r + x * (T)(r - (double)(float)r);
+  return x * (T)r;
+}
+
 // F[0..L] at T; `table` is the table in double (float64 kernels) or float (float32 kernels).
 template <typename T, int L, typename TT>
 B2_HD void b2_boys(T t, const TT *__restrict__ table, T *F) {
@@ -89,7 +102,7 @@ B2_HD void b2_boys(T t, const TT *__restrict__ table, T *F) {
       T et = b2_exp_neg<T>(t);
       T t2 = t + t;
 #pragma unroll
-      for (int m = L - 1; m >= 0; --m) F[m] = (t2 * F[m + 1] + et) * (T)(1.0 / (2 * m + 1));
+      for (int m = L - 1; m >= 0; --m) F[m] = b2_boys_odd<T>(t2 * F[m + 1] + et, m);
     }
   } else {
     T inv, rt;                                        // 1 / T, 1 / sqrt(T)

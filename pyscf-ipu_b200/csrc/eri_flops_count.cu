@@ -64,6 +64,7 @@ inline CF erf(CF a) { if (!a.k) ++g_special; CF c = a; c.v = std::erf(a.v); retu
 // the float32 kernels' Taylor length of the Boys table branch, and their error-function F_0
 template <> struct B2BoysTerms<CF> { static constexpr int n = B2BoysTerms<float>::n; };
 template <> struct B2BoysErfF0<CF> { static constexpr bool value = B2BoysErfF0<float>::value; };
+template <> struct B2BoysOddLow<CF> { static constexpr bool value = B2BoysOddLow<float>::value; };
 
 template <int TB, int TK>
 static void count(long long &fl, long long &sp, long long &kf) {
