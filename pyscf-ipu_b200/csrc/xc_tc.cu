@@ -833,7 +833,10 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, cons
       b2_fence_before();
       if (__syncthreads_or(fail)) { sAbort = 1; break; }            // [1]
       x_pending = true;
-      // ---- X = AO0 D = (A_h + A_l)(D_1 + D_2): three TF32 products per K step
+      // ---- X = AO0 D = (A_h + A_l)(D_1 + D_2): three TF32 products per K step, the two small ones of
+      // every step first.  The accumulator rounds towards zero at each product, by its size at that
+      // moment, which makes rho too small: mean error of E_xc over 256 molecules 9.9e-6 Ha with the
+      // three products side by side, 5.1e-6 so (2048 molecules: 5.92 -> 6.04 ms).
       if (tid == 0) {
         b2_fence_after();
         const uint32_t aH = b2_su32(sAh), aL = b2_su32(sAl), dH = b2_su32(sDh), dL = b2_su32(sDl);
@@ -846,6 +849,11 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, cons
           const uint64_t bl = b2_sdesc(dL + s * 2 * LBO_D, LBO_D, SBO_D);
           b2_mma_tf32(tbase + colX, al, bh, id1, s > 0 ? 1u : 0u);
           b2_mma_tf32(tbase + colX, ah, bl, id1, 1u);
+        }
+#pragma unroll 1
+        for (int s = 0; s < NB / 8; ++s) {
+          const uint64_t ah = b2_sdesc(aH + s * 2 * LBO_A, LBO_A, SBO_A);
+          const uint64_t bh = b2_sdesc(dH + s * 2 * LBO_D, LBO_D, SBO_D);
           b2_mma_tf32(tbase + colX, ah, bh, id1, 1u);
         }
         b2_mma_commit(mbar1);

@@ -465,3 +465,13 @@ def test_jk_energy_float32_error(both_precisions):
     dj = 0.5 * (_energies(e32, e32.J, D) - _energies(e64, e64.J, D))
     dk = -0.25 * 0.2 * (_energies(e32, e32.K, D) - _energies(e64, e64.K, D))
     assert np.abs(dj).mean() <= 5.9e-6 and np.abs(dk).mean() <= 2.0e-7
+
+
+def test_xc_energy_float32_error(both_precisions):
+    """E_xc of the tensor-core path at a float64 density: the mean error, which has one sign, no
+    larger than with the tile's columns in the order of the orbitals (8.7e-6 Ha, measured on the
+    same molecules)"""
+    e64, e32, D = both_precisions
+    for e in (e64, e32):
+        e.xc(D=D)
+    assert (e32.exc - e64.exc).abs().mean().item() <= 8.7e-6
