@@ -319,3 +319,19 @@ def test_eigh_density_coinciding_eigenvalues(cuda, atom):
         np.testing.assert_allclose(mat(eng.D), 2.0 * occ @ occ.T, atol=5e-12, rtol=0)
         np.testing.assert_allclose(eng.mo_energy[:N].cpu().numpy(), w, atol=2e-12, rtol=0)
     eng.close()
+
+
+def test_diis_single_entry(cuda):
+    """the first iteration's DIIS matrix [[0, 1], [1, e.e]] has the coefficient 1, so the extrapolated
+    Hamiltonian is the Hamiltonian itself: two terms of its pseudo-inverse, each at most 1 and
+    rounded four times, 8 eps of every entry"""
+    rng = np.random.default_rng(21)
+    mols = [Mole(random_molecule(rng, int(k))) for k in rng.integers(1, 10, size=48)]
+    eng = RKSEngine(mols, level=0, precision="fp64", guess="minao")
+    eng.prepare()
+    eng.initial()
+    eng.fock_diis()
+    want = eng.Hcore + eng.diffJK + eng.Vxc          # in the kernel's order
+    assert float(eng.diis_err.min()) > 1e-3
+    np.testing.assert_allclose(eng.H.cpu().numpy(), want.cpu().numpy(), rtol=8 * 2.3e-16, atol=0)
+    eng.close()
