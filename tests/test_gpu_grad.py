@@ -124,3 +124,67 @@ def test_gradient_slices_over_sizes(heavy, odd):
     assert hc.b2hc_grad_2e_super(*a, ctypes.c_double(HYB), _p(ref2, ctypes.c_double), _p(n, ctypes.c_int)) == 0
     for g, ref in zip(got, (ref1, ref2)):
         np.testing.assert_allclose(g, ref, atol=1e-10 * max(1.0, np.abs(ref).max()), rtol=0)
+
+
+def test_gradient_xc_odd_shells():
+    """the exchange-correlation part with shells off the STO-3G pattern against the host math, same
+    tolerance as for the regular ones"""
+    import torch
+    from test_gpu_kernels import _odd_mols
+    from test_hostcheck import _gs_args, _hc, _p
+    from b200dft.engine import RKSEngine
+    from b200dft._lib import check, lib, ptr, stream_handle
+    mols = _odd_mols()
+    eng = RKSEngine(mols, level=0, precision="fp64")
+    eng.device_setup()
+    P, rng, hc = eng.plan, np.random.default_rng(25), _hc()
+    Ds = []
+    for m in mols:
+        C = rng.normal(size=(m.nao, m.nao)) * 0.1 + np.diag(rng.uniform(0.5, 1.0, m.nao))
+        Ds.append(2.0 * C[:, :m.nelectron // 2] @ C[:, :m.nelectron // 2].T)
+    d = torch.from_numpy(P.pack(Ds)).cuda()
+    w, g = torch.zeros_like(d), torch.zeros(sum(m.natm for m in mols), 3, dtype=torch.float64, device="cuda")
+    check(lib().b2_grad(P.h, 4, HYB, None, None, ptr(eng.coords), ptr(eng.weights), ptr(d), ptr(w), ptr(g),
+                        stream_handle()), "b2_grad")
+    got, a0, xyz, wt = g.cpu().numpy(), 0, eng.coords.cpu().numpy().reshape(-1, 3), eng.weights.cpu().numpy()
+    for k, (m, D) in enumerate(zip(mols, Ds)):
+        gp = slice(P.grid_off[k], P.grid_off[k + 1])
+        ref, (x, q, D) = np.zeros((m.natm, 3)), (np.ascontiguousarray(a) for a in (xyz[gp], wt[gp], D))
+        keep, a = _gs_args(m, D)
+        assert hc.b2hc_grad_xc(*a, ctypes.c_longlong(len(q)), _p(x, ctypes.c_double), _p(q, ctypes.c_double),
+                               _p(ref, ctypes.c_double)) == 0
+        np.testing.assert_allclose(got[a0:a0 + m.natm], ref, atol=1e-9 * max(1.0, np.abs(ref).max()), rtol=0)
+        a0 += m.natm
+    eng.close()
+
+
+def test_gradient_many_tasks():
+    """two- and one-electron parts of a batch in which every warp takes several slices, neighbours of
+    other sizes: each molecule as alone.  Sums of the same float64 terms in another order (atomics)."""
+    import torch
+    from test_gpu_kernels import _big_batch
+    from b200dft.engine import Plan
+    from b200dft._lib import check, lib, ptr, stream_handle
+    kinds, order = _big_batch()
+    rng = np.random.default_rng(31)
+    mats = [[a + a.T for a in rng.normal(size=(2, m.nao, m.nao)) * 0.3] for m in kinds]
+
+    def parts(which):
+        plan = Plan([kinds[k] for k in which])
+        d, w = (torch.from_numpy(plan.pack([mats[k][i] for k in which])).cuda() for i in (0, 1))
+        g = torch.zeros(2, sum(kinds[k].natm for k in which), 3, dtype=torch.float64, device="cuda")
+        for i, part in enumerate((1, 2)):
+            check(lib().b2_grad(plan.h, part, HYB, None, None, None, None, ptr(d), ptr(w), ptr(g[i]),
+                                stream_handle()), "b2_grad")
+        out = g.cpu().numpy()
+        plan.close()
+        return out
+
+    alone = [parts([k]) for k in range(len(kinds))]
+    got, a0 = parts(order), 0
+    for k in order:
+        n = kinds[k].natm
+        for i in (0, 1):
+            np.testing.assert_allclose(got[i, a0:a0 + n], alone[k][i], rtol=0,
+                                       atol=1e-11 * max(1.0, np.abs(alone[k][i]).max()))
+        a0 += n

@@ -475,3 +475,130 @@ def test_xc_energy_float32_error(both_precisions):
     for e in (e64, e32):
         e.xc(D=D)
     assert (e32.exc - e64.exc).abs().mean().item() <= 8.7e-6
+
+
+def _odd_mols():
+    """shells off the STO-3G pattern (a p shell without its s, s shells of one and two primitives)
+    in every orbital bucket: the float32 kernel's columns then hold p functions of their own"""
+    from test_hostcheck import odd_shells
+    rng = np.random.default_rng(23)
+    return [odd_shells(Mole("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7572 -0.4692"))] + \
+        [odd_shells(Mole(random_molecule(rng, k))) for k in (2, 4, 6, 8, 9)]
+
+
+@pytest.mark.parametrize("prec, etol, vtol", [("fp64", 1e-11, 1e-11), ("mixed", 2e-6, 2e-5)])
+def test_xc_odd_shells(cuda, prec, etol, vtol):
+    """XC with shells off the STO-3G pattern against the oracle (tolerances as for the regular ones)"""
+    mols = _odd_mols()
+    eng = RKSEngine(mols, level=0, precision=prec)
+    eng.device_setup()
+    P, w = eng.plan, eng.weights.cpu().numpy()
+    xyz = eng.coords.cpu().numpy().reshape(-1, 3)
+    assert len({(n - 1) // 16 for n in P.nao}) >= 4
+    rng = np.random.default_rng(24)
+    Ds = []
+    for m in mols:
+        C = rng.normal(size=(m.nao, m.nao)) * 0.1 + np.diag(rng.uniform(0.5, 1.0, m.nao))
+        Ds.append(2.0 * C[:, :m.nelectron // 2] @ C[:, :m.nelectron // 2].T)
+    eng.xc(torch.from_numpy(P.pack(Ds)).to(cuda))
+    V, E = eng.Vxc.cpu().numpy(), eng.exc.cpu().numpy()
+    for k, m in enumerate(mols):
+        g = slice(P.grid_off[k], P.grid_off[k + 1])
+        Er, Vr, _ = rks.exchange_correlation(Ds[k], rks.ao_values(m, xyz[g]), w[g])
+        np.testing.assert_allclose(P.unpack(V, k), Vr, atol=vtol * max(1.0, np.abs(Vr).max()), rtol=0)
+        assert abs(E[k] - Er) <= etol * abs(Er)
+    eng.close()
+
+
+def _three_primitives(m):
+    """the molecule with its shorter contractions filled up with primitives of coefficient zero (the
+    host formulas take three)"""
+    t = Mole.__new__(Mole)
+    t.__dict__.update(m.__dict__)
+    t._bas, env = m._bas.copy(), m._env
+    for b in t._bas:
+        ex, c = env[b[5]:b[5] + b[2]], env[b[6]:b[6] + b[2]]
+        b[5], b[6] = len(env), len(env) + 3
+        env = np.concatenate([env, ex, np.ones(3 - b[2]), c, np.zeros(3 - b[2])])
+        b[2] = 3
+    t._env = env
+    return t
+
+
+def test_int1e_odd_shells(cuda):
+    """one-electron matrices with shells off the STO-3G pattern against the host formulas"""
+    from b200dft.int1e import int1e
+    mols = _odd_mols()
+    eng = RKSEngine(mols, level=0, precision="fp64")
+    eng.device_setup()
+    for k, m in enumerate(mols):
+        for name, ref in zip("STV", int1e(_three_primitives(m))):
+            got = eng.plan.unpack(getattr(eng, name).cpu().numpy(), k)
+            np.testing.assert_allclose(got, ref, atol=1e-11 * max(1.0, np.abs(ref).max()), rtol=0, err_msg=name)
+    eng.close()
+
+
+def _super_shells(m):
+    """(s-only, sp) super shells of a molecule with STO-3G shells or those of odd_shells"""
+    e = [tuple(m._env[b[5]:b[5] + b[2]]) + (b[0], b[2]) for b in m._bas]
+    s = {x for x, b in zip(e, m._bas) if b[1] == 0}
+    p = [x for x, b in zip(e, m._bas) if b[1] == 1]
+    merged = sum(x in s for x in p)
+    return int((m._bas[:, 1] == 0).sum()) - merged, len(p)
+
+
+def _big_batch():
+    """a batch in which every resident warp of the integral and gradient kernels takes several tasks
+    (148 x 8 CTAs of 4 warps) and one of the one-electron kernel eight pairs (148 x 4 x 8 warps), its
+    neighbours of other sizes"""
+    from test_hostcheck import odd_shells
+    rng = np.random.default_rng(29)
+    kinds = [Mole("H 0 0 0; H 0 0 0.74"), Mole(random_molecule(rng, 9)), odd_shells(Mole(random_molecule(rng, 4))),
+             Mole(random_molecule(rng, 9)), Mole("O 0 0 0.1173; H 0 0.7572 -0.4692; H 0 -0.7572 -0.4692"),
+             odd_shells(Mole(random_molecule(rng, 9)))]
+    order = [k for _ in range(20) for k in range(len(kinds))]
+    pairs, tasks = 0, np.zeros(6, int)
+    for k in order:
+        ns, np_ = _super_shells(kinds[k])
+        n = [ns * (ns + 1) // 2, ns * np_, np_ * (np_ + 1) // 2]
+        pairs += sum(n)
+        for c, (bra, ket) in enumerate(((n[0], n[0]), (n[0], n[1]), (n[1], n[1]), (n[0], n[2]), (n[1] + n[2], n[2]),
+                                        (3 * n[2], n[2]))):
+            tasks[c] += bra * -(-ket // 32)
+    assert pairs >= 8 * 148 * 4 * 8 and (tasks > 2 * 148 * 8 * 4).all()
+    return kinds, order
+
+
+@pytest.mark.parametrize("prec", [64, 32])
+def test_eri_many_tasks(cuda, prec):
+    """integrals of a batch in which every warp takes several tasks: the same bits as each molecule
+    alone, where no warp takes a second one in the classes with p bras"""
+    kinds, order = _big_batch()
+    dt = torch.float64 if prec == 64 else torch.float32
+    alone = [torch.from_numpy(_eri([m], prec, cuda)[1]).to(cuda) for m in kinds]
+    P = Plan([kinds[k] for k in order])
+    out = torch.full((P.n_eri,), float("nan"), dtype=dt, device=cuda)
+    check(lib().b2_eri_s8(P.h, prec, ptr(out), stream_handle()), "b2_eri_s8")
+    for i, k in enumerate(order):
+        o = int(P.eri_off[i])
+        assert torch.equal(out[o:o + len(alone[k])].double(), alone[k])
+    P.close()
+
+
+def test_int1e_many_pairs(cuda):
+    """one-electron matrices of a batch with eight pairs per warp, chunks crossing molecules: the same
+    bits as each molecule alone"""
+    kinds, order = _big_batch()
+
+    def matrices(mols):
+        P = Plan(mols)
+        a = [torch.full((P.n_mat,), float("nan"), dtype=torch.float64, device=cuda) for _ in range(3)]
+        check(lib().b2_int1e(P.h, *[ptr(x) for x in a], stream_handle()), "b2_int1e")
+        out = [[P.unpack(x.cpu().numpy(), k).copy() for x in a] for k in range(len(mols))]
+        P.close()
+        return out
+
+    alone = [matrices([m])[0] for m in kinds]
+    for got, k in zip(matrices([kinds[k] for k in order]), order):
+        for a, b in zip(got, alone[k]):
+            assert (a == b).all()
