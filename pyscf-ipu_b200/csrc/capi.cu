@@ -579,11 +579,7 @@ int b2_grad(void *plan, int parts, double hyb, const double *C, const double *mo
   if (!plan) return B2_ERR_ARG;
   B2PlanDev *P = (B2PlanDev *)plan;
   if (P->h.max_natm > B2_MAXNAO) return B2_ERR_SIZE;
-  try {                                            // its host tables allocate
-    return b2_launch_grad(*P, parts, hyb, C, mo_energy, coords, weights, D, W, grad, (cudaStream_t)stream);
-  } catch (const std::bad_alloc &) {
-    return B2_ERR_SIZE;
-  }
+  return b2_launch_grad(*P, parts, hyb, C, mo_energy, coords, weights, D, W, grad, (cudaStream_t)stream);
 }
 
 }  // extern "C"

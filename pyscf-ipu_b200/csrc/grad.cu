@@ -13,12 +13,10 @@
 //               points of one molecule, products with D by float64 MMA;
 //   k_grad_nuc  nuclear repulsion (grad_nuc, nanoDFT.py:428-438).
 //
-// The per-term math is grad_sp.cuh and grad_math.cuh, the same code the host-check build tests
-// against the finite-difference oracle.
+// The two- and one-electron math is grad_sp.cuh, which the host-check build runs too and compares with
+// the Obara-Saika forms of grad_math.cuh; those are compared with the finite-difference oracle.
 #include <algorithm>
-#include <vector>
 #include "device_plan.cuh"
-#include "grad_math.cuh"
 #include "grad_sp.cuh"
 #include "xc_f64.cuh"
 

@@ -1,4 +1,5 @@
-// Two-electron part of the RKS nuclear gradient for s / p shells (host and device code).
+// Nuclear gradient of the RKS energy for s / p shells, shell quartet by shell quartet: what the host-check
+// build compares the kernels' slices (grad_sp.cuh) and tiles with.  No kernel runs it.
 //
 // The reference's gradient (nanoDFT.py:403-426) contracts int2e_ip1 = (d/dA_x i j|k l) with the
 // density: vj = -sum (d_i j|k l) D_lk, vk = -sum (d_i j|k l) D_jk, de_A += 2 <vj - hyb/2 vk,

@@ -16,7 +16,6 @@
 //   g = -2 mu (A-B) E - (b/zeta) dE/d(P-A) + (a/zeta) dE/d(P-B).
 #pragma once
 #include "boys.cuh"
-#include "grad_math.cuh"
 #include "super.cuh"
 
 // component d of the gradient of W at the derivative index (i, j, k)

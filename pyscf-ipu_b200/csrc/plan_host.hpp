@@ -37,8 +37,8 @@ struct B2PlanHost {
   std::vector<long long> row_off;         // nmol + 1
   std::vector<B2Shell> shells;
   std::vector<B2PairInfo> pinfo;
-  std::vector<B2PairPrim<double>> pp64;   // filled by b2_plan_fill_pairs (host builds only;
-  std::vector<B2PairPrim<float>> pp32;    // the device plan computes them on the GPU)
+  std::vector<B2PairPrim<double>> pp64;   // filled by b2_plan_fill_pairs (host builds only)
+  std::vector<B2PairPrim<float>> pp32;
   std::vector<int> ao2sh;                 // per AO: local shell index
   std::vector<int> cls_list;              // per molecule nsp entries (offset sp_off)
   std::vector<int> cls_cnt;               // per molecule 4*nsp (offset 4*sp_off)
@@ -102,7 +102,7 @@ B2_HD void b2_pair_prims_packed(const B2Shell &a, const B2Shell &b, B2PairPrim<d
 
 // returns B2_OK or an error code
 // pair_tables: also fill pinfo / cls_list / cls_cnt here (the host test build); the device plan
-// builds them with k_plan_pairs and keeps only per-molecule and per-shell work on the host.
+// keeps per-molecule and per-shell work on the host and its pairs are super shells' (super.cuh).
 static int b2_plan_build(B2PlanHost &P, int nmol, const int *natm, const int *nbas, const int *atm,
                          const int *bas, const double *env, const long long *env_off,
                          bool pair_tables = true) {
@@ -229,7 +229,7 @@ static int b2_plan_build(B2PlanHost &P, int nmol, const int *natm, const int *nb
   return B2_OK;
 }
 
-// host copy of the primitive-pair tables (the device plan builds them with k_pair_prims)
+// primitive-pair tables of the shell pairs (host test build)
 static void b2_plan_fill_pairs(B2PlanHost &P) {
   P.pp64.assign((size_t)P.n_sp * B2_MAXPP, B2PairPrim<double>());
   P.pp32.assign((size_t)P.n_sp * B2_MAXPP, B2PairPrim<float>());

@@ -352,8 +352,7 @@ int b2_launch_int1e(const B2PlanDev &P, double *S, double *T, double *V, cudaStr
 int b2_launch_grid_build(B2PlanDev &P, int nz, const double *tmpl_host, const long long *tmpl_off_host,
                          double *coords, double *weights, cudaStream_t st) {
   if (!P.g.grid_off || nz < 10) return B2_ERR_ARG;
-  for (int m = 0; m < P.h.nmol; ++m)
-    if (P.h.mols[m].natm > 32) return B2_ERR_SIZE;      // per-point distance table in registers
+  if (P.h.max_natm > B2_GRID_MAXATM) return B2_ERR_SIZE;
   // per-atom point offsets from the templates; must agree with the registered grid layout
   std::vector<long long> apo(P.h.n_atm + 1, 0);
   long long tot = 0;
@@ -382,7 +381,6 @@ int b2_launch_grid_build(B2PlanDev &P, int nz, const double *tmpl_host, const lo
   for (int i = 0; i < 10; ++i) brs[i] = br[i] > 0 ? sqrt(br[i]) : 1.0;
   B2_CUDA_TRY(cudaMemcpyToSymbol(c_bragg_sqrt, brs, sizeof(brs)));
   if (P.g.n_points > 0) {
-    if (P.h.max_natm > B2_GRID_MAXATM) return B2_ERR_SIZE;
     auto smem = [](int na) { return sizeof(double) * (size_t)(2 * na * na + 128 * na); };
     B2_CUDA_TRY(cudaFuncSetAttribute(k_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem(P.h.max_natm)));
     bool small = false, large = false;

@@ -368,6 +368,7 @@ static int b2_xf_bucket(const B2PlanDev &P, bool one, const int *active, const d
   return B2_OK;
 }
 
+// the shell limit is k_xc_direct's table; the float64 kernel keeps none, but accepts the same molecules
 static int b2_xcd_zero(const B2PlanDev &P, const int *active, double *V, double *exc, cudaStream_t st) {
   if (P.h.max_nbas > B2_XD_MAXSH) return B2_ERR_SIZE;
   return b2_zero_xc(P, active, V, exc, st);

@@ -1052,6 +1052,7 @@ int b2_launch_xc_tq(const B2PlanDev &P, const int *active, const double *coords,
   const bool sub = P.sub.n > 0;
   const B2XtItem *items = (const B2XtItem *)(sub ? P.sub.xq_items : P.g.xq_items);
   const std::vector<long long> &off = sub ? P.sub.xq_off_h : P.g.xq_off_h;
+  // the shell limit is k_xc_tc's table; this kernel keeps none, but accepts the same molecules
   if (P.h.max_nbas > B2_XT_MAXSH || P.h.max_nao > 80) return B2_ERR_SIZE;
   if (!items || off.size() != B2_NBKT + 1 || !P.g.xq_queue) return B2_ERR_ARG;
   int rc = b2_zero_xc(P, active, V, exc, st);
