@@ -6,9 +6,9 @@ Knob: grid tiles (128 points) per work item of the per-bucket tensor-core XC ker
 separately for each orbital bucket (nao <= 16, 32, 48, 64, more).  Few tiles per item balance
 the work queue; many amortise the per-item load of D and the flush of V.  ``tune_xc_tiles``
 times ``b2_xc_direct`` on the molecules of one bucket at a time (the others inactive) for every
-candidate, with CUDA events, and keeps the fastest.  The choices are recorded per device in
-``tuned.json`` beside this file (``save``), and ``RKSEngine`` applies the recorded table of its
-device to every new plan (``apply``).
+candidate, with CUDA events, and keeps the shortest that is nearly the fastest (``SLACK``).  The
+choices are recorded per device in ``tuned.json`` beside this file (``save``), and ``RKSEngine``
+applies the recorded table of its device to every new plan (``apply``).
 """
 import json
 import os
@@ -18,11 +18,13 @@ import numpy as np
 from ._lib import lib, check, ptr
 
 NBKT = 5
-# An item's length is the same in every batch (a molecule's V must not depend on its batch), and the
-# tensor cores' float32 sums over an item round towards zero, 1e-5 of V over 32 tiles.  Longer items
-# than 16 tiles are 2.2% faster on 4096 molecules (12.1 -> 11.8 ms) and cost a single molecule of 40
-# orbitals (73 tiles) 192 instead of 102 us per evaluation.
-CANDIDATES = (1, 2, 4, 8, 16)
+CANDIDATES = (1, 2, 4, 8, 16, 32, 64)
+# An item's length is the same in every batch (a molecule's V must not depend on its batch).  Short
+# items are worth something beyond the timed batch: the tensor cores' float32 sums over an item round
+# towards zero, 1e-5 of V over 32 tiles, and a single molecule of 40 orbitals (73 tiles) takes 102 us
+# in items of 16 and 192 us in items of 32.  So the choice is the shortest length within SLACK of the
+# fastest: on 4096 molecules 12.3 ms against 11.8 ms with the fastest lengths (64, 32, 32, 32, 16).
+SLACK = 1.1
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned.json")
 
 
@@ -31,9 +33,9 @@ def bucket_of(nao):
     return min(NBKT - 1, (int(nao) - 1) // 16)
 
 
-def pick(times):
-    """times: {bucket: {candidate: ms}} -> {bucket: fastest candidate} (ties: fewer tiles)"""
-    return {b: min(sorted(t), key=lambda c: (t[c], c)) for b, t in times.items() if t}
+def pick(times, slack=1.0):
+    """times: {bucket: {candidate: ms}} -> {bucket: fewest tiles within ``slack`` of the fastest}"""
+    return {b: min(c for c in t if t[c] <= slack * min(t.values())) for b, t in times.items() if t}
 
 
 def tiles_array(choice):
@@ -74,7 +76,7 @@ def tune_xc_tiles(eng, candidates=CANDIDATES, reps=3):
             torch.cuda.synchronize()
             ms = [ev[2 * r].elapsed_time(ev[2 * r + 1]) for r in range(reps)]
             times[b][c] = float(np.median(ms))
-    choice = pick(times)
+    choice = pick(times, SLACK)
     set_bucket_tiles(P, choice)
     return choice, times
 

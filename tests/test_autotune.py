@@ -21,3 +21,12 @@ def test_table_round_trip(tmp_path):
     d = json.load(open(p))
     assert d["NVIDIA B200"]["xc_tiles"] == {"2": 8}
     assert autotune.load(p)["NVIDIA B200"]["xc_ms"]["2"]["8"] == 1.0
+
+
+def test_pick_shortest_within_slack_and_recorded_table():
+    assert autotune.pick({0: {1: 2.0, 4: 1.09, 16: 1.0}, 2: {8: 1.2, 16: 1.0}}, 1.1) == {0: 4, 2: 16}
+    d = autotune.load()["NVIDIA B200"]
+    times = {int(b): {int(c): v for c, v in t.items()} for b, t in d["xc_ms"].items()}
+    assert autotune.pick(times, autotune.SLACK) == {int(b): c for b, c in d["xc_tiles"].items()}
+    # sums in tensor memory lose 3e-7 of V per tile: at most 5e-6 of it
+    assert set(times) == set(range(autotune.NBKT)) and max(d["xc_tiles"].values()) <= 16
