@@ -197,7 +197,7 @@ __device__ int b2_jacobi1(double *G, int N, double *nrm, double *ev, double *nv,
 // G_k A_kl G_l^T to the 2 x 2 blocks.  What bounds it is the chain of rounds.  k_fock_diis per call at
 // 7 orbitals: 95 us in the serial order (45 dependent rotations per sweep), 61 us in rounds, 48 us with
 // the tangent in float32, 41 us over the leading rows alone.  The float32 tangent is brought to float64
-// by Newton's steps, which need no further division (4.7 us per call): with it alone the iteration
+// by Newton's steps with a float32 slope (2 us per call): with it alone the iteration
 // stops with 1e-14 of a coupling left, and the first coefficient came out 4e-15 to 9e-15 off where the
 // serial order had 3e-16.
 // Couplings below float32's range are far below the stopping norm (the border of B holds ones).
@@ -234,10 +234,12 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot, int *prs
         const double apq = A[p * n + q], app = A[p * n + p], aqq = A[q * n + q];
         if (fabs(apq) > 1e-36 && apq * apq > 1e-36 * fabs(app * aqq)) {
           // tau = (aqq - app) / (2 apq), t = sign(tau) / (|tau| + sqrt(1 + tau^2)) (sym.schur2)
-          const float tau = fminf(fmaxf((float)(aqq - app) / (float)(2.0 * apq), -1e18f), 1e18f);
-          double t = (double)(copysignf(1.0f, tau) / (fabsf(tau) + sqrtf(1.0f + tau * tau)));
-          // two Newton steps on apq t^2 + (aqq - app) t - apq = 0 (slope from the float32 tangent)
-          const double d = aqq - app, ri = (double)(1.0f / (float)(2.0 * apq * t + d));
+          const double d = aqq - app;
+          const float df = (float)d, bf = (float)(2.0 * apq), tau = fminf(fmaxf(df / bf, -1e18f), 1e18f);
+          const float tf = copysignf(1.0f, tau) / (fabsf(tau) + sqrtf(1.0f + tau * tau));
+          // two Newton steps on apq t^2 + d t - apq = 0 (slope from the float32 tangent)
+          const double ri = (double)__fdividef(1.0f, fmaf(bf, tf, df));
+          double t = (double)tf;
 #pragma unroll
           for (int k = 0; k < 2; ++k) t = fma(-fma(apq * t, t, fma(d, t, -apq)), ri, t);
           c = rsqrt(1.0 + t * t);
