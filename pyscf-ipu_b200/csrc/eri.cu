@@ -167,7 +167,7 @@ k_eri_ss(const long long *__restrict__ toff, int nmol, const B2gsMol *__restrict
 // registers).  Before: 16 kernels, one per l class over the unmerged shells, every integral
 // accumulated per primitive quartet: 2.2 times the quartets, each with its own Boys evaluation.
 // All classes and the exchange list, 2048 molecules float32: 67.6 -> 38.2 ms, 36.0 ms with the units
-// packed; 50 molecules float64: 5.21 -> 2.06 ms.
+// packed (36.4 ms with the float64 (ss|ss) sums and unbiased Boys values); 50 molecules float64: 5.21 -> 2.06 ms.
 template <typename T> struct __align__(16) B2EriWarp {
   B2EriBra<T> bra[B2_MAXPP];
   double CD[32][3];

@@ -42,9 +42,9 @@ static void b2hc_2e_group(const B2PlanHost &P, const std::vector<B2EriTask> &tas
   if constexpr (G < 15) b2hc_2e_group<G + 1>(P, tasks, goff, D, hyb, tab, g, bad);
 }
 
-// The GPU kernels' tabulated vertical recursion (B2gVrr, grad_math.cuh) run on the host: every
-// step of the table in order (an order the kernels' level-by-level lane split respects), summed
-// over the quartet's primitive quartets with the kernels' weights, against the serial b2g_e0f0
+// The shell-quartet form's tabulated vertical recursion (B2gVrr, grad_math.cuh): every
+// step of the table in order, summed over the quartet's primitive quartets with the gradient's weights,
+// against the serial b2g_e0f0
 // of the same quartet.  Returns the largest difference relative to max |entry|.
 template <int LE, int LF, bool KET>
 static double b2hc_vrr_table(const B2Shell &a, const B2Shell &b, const B2Shell &c, const B2Shell &d,

@@ -277,7 +277,7 @@ __device__ void b2_jacobi_small_warp(double *A, double *V, double *rot, int *prs
 // ring layout per molecule (offset mat_off * 9): errs[9][N*N], hams[9][N*N]; B: 100 doubles
 // Bound by latency at one molecule per CTA; 62 orbitals, one molecule: 172 us per call before (two
 // products with one output element per thread, serial 10 x 10 Jacobi), 139 us with element-wise
-// ring passes, 95 us with several elements' loads in flight.
+// ring passes, 95 us with several elements' loads in flight, 99 us with the tangents in float64.
 template <int Q>
 __global__ void __launch_bounds__(64 * Q, B2_SCF_CTAS(Q))
 k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
@@ -418,8 +418,9 @@ k_fock_diis(const B2MolDev *__restrict__ mols, const int *__restrict__ active,
 // and order of eigenvectors, which the density does not depend on.
 // Products: M = L^T W, T = H M, A = M^T T, W' = W V', C = L^T W', D = 2 C_occ C_occ^T, all by
 // float64 MMA; two matrices in shared memory (74 KB at 64 orbitals, 3 CTAs per SM).  62 orbitals,
-// one molecule: 428 us per call before, 161 us now (168 us with one
-// dot-product chain and the library's reciprocal root).
+// one molecule: 428 us per call before, 161 us with one sweep
+// fewer where the cosines alone decided the last one (168 us with one dot-product chain and the
+// library's reciprocal root), 171 us now.
 template <int Q>
 __global__ void __launch_bounds__(64 * Q, B2_SCF_CTAS(Q))
 k_eigh_density(const B2MolDev *__restrict__ mols, const int *__restrict__ active,

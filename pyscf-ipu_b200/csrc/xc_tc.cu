@@ -597,7 +597,7 @@ template <int Q> __host__ __device__ constexpr uint32_t b2_xq_tmem_cols() {
 // thread quarters in turn (functions of their own first: they cost twice an sp group), Q slots
 // each; 4 ceil(N / 4) <= NB columns are used.  Before, columns were the AOs in order with a table
 // look-up, type selects and a float64 displacement per orbital: 6.87 -> 5.72 ms per evaluation of
-// 2048 uneven molecules (the kernel is issue-bound, and these phases were 38% of its instructions).
+// 2048 uneven molecules (these phases were 38% of the kernel's instructions).
 template <int Q>
 __device__ void b2_xq_columns(const B2gsMol &g, const B2gSuper *__restrict__ su, float (*sGrp)[64], int *sTy, int *sMap) {
   constexpr int NB = 16 * Q;
