@@ -722,10 +722,9 @@ k_xc_tq(const B2MolDev *__restrict__ mols, const B2gsMol *__restrict__ gms, cons
     for (int e = tid; e < NB * NB; e += B2_XT_NT) {
       const int r = e / NB, k = e - r * NB;
       const int ra = sMap[r], rk = sMap[k];
-      const double v = (ra >= 0 && rk >= 0) ? D[md.mat_off + (long long)ra * N + rk] : 0.0;
+      const float v = (ra >= 0 && rk >= 0) ? (float)D[md.mat_off + (long long)ra * N + rk] : 0.f;
       float d1, d2, t;
-      b2_split_rn((float)v, d1, t);
-      t = (float)(v - (double)d1);                  // not of float32's D: that one is rounded already
+      b2_split_rn(v, d1, t);
       d2 = __uint_as_float((__float_as_uint(t) + 0x1000u) & 0xFFFFE000u);
       const int idx = (((k >> 2) * (NB / 8) + (r >> 3)) * 8 + (r & 7)) * 4 + (k & 3);
       sDh[idx] = d1;
