@@ -24,7 +24,7 @@ CANDIDATES = (1, 2, 4, 8, 16, 32, 64)
 # towards zero, 1e-5 of V over 32 tiles, and a single molecule of 40 orbitals (73 tiles) takes 102 us
 # in items of 16 and 192 us in items of 32.  So the choice is the shortest length within SLACK of the
 # fastest: on 4096 molecules 12.3 ms against 11.8 ms with the fastest lengths (64, 32, 32, 32, 16).
-SLACK = 1.1
+SLACK = 1.09
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tuned.json")
 
 
